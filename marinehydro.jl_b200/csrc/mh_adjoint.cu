@@ -1609,7 +1609,7 @@ int adjoint_mixed_chunk(const Batch& bt, Vjp& vj, const double* d_omegas, const 
     auto* BC = (double2*)ctx->ws[WS_RHS];
     auto* X = (double2*)ctx->ws[WS_PHI];
     auto* PHIi = (double2*)ctx->ws[WS_TMP];  // phi = S sigma (indirect)
-    auto* adj = (double2*)ws_get(ctx, WS_ADJ, sizeof(double2) * cnt * 5);
+    auto* adj = (double2*)ws_get(ctx, WS_ADJ, sizeof(double2) * cnt * 4);
     auto* R32 = (float2*)ws_get(ctx, WS_TMP32, sizeof(float2) * cnt);
     auto* misc = ws_get(ctx, WS_MISC, refine_ctl_bytes(nb) + 64);
     if (!adj || !R32 || !misc) return MH_ERR_OOM;
@@ -1617,7 +1617,6 @@ int adjoint_mixed_chunk(const Batch& bt, Vjp& vj, const double* d_omegas, const 
     double2* LAM = adj + cnt;
     double2* BB = adj + 2 * cnt;
     double2* RHS = adj + 3 * cnt;
-    double2* R = adj + 4 * cnt;
     int rc;
     const double* tab = delh_table_for(ctx, bt.mask, &rc);
     if (rc) return rc;
@@ -1629,7 +1628,7 @@ int adjoint_mixed_chunk(const Batch& bt, Vjp& vj, const double* d_omegas, const 
         MH_CUDA_TRY(ctx, launch_gemv(ctx, true, S64, n, nb, PB, nullptr, RHS, nrhs, 1.0, 0.0));
     }
     // D^H lam = RHS: low-precision factors + FP64 refinement, FP64 fallback
-    if ((rc = mixed_refine_solve(ctx, n, nb, nrhs, D64, Dlo, Dinv, RHS, LAM, R, R32, misc, true, tol, max_iter,
+    if ((rc = mixed_refine_solve(ctx, n, nb, nrhs, D64, Dlo, Dinv, RHS, LAM, R32, misc, true, tol, max_iter,
                                  fb, info)))
         return rc;
     if (bt.direct) MH_CUDA_TRY(ctx, launch_gemv(ctx, true, S64, n, nb, LAM, nullptr, BB, nrhs, 1.0, 0.0));

@@ -521,47 +521,153 @@ __global__ void k_add_f32(double2* __restrict__ x, const float2* __restrict__ d,
 // Batched complex matrix products with few columns in FP64 (refinement
 // residuals, S b, S^H lambda), bandwidth-bound reads of the n x n matrices
 // (column-major, nb of them, n*n apart), nrhs <= kMaxRhs:
-// k_resid_n: R = beta B + alpha A X, one thread per row i, coalesced down the
-// columns; k_resid_c: R = beta B + alpha A^H X, one warp per JW outputs j
-// reading columns j (each x entry loaded once for the JW columns).  B may be R (read before written) or null when beta = 0.
-// Q >= nrhs: accumulators per thread (4, 8 or 16, picked by the launcher).
-template <int Q>
-__global__ void __launch_bounds__(256)
-k_resid_n(const double2* __restrict__ A, const double2* __restrict__ X, const double2* B, double2* R, int64_t n,
+// k_resid_n: R = beta B + alpha A X; k_resid_c: R = beta B + alpha A^H X, one
+// warp per JW outputs j reading columns j (each x entry loaded once for the
+// JW columns).  B may be R (read before written) or null when beta = 0.
+// Where a result goes: R (may be null), its FP32 copy R32 (may be null, the
+// right-hand side of the next refinement sweep) and rmax (may be null, per
+// matrix and right-hand side the bits of max |r|, which order like the
+// numbers for r >= 0 and put a NaN above everything).
+struct ResidOut {
+    double2* R;
+    float2* R32;
+    unsigned long long* rmax;
+};
+
+__device__ __forceinline__ unsigned long long abs_bits(double re, double im)
+{
+    return (unsigned long long)__double_as_longlong(hypot(re, im));
+}
+
+// One CTA makes 32 RPL consecutive rows of one matrix: a lane holds RPL rows
+// (32 apart), the NW warps take the columns in turn, KS at a time, with the
+// right-hand sides' entries of those columns staged in the warp's own shared
+// memory (no barrier until the end), and the warps' sums are added in warp
+// order.  Splitting the columns over the warps is what fills the chip when
+// the matrices are few or small: one thread per row running down all columns
+// (the form before this one) left a chain of n loads on n / 256 CTAs.
+// Measured on a B200, N = panels, w = matrices, q = right-hand sides, us per
+// product (HBM time at 6.5 TB/s in brackets), before -> now:
+//   N 1224, w 16, q 8: 1625 -> 132 (59);   N 2048, w 1, q 3: 580 -> 30 (10);
+//   N 870, w 16, q 1: 258 -> 48 (30);      N 200, w 20, q 7: 177 -> 9 (2);
+//   N 1456, w 32, q 3: 455 -> 225 (167);   N 2997, w 24, q 2: 968 -> 602 (530);
+//   N 2048, w 64, q 3: 770 -> 717 (660).
+// Q >= nrhs: columns of x held (zero beyond nrhs).
+constexpr int resid_ks(int Q, int NW)
+{
+    int k = 32;
+    while (k * Q * NW > 2048) k /= 2;
+    return k;
+}
+
+template <int Q, int RPL, int NW>
+__global__ void __launch_bounds__(32 * NW)
+k_resid_n(const double2* __restrict__ A, const double2* __restrict__ X, const double2* B, ResidOut out, int64_t n,
           int nrhs, double alpha, double beta, const int* done, const int* bad)
 {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t b = blockIdx.y;
-    if (i >= n) return;
+    constexpr int KS = resid_ks(Q, NW);    // columns staged at a time
+    constexpr int U = Q * RPL > 8 ? 4 / RPL : 8 / RPL;  // columns whose loads are in flight together
+    constexpr int QR = 64 / (NW * RPL);    // right-hand sides reduced at a time
+    __shared__ double2 sm[2048];           // NW * KS * Q staged, or NW * QR * 32 RPL partial sums
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t b = blockIdx.y, i0 = (int64_t)blockIdx.x * (32 * RPL);
     if (done && (done[b] || bad[b])) return;  // refinement: converged or marked matrices
     const double2* M = A + b * n * n;
     const double2* x = X + b * n * nrhs;
-    double ar[Q], ai[Q];
+    int64_t row[RPL];  // rows past the end repeat the last one and are not stored
 #pragma unroll
-    for (int q = 0; q < Q; ++q) ar[q] = ai[q] = 0.0;
-#pragma unroll 4
-    for (int64_t j = 0; j < n; ++j) {
-        const double2 m = M[j * n + i];
+    for (int u = 0; u < RPL; ++u) row[u] = min(i0 + 32 * u + lane, n - 1);
+    double ar[RPL][Q], ai[RPL][Q];
 #pragma unroll
-        for (int q = 0; q < Q; ++q)
-            if (q < nrhs) {
-                const double2 v = __ldg(x + (int64_t)q * n + j);
-                ar[q] = fma(m.x, v.x, fma(-m.y, v.y, ar[q]));
-                ai[q] = fma(m.x, v.y, fma(m.y, v.x, ai[q]));
-            }
-    }
+    for (int u = 0; u < RPL; ++u)
 #pragma unroll
-    for (int q = 0; q < Q; ++q)
-        if (q < nrhs) {
-            const int64_t o = b * n * nrhs + (int64_t)q * n + i;
-            const double2 bo = B ? B[o] : make_double2(0.0, 0.0);
-            R[o] = make_double2(beta * bo.x + alpha * ar[q], beta * bo.y + alpha * ai[q]);
+        for (int q = 0; q < Q; ++q) ar[u][q] = ai[u][q] = 0.0;
+    double2* xs = sm + warp * (KS * Q);
+    for (int64_t g = (int64_t)warp * KS; g < n; g += NW * KS) {
+        __syncwarp();
+        if (lane < KS)
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+                xs[lane * Q + q] = (q < nrhs && g + lane < n) ? __ldg(x + (int64_t)q * n + g + lane) : make_double2(0.0, 0.0);
+        __syncwarp();
+        const double2* col = M + g * n;
+        const int kend = (int)min((int64_t)KS, n - g);
+        int c = 0;
+        for (; c + U <= kend; c += U) {
+            double2 m[U][RPL];
+#pragma unroll
+            for (int t = 0; t < U; ++t)
+#pragma unroll
+                for (int u = 0; u < RPL; ++u) m[t][u] = col[(c + t) * n + row[u]];
+#pragma unroll
+            for (int t = 0; t < U; ++t)
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    const double2 v = xs[(c + t) * Q + q];
+#pragma unroll
+                    for (int u = 0; u < RPL; ++u) {
+                        ar[u][q] = fma(m[t][u].x, v.x, fma(-m[t][u].y, v.y, ar[u][q]));
+                        ai[u][q] = fma(m[t][u].x, v.y, fma(m[t][u].y, v.x, ai[u][q]));
+                    }
+                }
         }
+        for (; c < kend; ++c) {
+            double2 m[RPL];
+#pragma unroll
+            for (int u = 0; u < RPL; ++u) m[u] = col[c * n + row[u]];
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const double2 v = xs[c * Q + q];
+#pragma unroll
+                for (int u = 0; u < RPL; ++u) {
+                    ar[u][q] = fma(m[u].x, v.x, fma(-m[u].y, v.y, ar[u][q]));
+                    ai[u][q] = fma(m[u].x, v.y, fma(m[u].y, v.x, ai[u][q]));
+                }
+            }
+        }
+    }
+    // QR right-hand sides at a time through the same shared memory
+#pragma unroll
+    for (int q0 = 0; q0 < Q; q0 += QR) {
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < QR; ++q)
+            if (q0 + q < Q)
+#pragma unroll
+                for (int u = 0; u < RPL; ++u)
+                    sm[(warp * QR + q) * (32 * RPL) + 32 * u + lane] = make_double2(ar[u][q0 + q < Q ? q0 + q : 0], ai[u][q0 + q < Q ? q0 + q : 0]);
+        __syncthreads();
+        for (int t = threadIdx.x; t < QR * 32 * RPL; t += 32 * NW) {  // a warp holds 32 rows of one q
+            const int q = q0 + t / (32 * RPL);
+            const int64_t i = i0 + t % (32 * RPL);
+            if (q >= nrhs) break;  // whole warps
+            double sr = 0.0, si = 0.0;
+#pragma unroll
+            for (int w = 0; w < NW; ++w) {
+                const double2 v = sm[w * (QR * 32 * RPL) + t];
+                sr += v.x;
+                si += v.y;
+            }
+            unsigned long long big = 0;
+            if (i < n) {
+                const int64_t o = b * n * nrhs + (int64_t)q * n + i;
+                const double2 bo = B ? B[o] : make_double2(0.0, 0.0);
+                const double2 r = make_double2(beta * bo.x + alpha * sr, beta * bo.y + alpha * si);
+                if (out.R) out.R[o] = r;
+                if (out.R32) out.R32[o] = make_float2((float)r.x, (float)r.y);
+                if (out.rmax) big = abs_bits(r.x, r.y);
+            }
+            if (out.rmax) {
+                for (int off = 16; off > 0; off >>= 1) big = max(big, __shfl_xor_sync(0xffffffffu, big, off));
+                if ((t & 31) == 0) atomicMax(out.rmax + b * nrhs + q, big);
+            }
+        }
+    }
 }
 
 template <int Q, int JW>
 __global__ void __launch_bounds__(256, 2)
-k_resid_c(const double2* __restrict__ A, const double2* __restrict__ X, const double2* B, double2* R, int64_t n,
+k_resid_c(const double2* __restrict__ A, const double2* __restrict__ X, const double2* B, ResidOut out, int64_t n,
           int nrhs, double alpha, double beta, const int* done, const int* bad)
 {
     const int lane = threadIdx.x & 31;
@@ -596,10 +702,11 @@ k_resid_c(const double2* __restrict__ A, const double2* __restrict__ X, const do
             }
     }
 #pragma unroll
-    for (int u = 0; u < JW; ++u)
+    for (int q = 0; q < Q; ++q)
+        if (q < nrhs) {
+            unsigned long long big = 0;
 #pragma unroll
-        for (int q = 0; q < Q; ++q)
-            if (q < nrhs) {
+            for (int u = 0; u < JW; ++u) {
                 for (int off = 16; off > 0; off >>= 1) {
                     ar[u][q] += __shfl_down_sync(0xffffffffu, ar[u][q], off);
                     ai[u][q] += __shfl_down_sync(0xffffffffu, ai[u][q], off);
@@ -607,55 +714,59 @@ k_resid_c(const double2* __restrict__ A, const double2* __restrict__ X, const do
                 if (lane == 0 && j0 + u < n) {
                     const int64_t o = b * n * nrhs + (int64_t)q * n + j0 + u;
                     const double2 bo = B ? B[o] : make_double2(0.0, 0.0);
-                    R[o] = make_double2(beta * bo.x + alpha * ar[u][q], beta * bo.y + alpha * ai[u][q]);
+                    const double2 r = make_double2(beta * bo.x + alpha * ar[u][q], beta * bo.y + alpha * ai[u][q]);
+                    if (out.R) out.R[o] = r;
+                    if (out.R32) out.R32[o] = make_float2((float)r.x, (float)r.y);
+                    if (out.rmax) big = max(big, abs_bits(r.x, r.y));
                 }
             }
+            if (out.rmax && lane == 0) atomicMax(out.rmax + b * nrhs + q, big);
+        }
 }
 
-// Per (frequency z = blockIdx.x): max over right-hand sides of
-// max_i |r_iq| / max_i |b_iq|.
+// Start of a refinement: X = 0, R32 = fp32(RHS) and max |RHS| per matrix
+// (blockIdx.z) and right-hand side (blockIdx.y).
 __global__ void __launch_bounds__(256)
-k_rel_residual(const double2* __restrict__ r, const double2* __restrict__ b, int64_t n, int nrhs,
-               double* __restrict__ out, double tol, int* done, const int* bad, int* sweeps, int sweep)
+k_refine_init(const double2* __restrict__ rhs, int64_t n, double2* __restrict__ x, float2* __restrict__ r32,
+              unsigned long long* __restrict__ bmax)
 {
-    __shared__ double sr[256], sb[256];
-    // refinement control (done != null): skip converged or marked matrices,
-    // mark the ones that reach tol and count the sweeps of each
-    if (done && (done[blockIdx.x] || bad[blockIdx.x])) return;
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    const int64_t v = (int64_t)blockIdx.z * gridDim.y + blockIdx.y;
+    unsigned long long big = 0;
+    if (i < n) {
+        const double2 b = rhs[v * n + i];
+        x[v * n + i] = make_double2(0.0, 0.0);
+        r32[v * n + i] = make_float2((float)b.x, (float)b.y);
+        big = abs_bits(b.x, b.y);
+    }
+    for (int off = 16; off > 0; off >>= 1) big = max(big, __shfl_xor_sync(0xffffffffu, big, off));
+    if ((threadIdx.x & 31) == 0) atomicMax(bmax + v, big);
+}
+
+// End of a sweep, one thread per matrix z: the largest max|r| / max|b| of its
+// right-hand sides (a NaN counts as infinite), the mark of a matrix that
+// reaches tol and its sweep count; matrices already marked keep theirs.
+__global__ void k_refine_mark(const unsigned long long* __restrict__ bmax, unsigned long long* __restrict__ rmax,
+                              int nb, int nrhs, double* __restrict__ res, double tol, int* __restrict__ done,
+                              const int* __restrict__ bad, int* __restrict__ sweeps, int sweep)
+{
+    const int z = blockIdx.x * blockDim.x + threadIdx.x;
+    if (z >= nb || done[z] || bad[z]) return;
     double worst = 0.0;
     for (int q = 0; q < nrhs; ++q) {
-        const int64_t off = ((int64_t)blockIdx.x * nrhs + q) * n;
-        double mr = 0.0, mb = 0.0;
-        for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-            mr = fmax(mr, hypot(r[off + i].x, r[off + i].y));
-            mb = fmax(mb, hypot(b[off + i].x, b[off + i].y));
-        }
-        sr[threadIdx.x] = mr;
-        sb[threadIdx.x] = mb;
-        __syncthreads();
-        for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-            if (threadIdx.x < s) {
-                sr[threadIdx.x] = fmax(sr[threadIdx.x], sr[threadIdx.x + s]);
-                sb[threadIdx.x] = fmax(sb[threadIdx.x], sb[threadIdx.x + s]);
-            }
-            __syncthreads();
-        }
-        if (sb[0] > 0.0) worst = fmax(worst, sr[0] / sb[0]);
-        else if (sr[0] > 0.0 || sr[0] != sr[0]) worst = INFINITY;
-        __syncthreads();
+        const double r = __longlong_as_double((long long)rmax[z * nrhs + q]);
+        const double b = __longlong_as_double((long long)bmax[z * nrhs + q]);
+        const double ratio = b > 0.0 ? r / b : r > 0.0 ? INFINITY : r;
+        worst = ratio == ratio ? fmax(worst, ratio) : INFINITY;
+        rmax[z * nrhs + q] = 0;
     }
-    if (threadIdx.x == 0) {
-        worst = (worst == worst) ? worst : INFINITY;
-        out[blockIdx.x] = worst;
-        if (done) {
-            sweeps[blockIdx.x] = sweep;
-            if (worst <= tol) done[blockIdx.x] = 1;
-        }
-    }
+    res[z] = worst;
+    sweeps[z] = sweep;
+    if (worst <= tol) done[z] = 1;
 }
 
-// X += d and R32 = fp32(R) of the refinement, skipping converged or marked
-// matrices (per = entries per matrix).
+// X += d of the refinement, skipping converged or marked matrices (per =
+// entries per matrix).
 __global__ void k_refine_add(double2* __restrict__ x, const float2* __restrict__ d, int64_t per, int64_t count,
                              const int* __restrict__ done, const int* __restrict__ bad)
 {
@@ -664,16 +775,6 @@ __global__ void k_refine_add(double2* __restrict__ x, const float2* __restrict__
     const int64_t z = t / per;
     if (done[z] || bad[z]) return;
     x[t] = make_double2(x[t].x + (double)d[t].x, x[t].y + (double)d[t].y);
-}
-
-__global__ void k_refine_to_f32(const double2* __restrict__ a, float2* __restrict__ b, int64_t per, int64_t count,
-                                const int* __restrict__ done, const int* __restrict__ bad)
-{
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count) return;
-    const int64_t z = t / per;
-    if (done[z] || bad[z]) return;
-    b[t] = make_float2((float)a[t].x, (float)a[t].y);
 }
 
 // ---------------------------------------------------------------------------
@@ -889,7 +990,7 @@ int run_mixed_chunk(const Batch& bt, const double* d_omegas, const double* d_k, 
     phase_end(ctx, PH_LU);
     phase_begin(ctx, PH_REFINE);
     RefineState h;
-    if ((rc = refine_sweeps(ctx, false, n, nb, nrhs, D64, Dlo, Dinv, RHS, X, R, R32, ctl, tol, max_iter, h)))
+    if ((rc = refine_sweeps(ctx, false, n, nb, nrhs, D64, Dlo, Dinv, RHS, X, R32, ctl, tol, max_iter, h)))
         return rc;
     phase_end(ctx, PH_REFINE);
     info->refine_iterations = std::max(info->refine_iterations, h.most_sweeps());
@@ -1082,7 +1183,10 @@ int fp64_batched_getrs(mh_ctx* ctx, bool conj_trans, int64_t n, int nb, int nrhs
     return MH_OK;
 }
 
-size_t refine_ctl_bytes(int nb) { return (sizeof(double) + 3 * sizeof(int)) * (size_t)nb + 16; }
+// res, bad, done, sweeps, then (8-byte aligned) bmax and rmax
+static size_t refine_ctl_head(int nb) { return ((sizeof(double) + 3 * sizeof(int)) * (size_t)nb + 7) / 8 * 8; }
+
+size_t refine_ctl_bytes(int nb) { return refine_ctl_head(nb) + 2 * sizeof(unsigned long long) * kMaxRhs * (size_t)nb; }
 
 RefineCtl refine_ctl(void* block, int nb)
 {
@@ -1091,6 +1195,8 @@ RefineCtl refine_ctl(void* block, int nb)
     c.bad = (int*)(c.res + nb);
     c.done = c.bad + nb;
     c.sweeps = c.done + nb;
+    c.bmax = (unsigned long long*)((char*)block + refine_ctl_head(nb));
+    c.rmax = c.bmax + (size_t)kMaxRhs * nb;
     return c;
 }
 
@@ -1103,13 +1209,15 @@ int RefineState::most_sweeps() const
 }
 
 int refine_sweeps(mh_ctx* ctx, bool conj_trans, int64_t n, int nb, int nrhs, const double2* D64,
-                  const float2* Dlo, const float2* Dinv, const double2* RHS, double2* X, double2* R, float2* R32,
+                  const float2* Dlo, const float2* Dinv, const double2* RHS, double2* X, float2* R32,
                   const RefineCtl& c, double tol, int max_iter, RefineState& h)
 {
     const int64_t nn = n * n, nv = n * nrhs, cnt = nv * nb;
-    MH_CUDA_TRY(ctx, cudaMemsetAsync(X, 0, sizeof(double2) * cnt, ctx->stream));
-    MH_CUDA_TRY(ctx, cudaMemcpyAsync(R, RHS, sizeof(double2) * cnt, cudaMemcpyDeviceToDevice, ctx->stream));
-    MH_CUDA_TRY(ctx, cudaMemsetAsync(c.done, 0, sizeof(int) * 2 * (size_t)nb, ctx->stream));  // done, sweeps
+    // done, sweeps, bmax and rmax are one stretch of the control block
+    MH_CUDA_TRY(ctx, cudaMemsetAsync(c.done, 0, (size_t)((char*)(c.rmax + (size_t)nb * kMaxRhs) - (char*)c.done),
+                                     ctx->stream));
+    k_refine_init<<<dim3(blocks(n, 256), (unsigned)nrhs, (unsigned)nb), 256, 0, ctx->stream>>>(RHS, n, X, R32, c.bmax);
+    ctx->launches += 1;
     const size_t bytes = (sizeof(double) + 3 * sizeof(int)) * (size_t)nb;
     std::vector<unsigned char> host(bytes);
     h.res.assign(nb, INFINITY);
@@ -1124,14 +1232,15 @@ int refine_sweeps(mh_ctx* ctx, bool conj_trans, int64_t n, int nb, int nrhs, con
         // next to nothing on matrices that converged or are marked
         for (int s = 0, k = it == 0 ? ahead : 1; s < k && it < max_iter; ++s) {
             ++it;
-            k_refine_to_f32<<<blocks(cnt, 256), 256, 0, ctx->stream>>>(R, R32, nv, cnt, c.done, c.bad);
             MH_CUDA_TRY(ctx, launch_lu_solve_persist(ctx, ctx->lu_backend, conj_trans, Dlo, n, nn, nb, Dinv, R32,
                                                      nv, nrhs, c.bad, c.done));
             k_refine_add<<<blocks(cnt, 256), 256, 0, ctx->stream>>>(X, R32, nv, cnt, c.done, c.bad);
-            // R = RHS - op(D) X, then the residual ratio and the marks
-            MH_CUDA_TRY(ctx, launch_gemv(ctx, conj_trans, D64, n, nb, X, RHS, R, nrhs, -1.0, 1.0, c.done, c.bad));
-            k_rel_residual<<<nb, 256, 0, ctx->stream>>>(R, RHS, n, nrhs, c.res, tol, c.done, c.bad, c.sweeps, it);
-            ctx->launches += 3;
+            // R32 = RHS - op(D) X with its largest entries, then the residual ratio and the marks
+            MH_CUDA_TRY(ctx, launch_gemv(ctx, conj_trans, D64, n, nb, X, RHS, nullptr, nrhs, -1.0, 1.0, c.done, c.bad,
+                                         R32, c.rmax));
+            k_refine_mark<<<blocks(nb, 64), 64, 0, ctx->stream>>>(c.bmax, c.rmax, nb, nrhs, c.res, tol, c.done, c.bad,
+                                                                  c.sweeps, it);
+            ctx->launches += 2;
             MH_CUDA_TRY(ctx, cudaGetLastError());
         }
         MH_CUDA_TRY(ctx, cudaMemcpyAsync(host.data(), c.res, bytes, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1156,7 +1265,7 @@ int refine_sweeps(mh_ctx* ctx, bool conj_trans, int64_t n, int nb, int nrhs, con
 }
 
 int mixed_refine_solve(mh_ctx* ctx, int64_t n, int nb, int nrhs, const double2* D64, const float2* Dlo,
-                       const float2* Dinv, const double2* RHS, double2* X, double2* R, float2* R32, void* ctl_block,
+                       const float2* Dinv, const double2* RHS, double2* X, float2* R32, void* ctl_block,
                        bool conj_trans, double tol, int max_iter, FallbackStore& fb, mh_batch_info* info)
 {
     const int64_t nn = n * n, nv = n * nrhs;
@@ -1168,7 +1277,7 @@ int mixed_refine_solve(mh_ctx* ctx, int64_t n, int nb, int nrhs, const double2* 
     MH_CUDA_TRY(ctx, cudaMemcpyAsync(c.bad, used.data(), sizeof(int) * (size_t)nb, cudaMemcpyHostToDevice,
                                      ctx->stream));
     RefineState h;
-    if ((rc = refine_sweeps(ctx, conj_trans, n, nb, nrhs, D64, Dlo, Dinv, RHS, X, R, R32, c, tol, max_iter, h)))
+    if ((rc = refine_sweeps(ctx, conj_trans, n, nb, nrhs, D64, Dlo, Dinv, RHS, X, R32, c, tol, max_iter, h)))
         return rc;
     info->refine_iterations = std::max(info->refine_iterations, h.most_sweeps());
     for (int z = 0; z < nb; ++z) {
@@ -1249,45 +1358,72 @@ cudaError_t launch_add_f32(mh_ctx* ctx, double2* x, const float2* d, int64_t cou
     return cudaGetLastError();
 }
 
+namespace {
+
+using ResidKernel = void (*)(const double2*, const double2*, const double2*, ResidOut, int64_t, int, double, double,
+                             const int*, const int*);
+
+template <int RPL, int NW>
+ResidKernel resid_n_of(int nrhs)
+{
+    switch (nrhs) {
+        case 1: return k_resid_n<1, RPL, NW>;
+        case 2: return k_resid_n<2, RPL, NW>;
+        case 3: return k_resid_n<3, RPL, NW>;
+        case 4: return k_resid_n<4, RPL, NW>;
+        case 5: return k_resid_n<5, 1, NW>;
+        case 6: return k_resid_n<6, 1, NW>;
+        case 7: return k_resid_n<7, 1, NW>;
+        case 8: return k_resid_n<8, 1, NW>;
+        default: return nrhs <= 12 ? k_resid_n<12, 1, NW> : k_resid_n<16, 1, NW>;
+    }
+}
+
+template <int JW>
+ResidKernel resid_c_of(int nrhs)
+{
+    switch (nrhs) {
+        case 1: return k_resid_c<1, JW>;
+        case 2: return k_resid_c<2, JW>;
+        case 3: return k_resid_c<3, JW>;
+        case 4: return k_resid_c<4, JW>;
+        default: return nrhs <= 8 ? k_resid_c<8, JW < 2 ? JW : 2> : k_resid_c<kMaxRhs, 1>;
+    }
+}
+
+constexpr int64_t kFewCtas = 2 * 148;  // two CTAs per SM
+
+}  // namespace
+
 cudaError_t launch_gemv(mh_ctx* ctx, bool conj_trans, const double2* A, int64_t n, int nb, const double2* X,
                         const double2* B, double2* R, int nrhs, double alpha, double beta, const int* done,
-                        const int* bad, cudaStream_t stream)
+                        const int* bad, float2* R32, unsigned long long* rmax)
 {
-    cudaStream_t strm = stream ? stream : ctx->stream;
     if (nrhs < 1 || nrhs > kMaxRhs) return cudaErrorInvalidValue;
     if (beta == 0.0) B = nullptr;
-    const dim3 gn(blocks(n, 256), (unsigned)nb);
-    if (conj_trans) {  // 8 warps per CTA, JW columns per warp
-        const dim3 g4(blocks(n, 32), (unsigned)nb);
-        if (nrhs == 1) k_resid_c<1, 4><<<g4, 256, 0, strm>>>(A, X, B, R, n, nrhs, alpha, beta, done, bad);
-        else if (nrhs == 2) k_resid_c<2, 4><<<g4, 256, 0, strm>>>(A, X, B, R, n, nrhs, alpha, beta, done, bad);
-        else if (nrhs == 3) k_resid_c<3, 4><<<g4, 256, 0, strm>>>(A, X, B, R, n, nrhs, alpha, beta, done, bad);
-        else if (nrhs == 4) k_resid_c<4, 4><<<g4, 256, 0, strm>>>(A, X, B, R, n, nrhs, alpha, beta, done, bad);
-        else if (nrhs <= 8)
-            k_resid_c<8, 2><<<dim3(blocks(n, 16), (unsigned)nb), 256, 0, strm>>>(A, X, B, R, n, nrhs, alpha,
-                                                                                      beta, done, bad);
-        else
-            k_resid_c<kMaxRhs, 1><<<dim3(blocks(n, 8), (unsigned)nb), 256, 0, strm>>>(A, X, B, R, n, nrhs,
-                                                                                           alpha, beta, done, bad);
+    const ResidOut out{R, R32, rmax};
+    ResidKernel k;
+    unsigned grid;
+    int threads = 256;
+    if (conj_trans) {
+        // 8 warps per CTA, four columns per warp where that still makes two
+        // CTAs per SM, one column per warp otherwise
+        const bool few = (int64_t)blocks(n, 32) * nb < kFewCtas;
+        const int jw = nrhs > 8 ? 1 : few ? 1 : nrhs > 4 ? 2 : 4;
+        k = few ? resid_c_of<1>(nrhs) : resid_c_of<4>(nrhs);
+        grid = blocks(n, 8 * jw);
     } else {
-        if (nrhs <= 4) k_resid_n<4><<<gn, 256, 0, strm>>>(A, X, B, R, n, nrhs, alpha, beta, done, bad);
-        else if (nrhs <= 8) k_resid_n<8><<<gn, 256, 0, strm>>>(A, X, B, R, n, nrhs, alpha, beta, done, bad);
-        else k_resid_n<kMaxRhs><<<gn, 256, 0, strm>>>(A, X, B, R, n, nrhs, alpha, beta, done, bad);
+        // two rows per lane (half the shared-memory reads of x per entry of
+        // A) where that still makes four CTAs per SM and the sums fit the
+        // registers; 16 warps per CTA where even one row per lane makes
+        // fewer than two CTAs per SM
+        const int rpl = (nrhs <= 4 && (int64_t)blocks(n, 64) * nb >= 2 * kFewCtas) ? 2 : 1;
+        const bool few = (int64_t)blocks(n, 32) * nb < kFewCtas;
+        k = rpl == 2 ? resid_n_of<2, 8>(nrhs) : few ? resid_n_of<1, 16>(nrhs) : resid_n_of<1, 8>(nrhs);
+        grid = blocks(n, 32 * rpl);
+        if (few) threads = 512;
     }
-    ctx->launches += 1;
-    return cudaGetLastError();
-}
-
-cudaError_t launch_residual(mh_ctx* ctx, bool conj_trans, const double2* A, int64_t n, int nb, const double2* X,
-                            const double2* B, double2* R, int nrhs)
-{
-    return launch_gemv(ctx, conj_trans, A, n, nb, X, B, R, nrhs, -1.0, 1.0);
-}
-
-cudaError_t launch_rel_residual(mh_ctx* ctx, const double2* r, const double2* b, int64_t n, int nrhs,
-                                int nb, double* out)
-{
-    k_rel_residual<<<nb, 256, 0, ctx->stream>>>(r, b, n, nrhs, out, 0.0, nullptr, nullptr, nullptr, 0);
+    k<<<dim3(grid, (unsigned)nb), threads, 0, ctx->stream>>>(A, X, B, out, n, nrhs, alpha, beta, done, bad);
     ctx->launches += 1;
     return cudaGetLastError();
 }

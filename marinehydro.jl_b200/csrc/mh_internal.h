@@ -255,15 +255,13 @@ cudaError_t launch_add_f32(mh_ctx* ctx, double2* x, const float2* d, int64_t cou
 // R = beta B + alpha op(A) X for nb n x n complex matrices (op = identity or
 // ^H), X and B n x nrhs per matrix; B may be R, or null when beta = 0.
 // done, bad (device, per matrix, both or neither): skip matrices with either set.
+// R may be null when only the following are wanted: R32, the FP32 copy of the
+// result, and rmax (per matrix and right-hand side; raised to the bits of
+// max |r|, start it at 0).
 cudaError_t launch_gemv(mh_ctx* ctx, bool conj_trans, const double2* A, int64_t n, int nb, const double2* X,
                         const double2* B, double2* R, int nrhs, double alpha, double beta,
-                        const int* done = nullptr, const int* bad = nullptr, cudaStream_t stream = nullptr);
-// R = B - op(A) X for nb n x n complex matrices (op = identity or ^H).
-cudaError_t launch_residual(mh_ctx* ctx, bool conj_trans, const double2* A, int64_t n, int nb, const double2* X,
-                            const double2* B, double2* R, int nrhs);
-// out[z] = max over right-hand sides of max|r| / max|b| for nb problems of n x nrhs.
-cudaError_t launch_rel_residual(mh_ctx* ctx, const double2* r, const double2* b, int64_t n, int nrhs,
-                                int nb, double* out);
+                        const int* done = nullptr, const int* bad = nullptr, float2* R32 = nullptr,
+                        unsigned long long* rmax = nullptr);
 // Device force layout (F then FK, see hydro_batch) to the reference's output arrays.
 void unpack_outputs(const double2* h, int64_t nomega, const double* omegas, int64_t ndof, int64_t nbeta,
                     double* added_mass, double* damping, double* diffraction, double* froude_krylov);
@@ -277,12 +275,16 @@ int fp64_lu_solve(mh_ctx* ctx, int64_t n, double2* A, double2* B, int nrhs);
 int fallback_factor(mh_ctx* ctx, FallbackStore* fb, int64_t n, int nb, int z, const double2* D);
 // Per-matrix control of a refinement run, in device memory (one block of
 // refine_ctl_bytes(nb)): residual ratios, then marks of bad matrices (low-
-// precision LU pivot or wait timeout), of converged ones, and sweep counts.
+// precision LU pivot or wait timeout), of converged ones, and sweep counts,
+// then per matrix and right-hand side the largest |b| and the largest |r| of
+// the sweep (as bits).
 struct RefineCtl {
     double* res;
     int* bad;
     int* done;
     int* sweeps;
+    unsigned long long* bmax;
+    unsigned long long* rmax;
 };
 size_t refine_ctl_bytes(int nb);
 RefineCtl refine_ctl(void* block, int nb);
@@ -299,16 +301,16 @@ struct RefineState {
 // converged (residual ratio <= tol) or are marked bad, and the host checks
 // only after the number of sweeps the last call needed (then one sweep at a
 // time), at most max_iter sweeps.  c.bad must hold the marks on entry;
-// timeouts of the solve add to them.  R (FP64), R32 (FP32): scratch of the
-// size of RHS.  Leaves the control block's host copy in h.
+// timeouts of the solve add to them.  R32 (FP32): scratch of the size of RHS.
+// Leaves the control block's host copy in h.
 int refine_sweeps(mh_ctx* ctx, bool conj_trans, int64_t n, int nb, int nrhs, const double2* D64,
-                  const float2* Dlo, const float2* Dinv, const double2* RHS, double2* X, double2* R, float2* R32,
+                  const float2* Dlo, const float2* Dinv, const double2* RHS, double2* X, float2* R32,
                   const RefineCtl& c, double tol, int max_iter, RefineState& h);
 // X = op(D)^-1 RHS for nb problems by refine_sweeps; problems whose forward
 // solve fell back (fb.used), are marked bad or do not converge use FP64
 // factors.  ctl: a device block of refine_ctl_bytes(nb).
 int mixed_refine_solve(mh_ctx* ctx, int64_t n, int nb, int nrhs, const double2* D64, const float2* Dlo,
-                       const float2* Dinv, const double2* RHS, double2* X, double2* R, float2* R32, void* ctl,
+                       const float2* Dinv, const double2* RHS, double2* X, float2* R32, void* ctl,
                        bool conj_trans, double tol, int max_iter, FallbackStore& fb, mh_batch_info* info);
 // Frequency-independent Rankine parts SR, DR (n x n real) of the mixed path.
 int rankine_real(const Batch& bt, double* SR, double* DR);

@@ -737,7 +737,7 @@ int hydro_batch_jvp(mh_ctx* ctx, const mh_mesh* m, int64_t nomega, const double*
             if (rc) break;
             const int64_t cnt = nv * nb;
             auto* dmat = (double2*)ws_get(ctx, WS_PART, sizeof(double2) * nn * nb * 2);
-            auto* vec = (double2*)ws_get(ctx, WS_ADJ, sizeof(double2) * cnt * 6);
+            auto* vec = (double2*)ws_get(ctx, WS_ADJ, sizeof(double2) * cnt * 4);
             auto* R32 = (float2*)ws_get(ctx, WS_TMP32, sizeof(float2) * cnt);
             auto* misc = ws_get(ctx, WS_MISC, refine_ctl_bytes(nb) + 64);
             if (!dmat || !vec || !R32 || !misc) return MH_ERR_OOM;
@@ -748,9 +748,9 @@ int hydro_batch_jvp(mh_ctx* ctx, const mh_mesh* m, int64_t nomega, const double*
             auto* BC = (double2*)ctx->ws[WS_RHS];
             auto* X = (double2*)ctx->ws[WS_PHI];
             const double2* PHI = direct ? X : (double2*)ctx->ws[WS_TMP];
-            double2 *dBC = vec, *T = vec + cnt, *DX = vec + 2 * cnt, *DPHI = vec + 3 * cnt, *R = vec + 4 * cnt;
+            double2 *dBC = vec, *T = vec + cnt, *DX = vec + 2 * cnt, *DPHI = vec + 3 * cnt;
             auto solve = [&](double2* rhs, double2* out) -> int {
-                return mixed_refine_solve(ctx, n, nb, nrhs, D64, Dlo, Dinv, rhs, out, R, R32, misc, false, tol,
+                return mixed_refine_solve(ctx, n, nb, nrhs, D64, Dlo, Dinv, rhs, out, R32, misc, false, tol,
                                           max_iter, fb, &local);
             };
             rc = tangent_chunk(bt, jv, d_om + z0, d_dom + z0, d_k + z0, d_dk + z0, nb, tab, S64, BC, X, PHI, dmat,
