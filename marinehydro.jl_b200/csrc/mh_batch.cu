@@ -23,6 +23,7 @@
 
 #include "mh_device.cuh"
 #include "mh_internal.h"
+#include "mh_rankine.cuh"
 
 namespace mh {
 namespace {
@@ -43,39 +44,12 @@ __device__ __forceinline__ void load_panel_field(Panel& p, int f, double v)
 }
 
 __device__ __forceinline__ void stage_panels(Panel* sp, const double* __restrict__ geom, int64_t n,
-                                             int64_t j0)
+                                             int64_t j0, int cols)
 {
-    for (int t = threadIdx.x; t < kCols * G_NFIELDS; t += blockDim.x) {
-        int f = t / kCols, jj = t % kCols;
+    for (int t = threadIdx.x; t < cols * G_NFIELDS; t += blockDim.x) {
+        int f = t / cols, jj = t % cols;
         int64_t j = j0 + jj;
         load_panel_field(sp[jj], f, (j < n) ? geom[(int64_t)f * n + j] : 0.0);
-    }
-}
-
-// Rankine / reflected terms (real, frequency independent), with the -1/(4 pi)
-// factor and the 1/2 diagonal of D already applied.
-__global__ void __launch_bounds__(kRows)
-k_rankine_real(const double* __restrict__ geom, int64_t n, uint32_t mask, int direct,
-               double* __restrict__ SR, double* __restrict__ DR)
-{
-    __shared__ Panel sp[kCols];
-    const int64_t j0 = (int64_t)blockIdx.y * kCols;
-    stage_panels(sp, geom, n, j0);
-    __syncthreads();
-    const int64_t i = (int64_t)blockIdx.x * kRows + threadIdx.x;
-    if (i >= n) return;
-    const double x[3] = {geom[G_CX * n + i], geom[G_CY * n + i], geom[G_CZ * n + i]};
-    const double ni[3] = {geom[G_NX * n + i], geom[G_NY * n + i], geom[G_NZ * n + i]};
-    const int jend = (int)min((int64_t)kCols, n - j0);
-    for (int jj = 0; jj < jend; ++jj) {
-        const Panel& p = sp[jj];
-        const int64_t j = j0 + jj;
-        cplx s, g[3];
-        pair_integrals(x, p, 0.0, mask, !direct, nullptr, s, g);
-        const double* nn = direct ? p.n : ni;
-        const int64_t o = j * n + i;
-        SR[o] = -kInv4Pi * s.re;
-        DR[o] = (i == j ? 0.5 : 0.0) - kInv4Pi * (nn[0] * g[0].re + nn[1] * g[1].re + nn[2] * g[2].re);
     }
 }
 
@@ -83,14 +57,14 @@ k_rankine_real(const double* __restrict__ geom, int64_t n, uint32_t mask, int di
 // complex (S64, D64) and the FP32 LU copy of D (Dlo).
 template <bool kDelh>
 __global__ void __launch_bounds__(kRows)
-k_wave_batch(const double* __restrict__ geom, int64_t n, int direct, const double* __restrict__ tab,
+k_wave_batch(const double* __restrict__ geom, int64_t n, int direct, int cols, const double* __restrict__ tab,
              const double* __restrict__ kvec, const double* __restrict__ SR,
              const double* __restrict__ DR, double2* __restrict__ S64, double2* __restrict__ D64,
              float2* __restrict__ Dlo, double2* __restrict__ tape)
 {
     __shared__ Panel sp[kCols];
-    const int64_t j0 = (int64_t)blockIdx.y * kCols;
-    stage_panels(sp, geom, n, j0);
+    const int64_t j0 = (int64_t)blockIdx.y * cols;
+    stage_panels(sp, geom, n, j0, cols);
     __syncthreads();
     const int64_t i = (int64_t)blockIdx.x * kRows + threadIdx.x;
     if (i >= n) return;
@@ -98,7 +72,7 @@ k_wave_batch(const double* __restrict__ geom, int64_t n, int direct, const doubl
     const int64_t mat = (int64_t)blockIdx.z * n * n;
     const double x[3] = {geom[G_CX * n + i], geom[G_CY * n + i], geom[G_CZ * n + i]};
     const double ni[3] = {geom[G_NX * n + i], geom[G_NY * n + i], geom[G_NZ * n + i]};
-    const int jend = (int)min((int64_t)kCols, n - j0);
+    const int jend = (int)min((int64_t)cols, n - j0);
     for (int jj = 0; jj < jend; ++jj) {
         const Panel& p = sp[jj];
         const int64_t j = j0 + jj;
@@ -215,7 +189,7 @@ __device__ __forceinline__ float hfma(float a, float b, float c) { return fmaf(a
 // terms and everything after the series stay in FP64.
 template <typename HT, typename CT>
 __global__ void __launch_bounds__(kWT, 3)
-k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, const double* __restrict__ tab,
+k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, int cols, const double* __restrict__ tab,
                  const double* __restrict__ kvec, int nb, const double* __restrict__ SR,
                  const double* __restrict__ DR, double2* __restrict__ S64, double2* __restrict__ D64,
                  float2* __restrict__ Dlo, double2* __restrict__ tape, int* __restrict__ fall)
@@ -226,8 +200,8 @@ k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, const d
     double* ksm = invk + kAllwMaxFreqs;            // [nb]
     HT* w = reinterpret_cast<HT*>(ksm + kAllwMaxFreqs);  // [4 * NU][kWT]
     __shared__ Panel sp[kCols];
-    const int64_t j0 = (int64_t)blockIdx.y * kCols;
-    stage_panels(sp, geom, n, j0);
+    const int64_t j0 = (int64_t)blockIdx.y * cols;
+    stage_panels(sp, geom, n, j0, cols);
     for (int t = threadIdx.x; t < nb; t += blockDim.x) {
         ksm[t] = kvec[t];
         logk[t] = log(kvec[t]);
@@ -241,7 +215,7 @@ k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, const d
     const double x[3] = {geom[G_CX * n + i], geom[G_CY * n + i], geom[G_CZ * n + i]};
     const double ni[3] = {geom[G_NX * n + i], geom[G_NY * n + i], geom[G_NZ * n + i]};
     const bool wrt_first = !direct;
-    const int jend = (int)min((int64_t)kCols, n - j0);
+    const int jend = (int)min((int64_t)cols, n - j0);
     for (int jj = 0; jj < jend; ++jj) {
         const Panel& p = sp[jj];
         const int64_t j = j0 + jj;
@@ -354,22 +328,22 @@ k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, const d
 // written by one kernel at least, whatever the rounding of d in each (a pair
 // written by both gets this kernel's value, which runs second).
 __global__ void __launch_bounds__(kWT)
-k_wave_delh_allw_rest(const int* __restrict__ fall, const double* __restrict__ geom, int64_t n, int direct,
+k_wave_delh_allw_rest(const int* __restrict__ fall, const double* __restrict__ geom, int64_t n, int direct, int cols,
                       const double* __restrict__ tab, const double* __restrict__ kvec, int nb,
                       const double* __restrict__ SR, const double* __restrict__ DR, double2* __restrict__ S64,
                       double2* __restrict__ D64, float2* __restrict__ Dlo, double2* __restrict__ tape)
 {
     if (*fall == 0) return;
     __shared__ Panel sp[kCols];
-    const int64_t j0 = (int64_t)blockIdx.y * kCols;
-    stage_panels(sp, geom, n, j0);
+    const int64_t j0 = (int64_t)blockIdx.y * cols;
+    stage_panels(sp, geom, n, j0, cols);
     __syncthreads();
     const int64_t i = (int64_t)blockIdx.x * kWT + threadIdx.x;
     if (i >= n) return;
     const int64_t nn = n * n;
     const double x[3] = {geom[G_CX * n + i], geom[G_CY * n + i], geom[G_CZ * n + i]};
     const double ni[3] = {geom[G_NX * n + i], geom[G_NY * n + i], geom[G_NZ * n + i]};
-    const int jend = (int)min((int64_t)kCols, n - j0);
+    const int jend = (int)min((int64_t)cols, n - j0);
     for (int jj = 0; jj < jend; ++jj) {
         const Panel& p = sp[jj];
         const int64_t o = (j0 + jj) * n + i;
@@ -923,12 +897,14 @@ int run_mixed_chunk(const Batch& bt, const double* d_omegas, const double* d_k, 
     if (rc) return rc;
     // matrices
     const uint32_t wave = bt.mask & (MH_GF_WU | MH_GF_DELHOMMEAU);
-    dim3 grid(blocks(n, kRows), blocks(n, kCols), (unsigned)nb);
+    const bool allw = wave == MH_GF_DELHOMMEAU && tab && nb >= kAllwMinFreqs;
+    const int cols = wave_cols(n, kCols, allw ? 1 : nb);  // the frequency-batched pass has one grid for all
+    dim3 grid(blocks(n, kRows), blocks(n, cols), (unsigned)nb);
     phase_begin(ctx, PH_WAVE);
     if (wave == MH_GF_WU)
-        k_wave_batch<false><<<grid, kRows, 0, ctx->stream>>>(bt.m->geom, n, bt.direct, nullptr, d_k, SR,
+        k_wave_batch<false><<<grid, kRows, 0, ctx->stream>>>(bt.m->geom, n, bt.direct, cols, nullptr, d_k, SR,
                                                             DR, S64, D64, Dlo, nullptr);
-    else if (wave == MH_GF_DELHOMMEAU && tab && nb >= kAllwMinFreqs) {
+    else if (allw) {
         const int lvl = ctx->wave_series_fp32;
         auto* wk = lvl == 2 ? k_wave_delh_allw<float, float>
                  : lvl == 1 ? k_wave_delh_allw<float, double> : k_wave_delh_allw<double, double>;
@@ -949,16 +925,16 @@ int run_mixed_chunk(const Batch& bt, const double* d_omegas, const double* d_k, 
             const int m = std::min(kAllwMaxFreqs, nb - z);
             const int64_t off = (int64_t)z * nn;
             double2* tp = bt.tape ? bt.tape + 2 * off : nullptr;
-            const dim3 g2(blocks(n, kWT), blocks(n, kCols));
+            const dim3 g2(blocks(n, kWT), blocks(n, cols));
             MH_CUDA_TRY(ctx, cudaMemsetAsync(d_fall, 0, sizeof(int), ctx->stream));
-            wk<<<g2, kWT, wsm, ctx->stream>>>(bt.m->geom, n, bt.direct, tab, d_k + z, m, SR, DR, S64 + off,
+            wk<<<g2, kWT, wsm, ctx->stream>>>(bt.m->geom, n, bt.direct, cols, tab, d_k + z, m, SR, DR, S64 + off,
                                               D64 + off, Dlo + off, tp, d_fall);
-            k_wave_delh_allw_rest<<<g2, kWT, 0, ctx->stream>>>(d_fall, bt.m->geom, n, bt.direct, tab, d_k + z, m,
+            k_wave_delh_allw_rest<<<g2, kWT, 0, ctx->stream>>>(d_fall, bt.m->geom, n, bt.direct, cols, tab, d_k + z, m,
                                                               SR, DR, S64 + off, D64 + off, Dlo + off, tp);
             ctx->launches += 1 + (z > 0);
         }
     } else if (wave == MH_GF_DELHOMMEAU)
-        k_wave_batch<true><<<grid, kRows, 0, ctx->stream>>>(bt.m->geom, n, bt.direct, tab, d_k, SR, DR,
+        k_wave_batch<true><<<grid, kRows, 0, ctx->stream>>>(bt.m->geom, n, bt.direct, cols, tab, d_k, SR, DR,
                                                            S64, D64, Dlo, bt.tape);
     else if (wave == 0)
         k_no_wave_batch<<<dim3(blocks(nn, 256), nb), 256, 0, ctx->stream>>>(nn, SR, DR, S64, D64, Dlo);
@@ -1054,13 +1030,15 @@ int run_fp64_chunk(const Batch& bt, const double* d_omegas, const double* d_k, i
     const double* tab = delh_table_for(ctx, bt.mask, &rc);
     if (rc) return rc;
     const uint32_t wave = bt.mask & (MH_GF_WU | MH_GF_DELHOMMEAU);
+    const bool allw = wave == MH_GF_DELHOMMEAU && tab && nb >= kAllwMinFreqs;
+    const int cols = wave_cols(n, kCols, allw ? 1 : nb);  // the frequency-batched pass has one grid for all
     phase_begin(ctx, PH_WAVE);
     if (wave == MH_GF_WU) {
-        dim3 grid(blocks(n, kRows), blocks(n, kCols), (unsigned)nb);
-        k_wave_batch<false><<<grid, kRows, 0, ctx->stream>>>(bt.m->geom, n, bt.direct, nullptr, d_k, SR, DR, S64,
+        dim3 grid(blocks(n, kRows), blocks(n, cols), (unsigned)nb);
+        k_wave_batch<false><<<grid, kRows, 0, ctx->stream>>>(bt.m->geom, n, bt.direct, cols, nullptr, d_k, SR, DR, S64,
                                                             D64, Dlo, nullptr);
         ctx->launches += 1;
-    } else if (wave == MH_GF_DELHOMMEAU && tab && nb >= kAllwMinFreqs) {
+    } else if (allw) {
         MH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_wave_delh_allw<double, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)kWaveAllwSmem));
         MH_CUDA_TRY(ctx, cudaMemcpyToSymbolAsync(c_polar_mono, tab + kTabMonoOff, sizeof(c_polar_mono), 0,
@@ -1068,18 +1046,18 @@ int run_fp64_chunk(const Batch& bt, const double* d_omegas, const double* d_k, i
         for (int z = 0; z < nb; z += kAllwMaxFreqs) {
             const int m = std::min(kAllwMaxFreqs, nb - z);
             const int64_t off = (int64_t)z * nn;
-            const dim3 g2(blocks(n, kWT), blocks(n, kCols));
+            const dim3 g2(blocks(n, kWT), blocks(n, cols));
             MH_CUDA_TRY(ctx, cudaMemsetAsync(d_fall, 0, sizeof(int), ctx->stream));
             double2* tp = bt.tape ? bt.tape + 2 * off : nullptr;
             k_wave_delh_allw<double, double><<<g2, kWT, kWaveAllwSmem, ctx->stream>>>(
-                bt.m->geom, n, bt.direct, tab, d_k + z, m, SR, DR, S64 + off, D64 + off, Dlo + off, tp, d_fall);
-            k_wave_delh_allw_rest<<<g2, kWT, 0, ctx->stream>>>(d_fall, bt.m->geom, n, bt.direct, tab, d_k + z, m,
+                bt.m->geom, n, bt.direct, cols, tab, d_k + z, m, SR, DR, S64 + off, D64 + off, Dlo + off, tp, d_fall);
+            k_wave_delh_allw_rest<<<g2, kWT, 0, ctx->stream>>>(d_fall, bt.m->geom, n, bt.direct, cols, tab, d_k + z, m,
                                                               SR, DR, S64 + off, D64 + off, Dlo + off, tp);
             ctx->launches += 2;
         }
     } else if (wave == MH_GF_DELHOMMEAU) {
-        dim3 grid(blocks(n, kRows), blocks(n, kCols), (unsigned)nb);
-        k_wave_batch<true><<<grid, kRows, 0, ctx->stream>>>(bt.m->geom, n, bt.direct, tab, d_k, SR, DR, S64, D64,
+        dim3 grid(blocks(n, kRows), blocks(n, cols), (unsigned)nb);
+        k_wave_batch<true><<<grid, kRows, 0, ctx->stream>>>(bt.m->geom, n, bt.direct, cols, tab, d_k, SR, DR, S64, D64,
                                                            Dlo, bt.tape);
         ctx->launches += 1;
     } else if (wave == 0) {
@@ -1315,14 +1293,9 @@ int fallback_factor(mh_ctx* ctx, FallbackStore* fb, int64_t n, int nb, int z, co
 int rankine_real(const Batch& bt, double* SR, double* DR)
 {
     mh_ctx* ctx = bt.ctx;
-    const int64_t n = bt.n;
     phase_begin(ctx, PH_RANKINE);
-    k_rankine_real<<<dim3(blocks(n, kRows), blocks(n, kCols)), kRows, 0, ctx->stream>>>(
-        bt.m->geom, n, bt.mask & (MH_GF_RANKINE | MH_GF_RANKINE_REFLECTED |
-                                  MH_GF_RANKINE_REFLECTED_NEGATIVE), bt.direct, SR, DR);
-    ctx->launches += 1;
+    MH_CUDA_TRY(ctx, launch_rankine_real(ctx, bt.m, bt.mask, bt.direct, SR, DR));
     phase_end(ctx, PH_RANKINE);
-    MH_CUDA_TRY(ctx, cudaGetLastError());
     return MH_OK;
 }
 

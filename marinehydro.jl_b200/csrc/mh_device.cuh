@@ -152,19 +152,26 @@ __device__ __forceinline__ double signd(double v) { return (double)((v > 0) - (v
 // both_integral_and_integral_gradient(::Rankine) (rankine.jl:65-123),
 // computed in one pass over the panel edges.  The gradient is w.r.t. the
 // source point; callers negate it for with_respect_to_first_variable.
+// rankine_far: the point-source form beyond seven panel radii (false, and
+// nothing written, within them); rankine_near: the closed form.
 template <class T>
-__device__ __forceinline__ void rankine_pair(const T x[3], const PanelT<T>& p, T& integral, T grad[3])
+__device__ __forceinline__ bool rankine_far(const T x[3], const PanelT<T>& p, T& integral, T grad[3])
 {
     T rb[3] = {x[0] - p.c[0], x[1] - p.c[1], x[2] - p.c[2]};
     T r = sqrt(dot3(rb, rb));
-    if (val(r) > 7.0 * val(p.radius)) {
-        T inv3 = 1.0 / (r * r * r);
-        integral = p.area / r;
-        grad[0] = rb[0] * inv3 * p.area;
-        grad[1] = rb[1] * inv3 * p.area;
-        grad[2] = rb[2] * inv3 * p.area;
-        return;
-    }
+    if (!(val(r) > 7.0 * val(p.radius))) return false;
+    T inv3 = 1.0 / (r * r * r);
+    integral = p.area / r;
+    grad[0] = rb[0] * inv3 * p.area;
+    grad[1] = rb[1] * inv3 * p.area;
+    grad[2] = rb[2] * inv3 * p.area;
+    return true;
+}
+
+template <class T>
+__device__ __forceinline__ void rankine_near(const T x[3], const PanelT<T>& p, T& integral, T grad[3])
+{
+    T rb[3] = {x[0] - p.c[0], x[1] - p.c[1], x[2] - p.c[2]};
     T I = tconst<T>(0.0), g0 = tconst<T>(0.0), g1 = tconst<T>(0.0), g2 = tconst<T>(0.0);
     T GZ = dot3(rb, p.n);
     T aGZ = fabs(GZ);
@@ -222,6 +229,12 @@ __device__ __forceinline__ void rankine_pair(const T x[3], const PanelT<T>& p, T
     grad[0] = g0;
     grad[1] = g1;
     grad[2] = g2;
+}
+
+template <class T>
+__device__ __forceinline__ void rankine_pair(const T x[3], const PanelT<T>& p, T& integral, T grad[3])
+{
+    if (!rankine_far(x, p, integral, grad)) rankine_near(x, p, integral, grad);
 }
 
 // ---------------------------------------------------------------------------

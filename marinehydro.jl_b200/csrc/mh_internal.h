@@ -174,6 +174,8 @@ cudaError_t raise_smem_cap(const void* kernel, size_t bytes);
 // tab: Delhommeau table or null (adaptive quadrature).
 cudaError_t launch_assemble_f64(mh_ctx* ctx, const mh_mesh* m, double k, uint32_t mask,
                                 int direct, const double* tab, double2* S, double2* D);
+// Real S and D of the Rankine terms of mask (n x n), with the 1/2 diagonal of D.
+cudaError_t launch_rankine_real(mh_ctx* ctx, const mh_mesh* m, uint32_t mask, int direct, double* SR, double* DR);
 // bc[i] = -i omega (n_i . dof_i); dof is a device 3-vector (dof_rows==1) or n x 3 col-major.
 cudaError_t launch_radiation_bc(mh_ctx* ctx, const mh_mesh* m, const double* dof, int64_t dof_rows,
                                 double omega, double2* bc);

@@ -29,6 +29,7 @@
 
 #include "mh_device.cuh"
 #include "mh_internal.h"
+#include "mh_rankine.cuh"
 
 namespace mh {
 namespace {
@@ -49,61 +50,28 @@ __device__ __forceinline__ void stage_t(Panel* tp, const double* __restrict__ tg
     stage(tp, tgeom, n, j0);
 }
 
-__device__ __forceinline__ PanelT<d1> dual_panel(const Panel& p, const Panel& t)
-{
-    PanelT<d1> q;
-    for (int a = 0; a < 3; ++a) {
-        q.c[a].v = p.c[a];
-        q.c[a].d[0] = t.c[a];
-        q.n[a].v = p.n[a];
-        q.n[a].d[0] = t.n[a];
-    }
-    for (int k = 0; k < 12; ++k) {
-        q.v[k].v = p.v[k];
-        q.v[k].d[0] = t.v[k];
-    }
-    q.area.v = p.area;
-    q.area.d[0] = t.area;
-    q.radius.v = p.radius;
-    q.radius.d[0] = 0.0;  // radii only select branches
-    return q;
-}
-
 // Tangent of the frequency-independent Rankine terms (rankine.jl,
 // rankine_reflected*.jl) along tgeom: dSR = -d(sum integral)/4pi,
 // dDR = -d(nD . sum gradient)/4pi, stored as complex with zero imaginary part.
-__global__ void __launch_bounds__(kJR)
-k_rankine_tangent(const double* __restrict__ geom, const double* __restrict__ tgeom, int64_t n, uint32_t mask,
-                  int direct, double2* __restrict__ dSR, double2* __restrict__ dDR)
-{
-    __shared__ Panel sp[kGradCols], tp[kGradCols];
-    const int64_t j0 = (int64_t)blockIdx.y * kGradCols;
-    stage(sp, geom, n, j0);
-    stage_t(tp, tgeom, n, j0);
-    __syncthreads();
-    const int64_t i = (int64_t)blockIdx.x * kJR + threadIdx.x;
-    if (i >= n) return;
-    d1 x[3], ni[3];
-    for (int c = 0; c < 3; ++c) {
-        x[c].v = geom[(G_CX + c) * n + i];
-        x[c].d[0] = tgeom[(G_CX + c) * n + i];
-        ni[c].v = geom[(G_NX + c) * n + i];
-        ni[c].d[0] = tgeom[(G_NX + c) * n + i];
+struct RankineTangentGeom {
+    const double *geom, *tgeom;
+    int64_t n;
+    __device__ __forceinline__ void field(int f, int64_t j, d1& v) const
+    {
+        v.v = geom[(int64_t)f * n + j];
+        v.d[0] = f == G_RADIUS ? 0.0 : tgeom[(int64_t)f * n + j];  // radii only select branches
     }
-    const int jend = (int)min((int64_t)kGradCols, n - j0);
-    const uint32_t rmask = mask & (MH_GF_RANKINE | MH_GF_RANKINE_REFLECTED | MH_GF_RANKINE_REFLECTED_NEGATIVE);
-    for (int jj = 0; jj < jend; ++jj) {
-        const PanelT<d1> q = dual_panel(sp[jj], tp[jj]);
-        const int64_t j = j0 + jj;
-        cx<d1> s, g[3];
-        pair_integrals(x, q, tconst<d1>(0.0), rmask, !direct, nullptr, s, g);
-        const d1* nD = direct ? q.n : ni;
-        const d1 dn = nD[0] * g[0].re + nD[1] * g[1].re + nD[2] * g[2].re;
-        const int64_t o = j * n + i;
-        dSR[o] = make_double2(-kI4P * s.re.d[0], 0.0);
-        dDR[o] = make_double2(-kI4P * dn.d[0], 0.0);
+};
+struct RankineTangentOut {
+    double2 *S, *D;
+    static __device__ __forceinline__ double take(const d1& v) { return v.d[0]; }
+    __device__ __forceinline__ void store(int64_t o, bool, double s, double d, const d1 (*)[kRkRows], int,
+                                          const PanelT<d1>&) const
+    {
+        S[o] = make_double2(-kI4P * s, 0.0);
+        D[o] = make_double2(-kI4P * d, 0.0);
     }
-}
+};
 
 // Pair tangents of the wave term (abstract_greens_function.jl:88-155 with
 // the one-point rule): s = k A G, g = (sg k^2 A u_x G_r, sg k^2 A u_y G_r,
@@ -667,10 +635,8 @@ int hydro_batch_jvp(mh_ctx* ctx, const mh_mesh* m, int64_t nomega, const double*
     jv.dSR = (double2*)ws_get(ctx, WS_WSD, sizeof(double2) * nn * 2);
     if (!jv.dSR) return MH_ERR_OOM;
     jv.dDR = jv.dSR + nn;
-    k_rankine_tangent<<<dim3(nblk(n, kJR), nblk(n, kGradCols)), kJR, 0, ctx->stream>>>(m->geom, d_tgeom, n, mask,
-                                                                                     direct, jv.dSR, jv.dDR);
-    ctx->launches += 1;
-    MH_CUDA_TRY(ctx, cudaGetLastError());
+    MH_CUDA_TRY(ctx, (launch_rankine_tile<d1>(ctx, RankineTangentGeom{m->geom, d_tgeom, n}, n, mask, direct,
+                                             RankineTangentOut{jv.dSR, jv.dDR})));
     int rc;
     const double* tab = delh_table_for(ctx, mask, &rc);
     if (rc) return rc;

@@ -1,70 +1,62 @@
 // FP64 kernels: influence-matrix assembly, boundary conditions and the
 // pressure -> force reduction.
 //
-// Assembly (src/matrix_assembly.jl:4-42): one CTA owns a tile of 128
-// collocation rows x 16 source columns.  The 16 source panels are staged in
-// shared memory (20 doubles each: centre, normal, area, radius, 4 vertices)
-// and broadcast to all threads; each thread keeps its collocation point in
-// registers and walks the 16 columns.  For a fixed column the 128 threads
+// Assembly (src/matrix_assembly.jl:4-42): the frequency-independent Rankine
+// terms by tiles with their near pairs listed, and the wave terms added where a
+// tile is stored (mh_rankine.cuh).  For a fixed column the 128 threads of a CTA
 // write 128 consecutive complex128 entries of the column-major matrix, so every
 // store is a fully coalesced 2 KiB run.
 #include <cuda_runtime.h>
 
 #include "mh_device.cuh"
 #include "mh_internal.h"
+#include "mh_rankine.cuh"
 
 namespace mh {
 
 namespace {
 
-constexpr int kRows = 128;
-constexpr int kCols = 16;
 constexpr double kInv4Pi = 1.0 / (4.0 * kPi);  // -1/(2 tau), tau = 2 pi (MarineHydro.jl:11)
 
-__device__ __forceinline__ void load_panel_field(Panel& p, int f, double v)
-{
-    // geometry field order -> Panel layout
-    if (f < 3) p.c[f] = v;
-    else if (f < 6) p.n[f - 3] = v;
-    else if (f == G_AREA) p.area = v;
-    else if (f == G_RADIUS) p.radius = v;
-    else p.v[f - G_V] = v;
-}
-
-__global__ void __launch_bounds__(kRows)
-k_assemble_f64(const double* __restrict__ geom, int64_t n, double k, uint32_t mask, int direct,
-               const double* __restrict__ tab, double2* __restrict__ S, double2* __restrict__ D)
-{
-    __shared__ Panel sp[kCols];
-    const int64_t j0 = (int64_t)blockIdx.y * kCols;
-    for (int t = threadIdx.x; t < kCols * G_NFIELDS; t += blockDim.x) {
-        int f = t / kCols, jj = t % kCols;
-        int64_t j = j0 + jj;
-        double v = (j < n) ? geom[(int64_t)f * n + j] : 0.0;
-        load_panel_field(sp[jj], f, v);
-    }
-    __syncthreads();
-    const int64_t i = (int64_t)blockIdx.x * kRows + threadIdx.x;
-    if (i >= n) return;
-    const double x[3] = {geom[G_CX * n + i], geom[G_CY * n + i], geom[G_CZ * n + i]};
-    const double ni[3] = {geom[G_NX * n + i], geom[G_NY * n + i], geom[G_NZ * n + i]};
-    const bool wrt_first = !direct;
-    const int jend = (int)min((int64_t)kCols, n - j0);
-    for (int jj = 0; jj < jend; ++jj) {
-        const Panel& p = sp[jj];
-        const int64_t j = j0 + jj;
-        cplx s, g[3];
-        pair_integrals(x, p, k, mask, wrt_first, tab, s, g);
-        const int64_t o = j * n + i;
-        if (S) S[o] = make_double2(-kInv4Pi * s.re, -kInv4Pi * s.im);
-        if (D) {
-            const double* nn = direct ? p.n : ni;
-            double dre = nn[0] * g[0].re + nn[1] * g[1].re + nn[2] * g[2].re;
-            double dim = nn[0] * g[0].im + nn[1] * g[1].im + nn[2] * g[2].im;
-            D[o] = make_double2((i == j ? 0.5 : 0.0) - kInv4Pi * dre, -kInv4Pi * dim);
+// S and D with the -1/(4 pi) factor and the 1/2 diagonal of D: complex, with
+// the wave terms kWave (bits) at wavenumber k added (either of S and D may be
+// null), or the real Rankine parts.
+template <uint32_t kWave>
+struct AssembleOut {
+    double2 *S, *D;
+    const double* tab;
+    double k;
+    int direct;
+    static __device__ __forceinline__ double take(double v) { return v; }
+    __device__ __forceinline__ void store(int64_t o, bool diag, double s, double d, const double (*xs)[kRkRows],
+                                          int row, const Panel& p) const
+    {
+        double si = 0.0, di = 0.0;
+        if (kWave) {
+            const double x[3] = {xs[0][row], xs[1][row], xs[2][row]};
+            cplx w, g[3];
+            pair_integrals(x, p, k, kWave, !direct, tab, w, g);
+            const double n0 = direct ? p.n[0] : xs[3][row], n1 = direct ? p.n[1] : xs[4][row],
+                         n2 = direct ? p.n[2] : xs[5][row];
+            s += w.re;
+            si = -kInv4Pi * w.im;
+            d += n0 * g[0].re + n1 * g[1].re + n2 * g[2].re;
+            di = -kInv4Pi * (n0 * g[0].im + n1 * g[1].im + n2 * g[2].im);
         }
+        if (S) S[o] = make_double2(-kInv4Pi * s, si);
+        if (D) D[o] = make_double2((diag ? 0.5 : 0.0) - kInv4Pi * d, di);
     }
-}
+};
+struct RankineRealOut {
+    double *S, *D;
+    static __device__ __forceinline__ double take(double v) { return v; }
+    __device__ __forceinline__ void store(int64_t o, bool diag, double s, double d, const double (*)[kRkRows], int,
+                                          const Panel&) const
+    {
+        S[o] = -kInv4Pi * s;
+        D[o] = (diag ? 0.5 : 0.0) - kInv4Pi * d;
+    }
+};
 
 __device__ __forceinline__ void dof_at(const double* dof, int64_t dof_rows, int64_t n, int64_t i,
                                        double d[3])
@@ -153,11 +145,19 @@ k_force(const double* __restrict__ geom, int64_t n, const double2* __restrict__ 
 cudaError_t launch_assemble_f64(mh_ctx* ctx, const mh_mesh* m, double k, uint32_t mask, int direct,
                                 const double* tab, double2* S, double2* D)
 {
-    const int64_t n = m->n;
-    dim3 grid((unsigned)((n + kRows - 1) / kRows), (unsigned)((n + kCols - 1) / kCols));
-    k_assemble_f64<<<grid, kRows, 0, ctx->stream>>>(m->geom, n, k, mask, direct, tab, S, D);
-    ctx->launches += 1;
-    return cudaGetLastError();
+    const RankineGeom in{m->geom, m->n};
+    const auto go = [&](auto out) { return launch_rankine_tile<double>(ctx, in, m->n, mask, direct, out); };
+    switch (mask & (MH_GF_WU | MH_GF_DELHOMMEAU)) {
+        case 0: return go(AssembleOut<0>{S, D, tab, k, direct});
+        case MH_GF_WU: return go(AssembleOut<MH_GF_WU>{S, D, tab, k, direct});
+        case MH_GF_DELHOMMEAU: return go(AssembleOut<MH_GF_DELHOMMEAU>{S, D, tab, k, direct});
+        default: return go(AssembleOut<MH_GF_WU | MH_GF_DELHOMMEAU>{S, D, tab, k, direct});
+    }
+}
+
+cudaError_t launch_rankine_real(mh_ctx* ctx, const mh_mesh* m, uint32_t mask, int direct, double* SR, double* DR)
+{
+    return launch_rankine_tile<double>(ctx, RankineGeom{m->geom, m->n}, m->n, mask, direct, RankineRealOut{SR, DR});
 }
 
 cudaError_t launch_radiation_bc(mh_ctx* ctx, const mh_mesh* m, const double* dof, int64_t dof_rows,
