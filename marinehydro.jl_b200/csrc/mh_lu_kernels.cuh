@@ -23,6 +23,11 @@ __device__ __forceinline__ float2 cfms(float2 a, float2 b, float2 c)
 {
     return make_float2(a.x - (b.x * c.x - b.y * c.y), a.y - (b.x * c.y + b.y * c.x));
 }
+// the same as a chain of four fused operations
+__device__ __forceinline__ float2 cfms4(float2 a, float2 b, float2 c)
+{
+    return make_float2(fmaf(b.y, c.y, fmaf(-b.x, c.x, a.x)), fmaf(-b.y, c.x, fmaf(-b.x, c.y, a.y)));
+}
 __device__ __forceinline__ float2 cdivf(float2 a, float2 b)
 {
     float d = b.x * b.x + b.y * b.y;
@@ -116,230 +121,262 @@ k_lu_diag(float2* __restrict__ A, int64_t n, int64_t stride, int64_t k0, float2*
 // images (8-row x 16-byte core matrices), rows R < 64 = [Re v | -Im v],
 // rows 64 + R = [Im v | Re v] of the complex row v = column R of inv(U11)
 // (image 0, for L21 = A21 inv(U11)) or row R of inv(L11) (image 1, for
-// U12^T = A12^T inv(L11)^T).  x holds inv(L) strictly below the diagonal
-// (unit diagonal implicit) and inv(U) on and above it.
+// U12^T = A12^T inv(L11)^T).  x[c][r] (column-major) holds inv(L) strictly
+// below the diagonal (unit diagonal implicit) and inv(U) on and above it.
+// An item reads eight entries of v (as FP16 pairs Re, Im) and writes them to the
+// four places of its two rows.
 constexpr int kTrsmBImage = 128 * 128 * 2;  // bytes per image
 
 template <int LD>
-__device__ __forceinline__ void pack_trsm_b(const float2 (*x)[LD], unsigned char* img)
+__device__ __forceinline__ void pack_trsm_b(const __half2 (*x)[LD], unsigned char* img)
 {
-    for (int e = threadIdx.x; e < 2 * 128 * 16; e += blockDim.x) {
-        const int im = e / (128 * 16), R = (e / 16) % 128, cc = e % 16;
-        const int r = R & 63, t0 = (cc & 7) * 8;
-        float v[8];
+    if (threadIdx.x >= 256) return;
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+        const int e = it * 256 + threadIdx.x;
+        const int im = e >> 9, r = e & 63, cc = (e >> 6) & 7, t0 = cc * 8;
+        __half2 v[8];
+        const __half2 zero = __floats2half2_rn(0.f, 0.f), one = __floats2half2_rn(1.f, 0.f);
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const int t = t0 + q;
-            float2 z;
-            if (im == 0) z = t <= r ? x[t][r] : make_float2(0.f, 0.f);  // inv(U)[t][r]
-            else z = t == r ? make_float2(1.f, 0.f) : (r > t ? x[r][t] : make_float2(0.f, 0.f));  // inv(L)[r][t]
-            const bool im_row = R >= 64, second = cc >= 8;
-            v[q] = im_row ? (second ? z.x : z.y) : (second ? -z.y : z.x);
+            if (im == 0) v[q] = t <= r ? x[r][t] : zero;                // inv(U)[t][r]
+            else v[q] = t == r ? one : (r > t ? x[t][r] : zero);        // inv(L)[r][t]
         }
-        uint4 w;
-        __half2 h0 = __floats2half2_rn(v[0], v[1]), h1 = __floats2half2_rn(v[2], v[3]);
-        __half2 h2 = __floats2half2_rn(v[4], v[5]), h3 = __floats2half2_rn(v[6], v[7]);
-        w.x = *reinterpret_cast<uint32_t*>(&h0);
-        w.y = *reinterpret_cast<uint32_t*>(&h1);
-        w.z = *reinterpret_cast<uint32_t*>(&h2);
-        w.w = *reinterpret_cast<uint32_t*>(&h3);
-        const uint32_t off = (uint32_t)((cc * 16 + R / 8) * 128 + (R % 8) * 16);
-        *reinterpret_cast<uint4*>(img + (size_t)im * kTrsmBImage + off) = w;
+        uint4 re, pi;  // Re v, Im v
+        auto bits = [](__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); };
+        auto lo = [&](int q) { return bits(__lows2half2(v[q], v[q + 1])); };
+        auto hi = [&](int q) { return bits(__highs2half2(v[q], v[q + 1])); };
+        re = make_uint4(lo(0), lo(2), lo(4), lo(6));
+        pi = make_uint4(hi(0), hi(2), hi(4), hi(6));
+        const uint4 mi = make_uint4(pi.x ^ 0x80008000u, pi.y ^ 0x80008000u, pi.z ^ 0x80008000u, pi.w ^ 0x80008000u);
+        unsigned char* o = img + (size_t)im * kTrsmBImage;
+        auto at = [&](int row, int chunk) {
+            return reinterpret_cast<uint4*>(o + ((chunk * 16 + row / 8) * 128 + (row % 8) * 16));
+        };
+        *at(r, cc) = re;
+        *at(r, 8 + cc) = mi;
+        *at(64 + r, cc) = pi;
+        *at(64 + r, 8 + cc) = re;
     }
 }
 
-// k_lu_diag for NB = 64, blocked by eight columns in shared memory: for each
-// panel P of columns 8P .. 8P+7, (1) one warp factors the panel (rows 8P ..
-// 63, two rows per lane, the pivot row passed by warp shuffles: no CTA
-// barrier inside the panel), (2) the panel's block row of U right of it is
-// solved with the panel's unit-lower 8 x 8 L, one column per thread, (3)
-// every thread applies the rank-8 update to its part of the trailing block:
-// three barriers per panel, 24 in all instead of one per column.  The
-// two triangular inverses are then built by recursive doubling from the
-// factored block in shared memory: with the inverses of the diagonal blocks
-// A and C of size s known, [A 0; B C]^-1 has the off-diagonal block
-// -inv(C) B inv(A) (and [A B; 0 C]^-1 has -inv(A) B inv(C)), two small
-// products per level, s = 1, 2, ..., 32: twelve barriers instead of one per
-// row.  The block is padded with the identity, so all 64 steps run for any
-// kb <= 64 and the padding stays the identity.  Same outputs as k_lu_diag.
-constexpr int kDiag64Threads = 512;
-// dynamic shared memory: the factored block, the inverses (inv(L) strictly
-// below the diagonal, inv(U) on and above), two product buffers
-constexpr int kDiagLd = 65;
-constexpr size_t kDiag64Smem = sizeof(float2) * (2 * 64 * kDiagLd + 2 * 32 * 32 * 2);
+// k_lu_diag for NB = 64: factors and both triangular inverses in one blocked
+// elimination, the whole block in registers.  A step takes the eight rows and
+// columns K of a panel.  With the pivot block X_KK = L_K U_K,
+//   c_iK = X_iK inv(U_K)  for every row i outside K: L below K, and above K
+//                         the final columns K of inv(U);
+//   R_Kj = inv(L_K) X_Kj  for every column j outside K: U right of K, and left
+//                         of K the final rows K of inv(L).
+// These four pieces leave for their places at once, and the step is one
+// rank-8 update X_ij -= c_iK R_Kj of all entries, rows and columns in K
+// starting from 0 with c = inv(U_K) and R = inv(L_K) there: below and right of
+// K it makes the Schur complement, below and left what inv(L) needs, above and
+// right what inv(U) needs; what it makes of the entries that have left is never
+// read.  The pivot block is factored and inverted by the same elimination, one
+// pivot at a time.
+// Thread (ti, tj) of 16 x 16 holds the entries (ti + 16 a, tj + 16 b); a ninth
+// warp does the pivot blocks (two entries per lane, exchanged by shuffles), the
+// next panel's while the others run this panel's update: they hand its eight
+// rows and columns over first.  What bounds it: the 64 dependent pivot steps (a
+// shuffle, a reciprocal and three products each), one CTA per matrix.
+// The panel loop is not unrolled: with the panel as a compile-time index the
+// code, run once, missed the instruction cache for a third of the time.
+// The block is padded with the identity, so all panels run for any kb <= 64.
+// Same outputs as k_lu_diag.  28 KB of shared memory, so that a CTA fits beside
+// two CTAs of the trailing update on an SM.
+// Measured on a B200: 44 us (panels of eight by one warp, then the inverses by
+// recursive doubling: 36 barriers) -> 26 us a block; 64 matrices of 2048 beside
+// their updates, 60 -> 39 us.
+constexpr int kDiag64Threads = 288;
 
 __global__ void __launch_bounds__(kDiag64Threads)
 k_lu_diag64(float2* __restrict__ A, int64_t n, int64_t stride, int64_t k0, float2* __restrict__ Dinv,
             int64_t dstride, int* __restrict__ bad, unsigned char* __restrict__ bimg, int64_t bstride)
 {
-    constexpr int NB = 64;
-    extern __shared__ float2 diag_smem[];
-    auto f = reinterpret_cast<float2 (*)[kDiagLd]>(diag_smem);                 // factored block
-    auto x = reinterpret_cast<float2 (*)[kDiagLd]>(diag_smem + NB * kDiagLd);  // the two inverses
-    float2* tl_buf = diag_smem + 2 * NB * kDiagLd;                               // products
-    float2* tu_buf = tl_buf + 2 * 32 * 32;
-    const int64_t b = blockIdx.x;
-    float2* M = A + b * stride;
+    constexpr int NB = 64, kLd = 65, kPad = NB + 1;  // odd leading dimensions: no bank conflicts down a column
+    __shared__ float2 c[8][kPad];  // c[m][i]: X_iK, then c_iK (row i in K: inv(U_K))
+    __shared__ float2 r[8][kPad];  // r[m][j]: X_Kj, then R_Kj (column j in K: inv(L_K))
+    __shared__ __align__(16) float2 iu[8][8];  // iu[t][m] = inv(U_K)[t][m], zero for t > m
+    __shared__ __align__(16) float2 il[8][8];  // il[t][m] = inv(L_K)[m][t], 1 for t = m, zero for t > m
+    __shared__ float2 pv[8][8];                // the next pivot block
+    __shared__ float2 prow[8][8], pcol[8][8];  // its row k before step k, c of step k
+    __shared__ __half2 hx[NB][kLd];            // hx[col][row]: the inverses as FP16 pairs
+    const int64_t b0 = blockIdx.x;
+    float2* M = A + b0 * stride + k0 * n + k0;
+    float2* invL = Dinv + b0 * dstride + (k0 / NB) * 2 * NB * NB;
+    float2* invU = invL + NB * NB;
     const int kb = (int)min((int64_t)NB, n - k0);
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    // the block, padded with the identity past kb, column by column (coalesced)
-    for (int e = t; e < NB * NB; e += blockDim.x) {
-        const int c = e / NB, r = e % NB;
-        f[r][c] = (r < kb && c < kb) ? M[(k0 + c) * n + k0 + r] : make_float2(r == c ? 1.f : 0.f, 0.f);
+    const int tid = threadIdx.x, ti = tid & 15, tj = tid >> 4, lane = tid & 31;
+    const bool pivots = tid >= 256;  // the ninth warp
+    const float2 z = make_float2(0.f, 0.f), one = make_float2(1.f, 0.f);
+    float2 X[4][4];
+    if (!pivots) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                const int i = ti + 16 * a, j = tj + 16 * b;
+                X[a][b] = (i < kb && j < kb) ? M[(int64_t)j * n + i] : i == j ? one : z;
+                if (i < j) invL[j * NB + i] = z;
+                if (i > j) invU[j * NB + i] = z;
+            }
+        if (ti < 8 && tj < 8) pv[ti][tj] = X[0][0];
     }
+    bool poor = false;
     __syncthreads();
 #pragma unroll 1
-    for (int P = 0; P < NB / 8; ++P) {
-        const int p0 = 8 * P;
-        // (1) panel: lane l holds rows p0 + l and p0 + l + 32 (when < 64)
-        if (warp == 0) {
-            const int ra = p0 + lane, rb = ra + 32;
-            const bool has_a = ra < NB, has_b = rb < NB;
-            float2 va[8], vb[8];
+    for (int K = -8; K < NB; K += 8) {
+        if (pivots) {
+            const int N = K + 8;  // the panel after K
+            if (N < NB) {
+                // lane (i, g) holds the entries (i, g) and (i, g + 4) of the pivot block
+                const int i = lane & 7, g = lane >> 3;
+                float2 x[2] = {pv[i][g], pv[i][4 + g]};
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                va[j] = has_a ? f[ra][p0 + j] : make_float2(0.f, 0.f);
-                vb[j] = has_b ? f[rb][p0 + j] : make_float2(0.f, 0.f);
+                for (int k = 0; k < 8; ++k) {
+                    const int ek = k >> 2, gk = k & 3;
+                    auto from = [](float2 v, int src) {
+                        return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+                    };
+                    const float2 p = from(x[ek], 8 * gk + k), xk = from(x[ek], 8 * gk + i);
+                    float2 pr[2] = {from(x[0], 8 * g + k), from(x[1], 8 * g + k)};
+                    const float mag = fmaf(p.x, p.x, p.y * p.y);
+                    const float im2 = 1.f / mag;
+                    const float2 ip = make_float2(p.x * im2, -p.y * im2);
+                    float2 ck = cmulf(xk, ip);
+                    ck.x = i == k ? ip.x : ck.x;
+                    ck.y = i == k ? ip.y : ck.y;
+                    pcol[k][i] = ck;
+                    if (i == k) {
+                        prow[k][g] = x[0];
+                        prow[k][g + 4] = x[1];
+                    }
+                    const bool own = g == gk;  // column k itself: 0 - c
+                    pr[ek].x = own ? 1.f : pr[ek].x;
+                    pr[ek].y = own ? 0.f : pr[ek].y;
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const bool zero = i == k || (e == ek && own);
+                        x[e].x = zero ? 0.f : x[e].x;
+                        x[e].y = zero ? 0.f : x[e].y;
+                        x[e] = cfms4(x[e], ck, pr[e]);
+                    }
+                }
+                __syncwarp();
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int j = g + 4 * e;
+                    const float2 pc = pcol[j][i], pw = prow[i][j];  // i > j: L, inv(L); i <= j: inv(U), U
+                    iu[i][j] = i <= j ? pc : z;
+                    il[j][i] = i > j ? pw : i == j ? one : z;
+                    if (N + i < kb && N + j < kb) M[(int64_t)(N + j) * n + N + i] = i > j ? pc : pw;
+                    const float2 inv = i > j ? pw : pc;
+                    (i > j ? invL : invU)[(N + j) * NB + N + i] = inv;
+                    if (i == j) {
+                        const float mag = fmaf(pw.x, pw.x, pw.y * pw.y);  // the pivot
+                        poor = poor || (N + i < kb && !(mag > 1e-30f && mag < 3e38f));
+                        invL[(N + j) * NB + N + i] = one;
+                    }
+                    hx[N + j][N + i] = __floats2half2_rn(inv.x, inv.y);
+                }
             }
+        } else if (K >= 0) {
+#pragma unroll 2
+            for (int m = 0; m < 8; ++m) {
+                float2 cv[4], rv[4];
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                // pivot row p0 + c is lane c's first row
-                float2 pr[8];
-#pragma unroll
-                for (int j = c; j < 8; ++j)
-                    pr[j] = make_float2(__shfl_sync(0xffffffffu, va[j].x, c), __shfl_sync(0xffffffffu, va[j].y, c));
-                const float2 piv = pr[c];
-                if (lane == c && p0 + c < kb) {
-                    const float mag = piv.x * piv.x + piv.y * piv.y;
-                    if (!(mag > 1e-30f && mag < 3e38f)) atomicExch(bad + b, 1);
+                for (int a = 0; a < 4; ++a) {
+                    cv[a] = c[m][ti + 16 * a];
+                    rv[a] = r[m][tj + 16 * a];
                 }
-                // 1 / piv once per step (one division), then products
-                const float im2 = 1.f / (piv.x * piv.x + piv.y * piv.y);
-                const float2 ip = make_float2(piv.x * im2, -piv.y * im2);
-                if (has_a && ra > p0 + c) {
-                    const float2 l = make_float2(va[c].x * ip.x - va[c].y * ip.y, va[c].x * ip.y + va[c].y * ip.x);
-                    va[c] = l;
 #pragma unroll
-                    for (int j = c + 1; j < 8; ++j) va[j] = cfms(va[j], l, pr[j]);
-                }
-                if (has_b) {  // rb >= 32 > p0 + c for every panel with rows past 32
-                    const float2 l = make_float2(vb[c].x * ip.x - vb[c].y * ip.y, vb[c].x * ip.y + vb[c].y * ip.x);
-                    vb[c] = l;
+                for (int b = 0; b < 4; ++b)
 #pragma unroll
-                    for (int j = c + 1; j < 8; ++j) vb[j] = cfms(vb[j], l, pr[j]);
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (has_a) f[ra][p0 + j] = va[j];
-                if (has_b) f[rb][p0 + j] = vb[j];
-            }
-        }
-        __syncthreads();
-        const int q0 = p0 + 8;  // first column (and row) past the panel
-        if (q0 >= NB) break;
-        // (2) U block row: rows p0 .. p0+7, columns q0 .. 63, by the panel's unit-lower L
-        if (t < NB - q0) {
-            const int cq = q0 + t;
-            float2 u[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) u[i] = f[p0 + i][cq];
-#pragma unroll
-            for (int i = 1; i < 8; ++i)
-#pragma unroll
-                for (int k2 = 0; k2 < i; ++k2) u[i] = cfms(u[i], f[p0 + i][p0 + k2], u[k2]);
-#pragma unroll
-            for (int i = 1; i < 8; ++i) f[p0 + i][cq] = u[i];
-        }
-        __syncthreads();
-        // (3) rank-8 update of rows and columns q0 .. 63: thread t takes row
-        // q0 + t / 8 and the columns q0 + t % 8 + 8 j
-        {
-            const int r = q0 + (t >> 3), g = t & 7;
-            if (r < NB) {
-                float2 lr[8];
-#pragma unroll
-                for (int k2 = 0; k2 < 8; ++k2) lr[k2] = f[r][p0 + k2];
-                for (int cq = q0 + g; cq < NB; cq += 8) {
-                    float2 acc = f[r][cq];
-#pragma unroll
-                    for (int k2 = 0; k2 < 8; ++k2) acc = cfms(acc, lr[k2], f[p0 + k2][cq]);
-                    f[r][cq] = acc;
-                }
+                    for (int a = 0; a < 4; ++a) X[a][b] = cfms4(X[a][b], cv[a], rv[b]);
             }
         }
+        if (K + 8 >= NB) break;
+        __syncthreads();  // c and r are read; the next pivot block's inverses are there
+        const int N = K + 8;
+        // a thread holds row N + (ti & 7) in a = nq, column N + (tj & 7) in b = nq
+        const int nq = N >> 4, h = (N >> 3) & 1;
+        const bool row_n = !pivots && (ti >> 3) == h, col_n = !pivots && (tj >> 3) == h;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (q == nq) {
+                if (row_n)
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) r[ti & 7][tj + 16 * b] = X[q][b];
+                if (col_n)
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) c[tj & 7][ti + 16 * a] = X[a][q];
+            }
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+                if ((a == nq && row_n) || (b == nq && col_n)) X[a][b] = z;
         __syncthreads();
+        // c (threads 0 .. 127) and R (128 .. 255): index eq, entries 4 mh .. 4 mh + 3, in place (a pair of lanes per index)
+        const int eq = (tid >> 1) & 63, mh = tid & 1;
+        const bool is_c = tid < 128;
+        float2 acc[4] = {z, z, z, z};
+        if (!pivots) {
+            float2 (*v)[kPad] = is_c ? c : r;
+            const float4* tab = reinterpret_cast<const float4*>(is_c ? &iu[0][0] : &il[0][0]) + 2 * mh;
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+                const float2 x = make_float2(-v[t][eq].x, -v[t][eq].y);
+                const float4 u0 = tab[4 * t], u1 = tab[4 * t + 1];
+                acc[0] = cfms4(acc[0], x, make_float2(u0.x, u0.y));
+                acc[1] = cfms4(acc[1], x, make_float2(u0.z, u0.w));
+                acc[2] = cfms4(acc[2], x, make_float2(u1.x, u1.y));
+                acc[3] = cfms4(acc[3], x, make_float2(u1.z, u1.w));
+            }
+            __syncwarp();
+            if ((eq & ~7) == N) {  // in the panel: the operand itself
+                const float4 u0 = tab[4 * (eq & 7)], u1 = tab[4 * (eq & 7) + 1];
+                acc[0] = make_float2(u0.x, u0.y);
+                acc[1] = make_float2(u0.z, u0.w);
+                acc[2] = make_float2(u1.x, u1.y);
+                acc[3] = make_float2(u1.z, u1.w);
+            }
+#pragma unroll
+            for (int s = 0; s < 4; ++s) v[4 * mh + s][eq] = acc[s];
+        }
+        __syncthreads();
+        // the pivot block after this panel, updated ahead of the rest
+        const int P = N + 8;
+        if (!pivots && P < NB && (ti >> 3) == ((P >> 3) & 1) && (tj >> 3) == ((P >> 3) & 1)) {
+            const int pq = P >> 4;
+            float2 x = pq == 0 ? X[0][0] : pq == 1 ? X[1][1] : pq == 2 ? X[2][2] : X[3][3];
+#pragma unroll
+            for (int m = 0; m < 8; ++m) x = cfms4(x, c[m][ti + 16 * pq], r[m][tj + 16 * pq]);
+            pv[ti & 7][tj & 7] = x;
+        }
+        __syncthreads();
+        if (!pivots && (eq & ~7) != N) {
+            // c and R to their places while the next pivot block is factored: past the panel the factors (L by
+            // columns, U by rows), before it the inverses
+            const bool past = eq >= N + 8;
+            const int nin = N + 4 * mh;
+            float2* out = past ? (is_c ? M + (int64_t)nin * n + eq : M + (int64_t)eq * n + nin)
+                               : (is_c ? invU + nin * NB + eq : invL + eq * NB + nin);
+            const int64_t step = is_c ? (past ? n : (int64_t)NB) : 1;
+            const int live = !past ? 4 : eq < kb ? min(4, kb - nin) : 0;
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+                if (s < live) out[s * step] = acc[s];
+            if (!past)
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+                    (is_c ? hx[nin + s][eq] : hx[eq][nin + s]) = __floats2half2_rn(acc[s].x, acc[s].y);
+        }
     }
-    // the factors back over the block (coalesced)
-    for (int e = t; e < NB * NB; e += blockDim.x) {
-        const int c = e / NB, r = e % NB;
-        if (r < kb && c < kb) M[(k0 + c) * n + k0 + r] = f[r][c];
-    }
+    if (poor) atomicExch(bad + b0, 1);
     __syncthreads();
-    // inverses by recursive doubling; x starts as the inverse diagonal of U
-    for (int e = t; e < NB * NB; e += blockDim.x) {
-        const int i = e / NB, j = e % NB;
-        x[i][j] = i == j ? cdivf(make_float2(1.f, 0.f), f[i][i]) : make_float2(0.f, 0.f);
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int lsz = 0; (1 << lsz) < NB; ++lsz) {  // block size sz = 2^lsz: index arithmetic by shifts
-        const int sz = 1 << lsz;
-        const int items = (NB / (2 * sz)) * sz * sz;  // outputs per triangle and phase
-        // phase 1: -L[C,A] inv(L)[A,A] and -U[A,C] inv(U)[C,C]
-        for (int e = t; e < 2 * items; e += blockDim.x) {
-            const bool up = e >= items;
-            const int ee = up ? e - items : e;
-            const int pr = ee >> (2 * lsz), i = (ee >> lsz) & (sz - 1), j = ee & (sz - 1);
-            const int a0 = 2 * sz * pr, c0 = a0 + sz;
-            float2 acc = make_float2(0.f, 0.f);
-            if (!up) {  // row c0 + i, column a0 + j; inv(L) is 1 on the diagonal
-                for (int u = j; u < sz; ++u) {
-                    const float2 xl = u == j ? make_float2(1.f, 0.f) : x[a0 + u][a0 + j];
-                    acc = cfms(acc, f[c0 + i][a0 + u], xl);
-                }
-                tl_buf[ee] = acc;
-            } else {  // row a0 + i, column c0 + j; inv(U)[u][j] for u <= j
-                for (int u = 0; u <= j; ++u) acc = cfms(acc, f[a0 + i][c0 + u], x[c0 + u][c0 + j]);
-                tu_buf[ee] = acc;
-            }
-        }
-        __syncthreads();
-        // phase 2: inv(L)[C,A] = inv(L)[C,C] (phase 1), inv(U)[A,C] = inv(U)[A,A] (phase 1)
-        for (int e = t; e < 2 * items; e += blockDim.x) {
-            const bool up = e >= items;
-            const int ee = up ? e - items : e;
-            const int pr = ee >> (2 * lsz), i = (ee >> lsz) & (sz - 1), j = ee & (sz - 1);
-            const int a0 = 2 * sz * pr, c0 = a0 + sz;
-            const float2* T = (up ? tu_buf : tl_buf) + pr * sz * sz;
-            float2 acc = make_float2(0.f, 0.f);
-            if (!up) {  // inv(L)[c0+i][c0+u] for u <= i (1 on the diagonal)
-                for (int u = 0; u <= i; ++u) {
-                    const float2 xl = u == i ? make_float2(1.f, 0.f) : x[c0 + i][c0 + u];
-                    const float2 tv = T[u * sz + j];
-                    acc.x += xl.x * tv.x - xl.y * tv.y;
-                    acc.y += xl.x * tv.y + xl.y * tv.x;
-                }
-                x[c0 + i][a0 + j] = acc;
-            } else {  // inv(U)[a0+i][a0+u] for u >= i
-                for (int u = i; u < sz; ++u) {
-                    const float2 xu = x[a0 + i][a0 + u];
-                    const float2 tv = T[u * sz + j];
-                    acc.x += xu.x * tv.x - xu.y * tv.y;
-                    acc.y += xu.x * tv.y + xu.y * tv.x;
-                }
-                x[a0 + i][c0 + j] = acc;
-            }
-        }
-        __syncthreads();
-    }
-    float2* out = Dinv + b * dstride + (k0 / NB) * 2 * NB * NB;
-    for (int e = t; e < NB * NB; e += blockDim.x) {
-        const int c = e / NB, rr = e % NB;
-        out[e] = rr == c ? make_float2(1.f, 0.f) : (rr > c ? x[rr][c] : make_float2(0.f, 0.f));
-        out[NB * NB + e] = rr <= c ? x[rr][c] : make_float2(0.f, 0.f);
-    }
-    if (bimg) pack_trsm_b<kDiagLd>(x, bimg + b * bstride + (k0 / NB) * 2 * kTrsmBImage);
+    if (bimg) pack_trsm_b<kLd>(hx, bimg + b0 * bstride + (k0 / NB) * 2 * kTrsmBImage);
 }
 
 // blockIdx.y == 0: rows of L21 = A21 U11^-1; blockIdx.y == 1: columns of

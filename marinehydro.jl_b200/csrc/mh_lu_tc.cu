@@ -3,8 +3,9 @@
 //
 // Panels of NB = 64 complex columns, trailing updates every two panels (one
 // 128-wide tile).  Per panel k0:
-//   k_lu_diag64        factor the 64 x 64 diagonal block (registers, one
-//                      barrier per elimination step), store inv(L11), inv(U11);
+//   k_lu_diag64        factor the 64 x 64 diagonal block and form inv(L11),
+//                      inv(U11) in the same elimination (registers, one
+//                      barrier per step);
 //   k_lu_trsm_tc       L21 = A21 inv(U11) and U12^T = A12^T inv(L11)^T as
 //                      tcgen05 GEMMs (M=128, N=128, K=128); writes the FP32
 //                      factors into the matrix and the FP16 operand panels of
@@ -1954,7 +1955,7 @@ cudaError_t lu_tc_group(mh_ctx* ctx, float2* A, int64_t n, int64_t stride, int n
         return cudaGetLastError();
     };
     auto strip_join = [&]() { return cudaStreamWaitEvent(main_s, st.ev_strip_done, 0); };
-    k_lu_diag64<<<nbatch, kDiag64Threads, kDiag64Smem, main_s>>>(A, n, stride, 0, Dinv, dstride, bad, bimg,
+    k_lu_diag64<<<nbatch, kDiag64Threads, 0, main_s>>>(A, n, stride, 0, Dinv, dstride, bad, bimg,
                                                                    bstride);
     ctx->launches += 1;
     int outer = 0;
@@ -2001,7 +2002,7 @@ cudaError_t lu_tc_group(mh_ctx* ctx, float2* A, int64_t n, int64_t stride, int n
                     q.U[np] = pp.U[r];
                 }
                 if ((e = strip(t0, nt, 1, q, np, k + TC_NB)) != cudaSuccess) return e;
-                k_lu_diag64<<<nbatch, kDiag64Threads, kDiag64Smem, main_s>>>(A, n, stride, k + TC_NB, Dinv, dstride,
+                k_lu_diag64<<<nbatch, kDiag64Threads, 0, main_s>>>(A, n, stride, k + TC_NB, Dinv, dstride,
                                                                            bad, bimg, bstride);
                 ctx->launches += 1;
             }
@@ -2032,7 +2033,7 @@ cudaError_t lu_tc_group(mh_ctx* ctx, float2* A, int64_t n, int64_t stride, int n
         prev = pp;
         nprev = op;
         if (lo < n) {
-            k_lu_diag64<<<nbatch, kDiag64Threads, kDiag64Smem, main_s>>>(A, n, stride, lo, Dinv, dstride, bad,
+            k_lu_diag64<<<nbatch, kDiag64Threads, 0, main_s>>>(A, n, stride, lo, Dinv, dstride, bad,
                                                                          bimg, bstride);
             ctx->launches += 1;
         }
@@ -2069,9 +2070,6 @@ cudaError_t launch_lu_tc(mh_ctx* ctx, float2* A, int64_t n, int64_t stride, int 
         return e;
     if ((e = cudaFuncSetAttribute(k_lu_trsm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(kSmemA + kSmemA))) != cudaSuccess)
-        return e;
-    if ((e = cudaFuncSetAttribute(k_lu_diag64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)kDiag64Smem)) != cudaSuccess)
         return e;
     const int groups = std::min(sched.groups, nbatch);
     const int64_t dstride = lu_dinv_stride_tc(n);
