@@ -24,34 +24,15 @@
 #include "mh_device.cuh"
 #include "mh_internal.h"
 #include "mh_rankine.cuh"
+#include "mh_rings.cuh"
+#include "mh_wave.cuh"
 
 namespace mh {
 namespace {
 
 constexpr int kRows = 128;
-constexpr int kCols = 16;
-constexpr double kInv4Pi = 1.0 / (4.0 * kPi);
 constexpr size_t kBatchBytes = 16ull << 30;  // device memory budget of one frequency chunk
 constexpr int kAllwMinFreqs = 6;  // chunks this large use the frequency-batched Delhommeau pass
-
-__device__ __forceinline__ void load_panel_field(Panel& p, int f, double v)
-{
-    if (f < 3) p.c[f] = v;
-    else if (f < 6) p.n[f - 3] = v;
-    else if (f == G_AREA) p.area = v;
-    else if (f == G_RADIUS) p.radius = v;
-    else p.v[f - G_V] = v;
-}
-
-__device__ __forceinline__ void stage_panels(Panel* sp, const double* __restrict__ geom, int64_t n,
-                                             int64_t j0, int cols)
-{
-    for (int t = threadIdx.x; t < cols * G_NFIELDS; t += blockDim.x) {
-        int f = t / cols, jj = t % cols;
-        int64_t j = j0 + jj;
-        load_panel_field(sp[jj], f, (j < n) ? geom[(int64_t)f * n + j] : 0.0);
-    }
-}
 
 // Per frequency z = blockIdx.z: S = SR + wave, D = DR + wave, written as FP64
 // complex (S64, D64) and the FP32 LU copy of D (Dlo).
@@ -107,50 +88,12 @@ k_wave_batch(const double* __restrict__ geom, int64_t n, int direct, int cols, c
 // transcendental calls; the log term splits as log(k) + log((d + |zeta|)/2).
 // The series in R use the table's monomial-in-u copy (Horner's rule, four
 // frequencies per pass).
-// Frequencies at which the pair leaves the polar patch use the full table.
+// Frequencies at which the pair leaves the polar patch use the table's rings.
 // Same arithmetic as wave_pair<true> up to reassociation (~1e-16).
-// One pair of the frequency-batched pass and its output: S, D (FP64 and the
-// FP32 copy of D) and the tape of frequency z from the dimensionless
-// (G, G_r, G_z) in o3.
-struct AllwPair {
-    double dx, dy, rho, inv_rho, area, sr, dr;
-    double n0, n1, n2;  // the normal of D (source panel when direct), held in registers
-    int64_t o;          // pair offset j * n + i
-    bool wrt_first;
-};
-
-__device__ __forceinline__ void allw_emit(const AllwPair& q, int z, double k, const cplx o3[3], int64_t nn,
-                                          double2* __restrict__ S64, double2* __restrict__ D64,
-                                          float2* __restrict__ Dlo, double2* __restrict__ tape)
-{
-    const double r = k * q.rho;
-    double d1 = 0.0, d2 = 0.0;
-    if (fabs(r) > 1e-6) {
-        const double f = k * q.inv_rho;  // k^2 / r
-        d1 = q.wrt_first ? f * q.dx : -f * q.dx;
-        d2 = q.wrt_first ? f * q.dy : -f * q.dy;
-    }
-    const double ka = k * q.area;
-    const cplx s = ka * o3[0];
-    const cplx g0 = (ka * d1) * o3[1], g1 = (ka * d2) * o3[1], g2 = (ka * k) * o3[2];
-    const double Sr = q.sr - kInv4Pi * s.re, Si = -kInv4Pi * s.im;
-    const double Dr = q.dr - kInv4Pi * (q.n0 * g0.re + q.n1 * g1.re + q.n2 * g2.re);
-    const double Di = -kInv4Pi * (q.n0 * g0.im + q.n1 * g1.im + q.n2 * g2.im);
-    const int64_t m = (int64_t)z * nn + q.o;
-    S64[m] = make_double2(Sr, Si);
-    D64[m] = make_double2(Dr, Di);
-    Dlo[m] = make_float2((float)Dr, (float)Di);
-    if (tape) {  // (G, G_r) for the adjoint of the same call
-        tape[2 * m] = make_double2(o3[0].re, o3[0].im);
-        tape[2 * m + 1] = make_double2(o3[1].re, o3[1].im);
-    }
-}
-
 // The four polar functions' monomial-in-u coefficients in constant memory:
 // every lane of the alpha contraction reads the same coefficient, which the
-// constant cache broadcasts.  Copied from the context's table before each
-// launch; every context builds the same table, so concurrent copies write
-// identical bytes.
+// constant cache broadcasts.  Written when a context builds its table; every
+// context builds the same one, so a later copy writes identical bytes.
 __constant__ double c_polar_mono[4 * kTabPolarFn];
 // The same coefficients rounded to FP32 (the FP32 alpha contraction).
 __constant__ float c_polar_mono_f[4 * kTabPolarFn];
@@ -163,7 +106,6 @@ template <>
 __device__ __forceinline__ float polar_coef<float>(int i) { return c_polar_mono_f[i]; }
 
 constexpr int kWT = 128;  // threads (rows) per CTA of k_wave_delh_allw
-constexpr int kAllwMaxFreqs = 128;  // frequencies per launch of k_wave_delh_allw
 // k, log k and 1/k per frequency, then the contracted series of every row
 // in the type HT of the per-frequency Horner pass (the polar coefficients
 // are read from constant memory)
@@ -173,12 +115,6 @@ constexpr size_t wave_allw_smem()
     return sizeof(double) * 3 * kAllwMaxFreqs + sizeof(HT) * 4 * kTabNU * kWT;
 }
 constexpr size_t kWaveAllwSmem = wave_allw_smem<double>();
-
-__global__ void k_coef_to_f32(const double* __restrict__ a, float* __restrict__ b, int count)
-{
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < count) b[t] = (float)a[t];
-}
 
 __device__ __forceinline__ double hfma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float hfma(float a, float b, float c) { return fmaf(a, b, c); }
@@ -261,8 +197,8 @@ k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, int col
                          direct ? p.n[2] : ni[2], o, wrt_first};
         // four frequencies per Horner pass: each coefficient read from shared
         // memory feeds four recurrences.  Frequencies off the polar patch are
-        // only counted here: k_wave_delh_allw_rest evaluates them with the
-        // full table, so this kernel makes no out-of-line call (whose calling
+        // only noted here: k_wave_delh_ring evaluates them with the
+        // table's rings, so this kernel makes no out-of-line call (whose calling
         // convention would cost spills on the hot path)
         constexpr int kZP = 4;
         int nfall = 0;
@@ -322,48 +258,48 @@ k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, int col
     }
 }
 
-// The frequencies k_wave_delh_allw left to the full table (pairs above the
-// free surface or at R = k d >= 2); exits at once when it flagged none.  The
-// test takes a margin of 1e-12 in R so that a pair on the patch edge is
-// written by one kernel at least, whatever the rounding of d in each (a pair
-// written by both gets this kernel's value, which runs second).
+// The frequencies the rings do not reach either (pairs above the free surface
+// or at R = k d >= 16), by the full table and the quadrature; exits at once
+// when k_wave_delh_rings flagged none.
 __global__ void __launch_bounds__(kWT)
 k_wave_delh_allw_rest(const int* __restrict__ fall, const double* __restrict__ geom, int64_t n, int direct, int cols,
                       const double* __restrict__ tab, const double* __restrict__ kvec, int nb,
                       const double* __restrict__ SR, const double* __restrict__ DR, double2* __restrict__ S64,
                       double2* __restrict__ D64, float2* __restrict__ Dlo, double2* __restrict__ tape)
 {
-    if (*fall == 0) return;
+    if (fall[kRings] == 0) return;
     __shared__ Panel sp[kCols];
-    const int64_t j0 = (int64_t)blockIdx.y * cols;
-    stage_panels(sp, geom, n, j0, cols);
-    __syncthreads();
     const int64_t i = (int64_t)blockIdx.x * kWT + threadIdx.x;
-    if (i >= n) return;
-    const int64_t nn = n * n;
-    const double x[3] = {geom[G_CX * n + i], geom[G_CY * n + i], geom[G_CZ * n + i]};
-    const double ni[3] = {geom[G_NX * n + i], geom[G_NY * n + i], geom[G_NZ * n + i]};
-    const int jend = (int)min((int64_t)cols, n - j0);
-    for (int jj = 0; jj < jend; ++jj) {
-        const Panel& p = sp[jj];
-        const int64_t o = (j0 + jj) * n + i;
-        const double dx = x[0] - p.c[0], dy = x[1] - p.c[1];
-        const double dis2 = dx * dx + dy * dy;
-        const double purt = 1e-18;
-        const double rho = (dis2 == 0.0) ? sqrt(dis2 + purt * purt) - purt : sqrt(dis2);
-        const double zeta = x[2] + p.c[2];
-        const double d = hypot(rho, zeta);
-        const bool polar_ok = -zeta >= 0.0;
-        const double* nn3 = direct ? p.n : ni;
-        const AllwPair q{dx, dy, rho, rho > 0.0 ? 1.0 / rho : 0.0, p.area, SR[o], DR[o], nn3[0], nn3[1], nn3[2], o,
-                         !direct};
-#pragma unroll 1
-        for (int z = 0; z < nb; ++z) {
-            const double k = kvec[z];
-            if (polar_ok && k * d < kTabRPolar * (1.0 - 1e-12)) continue;
-            cplx o3[3];
-            delh_dimless_table(tab, k * rho, k * zeta, o3);
-            allw_emit(q, z, k, o3, nn, S64, D64, Dlo, tape);
+    for (int64_t j0 = (int64_t)blockIdx.y * cols; j0 < n; j0 += (int64_t)gridDim.y * cols) {
+        __syncthreads();  // the last columns are read
+        stage_panels(sp, geom, n, j0, cols);
+        __syncthreads();
+        if (i >= n) continue;
+        const int64_t nn = n * n;
+        const double x[3] = {geom[G_CX * n + i], geom[G_CY * n + i], geom[G_CZ * n + i]};
+        const double ni[3] = {geom[G_NX * n + i], geom[G_NY * n + i], geom[G_NZ * n + i]};
+        const int jend = (int)min((int64_t)cols, n - j0);
+        for (int jj = 0; jj < jend; ++jj) {
+            const Panel& p = sp[jj];
+            const int64_t o = (j0 + jj) * n + i;
+            const double dx = x[0] - p.c[0], dy = x[1] - p.c[1];
+            const double dis2 = dx * dx + dy * dy;
+            const double purt = 1e-18;
+            const double rho = (dis2 == 0.0) ? sqrt(dis2 + purt * purt) - purt : sqrt(dis2);
+            const double zeta = x[2] + p.c[2];
+            const double d = hypot(rho, zeta);
+            const bool polar_ok = -zeta >= 0.0;
+            const double* nn3 = direct ? p.n : ni;
+            const AllwPair q{dx, dy, rho, rho > 0.0 ? 1.0 / rho : 0.0, p.area, SR[o], DR[o], nn3[0], nn3[1], nn3[2], o,
+                             !direct};
+    #pragma unroll 1
+            for (int z = 0; z < nb; ++z) {
+                const double k = kvec[z];
+                if (polar_ok && k * d < kRingMax * (1.0 - 1e-12)) continue;
+                cplx o3[3];
+                delh_dimless_table(tab, k * rho, k * zeta, o3);
+                allw_emit(q, z, k, o3, nn, S64, D64, Dlo, tape);
+            }
         }
     }
 }
@@ -891,7 +827,7 @@ int run_mixed_chunk(const Batch& bt, const double* d_omegas, const double* d_k, 
     double2* RHS = R + nv * nb;  // right-hand side of the D (or K) system
     const RefineCtl ctl = refine_ctl(misc, nb);
     int* d_bad = ctl.bad;
-    auto* d_fall = (int*)(misc + refine_ctl_bytes(nb));  // set when the frequency-batched pass left pairs to the full table
+    auto* d_fall = (int*)(misc + refine_ctl_bytes(nb));  // what the frequency-batched pass left to the rings and the full table
     int rc;
     const double* tab = delh_table_for(ctx, bt.mask, &rc);
     if (rc) return rc;
@@ -910,26 +846,16 @@ int run_mixed_chunk(const Batch& bt, const double* d_omegas, const double* d_k, 
                  : lvl == 1 ? k_wave_delh_allw<float, double> : k_wave_delh_allw<double, double>;
         const size_t wsm = lvl ? wave_allw_smem<float>() : wave_allw_smem<double>();
         MH_CUDA_TRY(ctx, cudaFuncSetAttribute(wk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm));
-        if (lvl == 2) {  // FP32 copy of the polar coefficients for the FP32 contraction
-            auto* cf = (float*)ws_get(ctx, WS_COEF32, sizeof(float) * 4 * kTabPolarFn);
-            if (!cf) return MH_ERR_OOM;
-            k_coef_to_f32<<<blocks(4 * kTabPolarFn, 256), 256, 0, ctx->stream>>>(tab + kTabMonoOff, cf,
-                                                                                 4 * kTabPolarFn);
-            ctx->launches += 1;
-            MH_CUDA_TRY(ctx, cudaMemcpyToSymbolAsync(c_polar_mono_f, cf, sizeof(float) * 4 * kTabPolarFn, 0,
-                                                     cudaMemcpyDeviceToDevice, ctx->stream));
-        }
-        MH_CUDA_TRY(ctx, cudaMemcpyToSymbolAsync(c_polar_mono, tab + kTabMonoOff, sizeof(c_polar_mono), 0,
-                                                 cudaMemcpyDeviceToDevice, ctx->stream));
         for (int z = 0; z < nb; z += kAllwMaxFreqs) {
             const int m = std::min(kAllwMaxFreqs, nb - z);
             const int64_t off = (int64_t)z * nn;
             double2* tp = bt.tape ? bt.tape + 2 * off : nullptr;
             const dim3 g2(blocks(n, kWT), blocks(n, cols));
-            MH_CUDA_TRY(ctx, cudaMemsetAsync(d_fall, 0, sizeof(int), ctx->stream));
+            MH_CUDA_TRY(ctx, cudaMemsetAsync(d_fall, 0, (kRings + 1) * sizeof(int), ctx->stream));
             wk<<<g2, kWT, wsm, ctx->stream>>>(bt.m->geom, n, bt.direct, cols, tab, d_k + z, m, SR, DR, S64 + off,
                                               D64 + off, Dlo + off, tp, d_fall);
-            k_wave_delh_allw_rest<<<g2, kWT, 0, ctx->stream>>>(d_fall, bt.m->geom, n, bt.direct, cols, tab, d_k + z, m,
+            MH_CUDA_TRY(ctx, launch_wave_rings(bt, d_k + z, m, SR, DR, S64 + off, D64 + off, Dlo + off, tp, d_fall));
+            k_wave_delh_allw_rest<<<dim3(g2.x, std::min(g2.y, 64u)), kWT, 0, ctx->stream>>>(d_fall, bt.m->geom, n, bt.direct, cols, tab, d_k + z, m,
                                                               SR, DR, S64 + off, D64 + off, Dlo + off, tp);
             ctx->launches += 1 + (z > 0);
         }
@@ -1041,17 +967,16 @@ int run_fp64_chunk(const Batch& bt, const double* d_omegas, const double* d_k, i
     } else if (allw) {
         MH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_wave_delh_allw<double, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)kWaveAllwSmem));
-        MH_CUDA_TRY(ctx, cudaMemcpyToSymbolAsync(c_polar_mono, tab + kTabMonoOff, sizeof(c_polar_mono), 0,
-                                                 cudaMemcpyDeviceToDevice, ctx->stream));
         for (int z = 0; z < nb; z += kAllwMaxFreqs) {
             const int m = std::min(kAllwMaxFreqs, nb - z);
             const int64_t off = (int64_t)z * nn;
             const dim3 g2(blocks(n, kWT), blocks(n, cols));
-            MH_CUDA_TRY(ctx, cudaMemsetAsync(d_fall, 0, sizeof(int), ctx->stream));
+            MH_CUDA_TRY(ctx, cudaMemsetAsync(d_fall, 0, (kRings + 1) * sizeof(int), ctx->stream));
             double2* tp = bt.tape ? bt.tape + 2 * off : nullptr;
             k_wave_delh_allw<double, double><<<g2, kWT, kWaveAllwSmem, ctx->stream>>>(
                 bt.m->geom, n, bt.direct, cols, tab, d_k + z, m, SR, DR, S64 + off, D64 + off, Dlo + off, tp, d_fall);
-            k_wave_delh_allw_rest<<<g2, kWT, 0, ctx->stream>>>(d_fall, bt.m->geom, n, bt.direct, cols, tab, d_k + z, m,
+            MH_CUDA_TRY(ctx, launch_wave_rings(bt, d_k + z, m, SR, DR, S64 + off, D64 + off, Dlo + off, tp, d_fall));
+            k_wave_delh_allw_rest<<<dim3(g2.x, std::min(g2.y, 64u)), kWT, 0, ctx->stream>>>(d_fall, bt.m->geom, n, bt.direct, cols, tab, d_k + z, m,
                                                               SR, DR, S64 + off, D64 + off, Dlo + off, tp);
             ctx->launches += 2;
         }
@@ -1288,6 +1213,18 @@ int fallback_factor(mh_ctx* ctx, FallbackStore* fb, int64_t n, int nb, int z, co
                                      cudaMemcpyDeviceToDevice, ctx->stream));
     fb->used[z] = 1;
     return fp64_lu_factor(ctx, n, fb->lu + (int64_t)z * nn, fb->piv + (int64_t)z * n);
+}
+
+cudaError_t upload_wave_constants(mh_ctx* ctx, const double* mono, const RingTable& rings)
+{
+    std::vector<float> f(mono, mono + 4 * kTabPolarFn);
+    cudaError_t e = cudaMemcpyToSymbolAsync(c_polar_mono, mono, sizeof(c_polar_mono), 0, cudaMemcpyHostToDevice,
+                                            ctx->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyToSymbolAsync(c_polar_mono_f, f.data(), sizeof(c_polar_mono_f), 0, cudaMemcpyHostToDevice,
+                                    ctx->stream);
+    if (e == cudaSuccess) e = upload_ring_constants(ctx, rings);
+    return e == cudaSuccess ? cudaStreamSynchronize(ctx->stream) : e;
 }
 
 int rankine_real(const Batch& bt, double* SR, double* DR)

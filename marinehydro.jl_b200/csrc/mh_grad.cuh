@@ -17,10 +17,11 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
-__device__ __forceinline__ void stage(Panel* sp, const double* __restrict__ geom, int64_t n, int64_t j0)
+__device__ __forceinline__ void stage(Panel* sp, const double* __restrict__ geom, int64_t n, int64_t j0,
+                                      int cols = kGradCols)
 {
-    for (int t = threadIdx.x; t < kGradCols * G_NFIELDS; t += blockDim.x) {
-        const int f = t / kGradCols, jj = t % kGradCols;
+    for (int t = threadIdx.x; t < cols * G_NFIELDS; t += blockDim.x) {
+        const int f = t / cols, jj = t % cols;
         const int64_t j = j0 + jj;
         const double v = (j < n) ? geom[(int64_t)f * n + j] : 0.0;
         Panel& p = sp[jj];

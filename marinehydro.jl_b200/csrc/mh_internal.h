@@ -49,7 +49,7 @@ struct mh_mesh {
 // Workspace slots of a context; each is a grow-only device buffer.
 enum WsSlot : int {
     WS_S = 0, WS_D, WS_RHS, WS_PHI, WS_TMP, WS_PIV, WS_INFO, WS_LWORK,
-    WS_DOF, WS_OUT, WS_LO, WS_DINV, WS_TMP32, WS_MISC, WS_SR, WS_TMP32B, WS_PANEL, WS_FB, WS_COEF32,
+    WS_DOF, WS_OUT, WS_LO, WS_DINV, WS_TMP32, WS_MISC, WS_SR, WS_TMP32B, WS_PANEL, WS_FB,
     WS_ADJ, WS_WSD, WS_PART, WS_GBAR, WS_TAPE, WS_FLAGS, WS_FLAGS2, WS_NEAR, WS_NEARRES, WS_FALL, WS_REPACK, WS_NSLOTS
 };
 
@@ -245,6 +245,13 @@ struct Batch {
     // dimensionless (G, G_r), 2 double2 in the layout of S, for the adjoint
     double2* tape = nullptr;
 };
+// The frequency-batched Delhommeau pass past the polar patch (mh_rings.cu) for
+// m <= kAllwMaxFreqs frequencies; fall: four flags, zero but for the first, which
+// the pass before sets when it left any pair and frequency.  Sets fall[1] and
+// fall[2] for the rings past the first, and fall[3] when a pair lies outside
+// the rings too.
+cudaError_t launch_wave_rings(const Batch& bt, const double* d_k, int m, const double* SR, const double* DR,
+                              double2* S64, double2* D64, float2* Dlo, double2* tape, int* fall);
 // FP64 factors of the problems of a chunk that left the mixed path, kept for
 // the adjoint solve (lu: nb matrices, piv: nb x n, used[z] != 0 when set).
 struct FallbackStore {
@@ -360,6 +367,14 @@ int hydro_batch_jvp(mh_ctx* ctx, const mh_mesh* m, int64_t nomega, const double*
 
 // ---- Delhommeau table (mh_table.cu) ----
 int ensure_delh_table(mh_ctx* ctx);
+// The table's constant-memory copies of the frequency-batched passes, written
+// on the ctx stream when a context builds its table (host sources, waited
+// for by the caller): polar functions in powers of u (mono) or as Chebyshev
+// series (cheb), and the rings.  Every context on a device writes the same bytes.
+struct RingTable;
+cudaError_t upload_wave_constants(mh_ctx* ctx, const double* mono, const RingTable& rings);   // mh_batch.cu
+cudaError_t upload_ring_constants(mh_ctx* ctx, const RingTable& rings);                       // mh_rings.cu
+cudaError_t upload_tangent_constants(mh_ctx* ctx, const double* cheb, const RingTable& rings);  // mh_jvp.cu
 // Table to use for `mask` on this ctx (null: no Delhommeau term or exact quadrature).
 const double* delh_table_for(mh_ctx* ctx, uint32_t mask, int* status);
 cudaError_t launch_wave_term(mh_ctx* ctx, const double* tab, uint32_t which, int64_t n,

@@ -30,6 +30,7 @@
 #include "mh_device.cuh"
 #include "mh_internal.h"
 #include "mh_rankine.cuh"
+#include "mh_rings.cuh"
 
 namespace mh {
 namespace {
@@ -45,9 +46,10 @@ unsigned nblk(int64_t count, int threads) { return (unsigned)((count + threads -
 #include "mh_grad.cuh"
 
 // Tangent panel (the same fields as a Panel).
-__device__ __forceinline__ void stage_t(Panel* tp, const double* __restrict__ tgeom, int64_t n, int64_t j0)
+__device__ __forceinline__ void stage_t(Panel* tp, const double* __restrict__ tgeom, int64_t n, int64_t j0,
+                                        int cols = kGradCols)
 {
-    stage(tp, tgeom, n, j0);
+    stage(tp, tgeom, n, j0, cols);
 }
 
 // Tangent of the frequency-independent Rankine terms (rankine.jl,
@@ -181,13 +183,26 @@ constexpr int kTS = 4;   // series: B, C, E0, E1
 size_t tan_allw_smem(int nb) { return sizeof(double) * ((size_t)kTS * kTabNU * kTW + 4 * (size_t)nb); }
 
 // The four polar functions' Chebyshev coefficients in constant memory (every
-// lane of the alpha contraction reads the same one); copied from the
-// context's table before each launch (every context builds the same table).
+// lane of the alpha contraction reads the same one); written when a context
+// builds its table (every context builds the same one).
 __constant__ double c_polar_cheb[kTS * kTabPolarFn];
+
+// G and its derivatives from the four functions' values, L = log((R + |z|) / 2),
+// gpk = r / (R (R + |z|)), R = k rho.
+__device__ __forceinline__ void delh_tangent_values(double B, double C, double E0, double E1, double L, double gpk,
+                                                    double R, double k, const WaveGeom& wg, GDer& o3)
+{
+    cplx G[3];
+    const double G_re = -2.0 * E0 * L + B, G_im = 2.0 * kPi * E0;
+    G[0] = mk(G_re, G_im);
+    G[1] = mk(2.0 * E1 * L - 2.0 * E0 * gpk + C, -2.0 * kPi * E1);
+    G[2] = mk(G_re + 2.0 / R, G_im);
+    gder_identities(G, k * wg.dis, k * wg.zs, R, o3);
+}
 
 __global__ void __launch_bounds__(kTW, 5)
 k_wave_tangent_allw(const double* __restrict__ geom, const double* __restrict__ tgeom, int64_t n, int direct,
-                    const double* __restrict__ kvec,
+                    int cols, const double* __restrict__ kvec,
                     const double* __restrict__ dkvec, int nb, const double2* __restrict__ dSR,
                     const double2* __restrict__ dDR, double2* __restrict__ dS, double2* __restrict__ dD,
                     int* __restrict__ fall)
@@ -199,9 +214,9 @@ k_wave_tangent_allw(const double* __restrict__ geom, const double* __restrict__ 
     double* logk = iksh + nb;               // [nb] log k
     double* dksh = logk + nb;               // [nb] dk
     __shared__ Panel sp[kGradCols], tp[kGradCols];
-    const int64_t j0 = (int64_t)blockIdx.y * kGradCols;
-    stage(sp, geom, n, j0);
-    stage_t(tp, tgeom, n, j0);
+    const int64_t j0 = (int64_t)blockIdx.y * cols;
+    stage(sp, geom, n, j0, cols);
+    stage_t(tp, tgeom, n, j0, cols);
     for (int t = threadIdx.x; t < nb; t += blockDim.x) {
         ksh[t] = kvec[t];
         iksh[t] = 1.0 / kvec[t];
@@ -219,7 +234,7 @@ k_wave_tangent_allw(const double* __restrict__ geom, const double* __restrict__ 
         tx[c] = tgeom[(G_CX + c) * n + i];
         tni[c] = tgeom[(G_NX + c) * n + i];
     }
-    const int jend = (int)min((int64_t)kGradCols, n - j0);
+    const int jend = (int)min((int64_t)cols, n - j0);
     const int64_t nn = n * n;
     double* wt = w + tid;
     for (int jj = 0; jj < jend; ++jj) {
@@ -256,7 +271,7 @@ k_wave_tangent_allw(const double* __restrict__ geom, const double* __restrict__ 
         for (int z = 0; z < nb; ++z) {
             const double k = ksh[z];
             const double R = k * rho;
-            if (!(polar_ok && R < kTabRPolar)) {  // left to k_wave_tangent_allw_rest
+            if (!(polar_ok && R < kTabRPolar)) {  // left to k_wave_tangent_ring
                 nfall = true;
                 continue;
             }
@@ -278,13 +293,7 @@ k_wave_tangent_allw(const double* __restrict__ geom, const double* __restrict__ 
                 double sv[kTS];
 #pragma unroll
                 for (int q = 0; q < kTS; ++q) sv[q] = fma(u, b1[q], wt[q * kTabNU * kTW] - b2[q]);
-                const double L = logk[z] + lp;
-                cplx G[3];
-                const double G_re = -2.0 * sv[2] * L + sv[0], G_im = 2.0 * kPi * sv[2];
-                G[0] = mk(G_re, G_im);
-                G[1] = mk(2.0 * sv[3] * L - 2.0 * sv[2] * gp * iksh[z] + sv[1], -2.0 * kPi * sv[3]);
-                G[2] = mk(G_re + 2.0 / R, G_im);
-                gder_identities(G, k * wg.dis, k * wg.zs, R, o3);
+                delh_tangent_values(sv[0], sv[1], sv[2], sv[3], logk[z] + lp, gp * iksh[z], R, k, wg, o3);
             }
             cplx ds, dDn;
             wave_tangent(o3, wg, k, p.area, !direct, nD, t, ds, dDn);
@@ -295,10 +304,101 @@ k_wave_tangent_allw(const double* __restrict__ geom, const double* __restrict__ 
     }
 }
 
-// The (pair, frequency) tangents k_wave_tangent_allw left to the full table
-// (pairs above the free surface or at R = k d >= 2); exits at once when it
-// flagged none.  The test takes a margin of 1e-12 in R, so a pair on the
-// patch edge is written by one kernel at least (by this one last when both).
+// The frequencies at which a pair is in ring q of the table (the tangent of
+// the forward's k_wave_delh_ring, with its margins and flags).
+size_t tan_ring_smem(int q, int nb) { return sizeof(double) * (4 * (size_t)ring_nu(q) * kTW + 4 * (size_t)nb); }
+
+template <int q>
+__global__ void __launch_bounds__(kTW, 5)
+k_wave_tangent_ring(int* __restrict__ fall, const double* __restrict__ geom, const double* __restrict__ tgeom,
+                    int64_t n, int direct, int cols, const double* __restrict__ kvec, const double* __restrict__ dkvec,
+                    int nb, const double2* __restrict__ dSR, const double2* __restrict__ dDR, double2* __restrict__ dS,
+                    double2* __restrict__ dD)
+{
+    if (fall[q] == 0) return;
+    extern __shared__ double dsm[];
+    double* w = dsm + threadIdx.x;             // [4 NU][kTW]
+    double* ksh = dsm + 4 * ring_nu(q) * kTW;  // [nb] k
+    double* iksh = ksh + nb;                   // [nb] 1/k
+    double* logk = iksh + nb;                  // [nb] log k
+    double* dksh = logk + nb;                  // [nb] dk
+    __shared__ Panel sp[kRingCols], tp[kRingCols];
+    __shared__ double xs[12][kTW];  // collocation points and normals, then their tangents
+    __shared__ unsigned short list[kRingCols * kTW];
+    __shared__ int count;
+    for (int t = threadIdx.x; t < nb; t += blockDim.x) {
+        ksh[t] = kvec[t];
+        iksh[t] = 1.0 / kvec[t];
+        logk[t] = log(kvec[t]);
+        dksh[t] = dkvec[t];
+    }
+    __syncthreads();
+    double kmax = 0.0;
+    for (int z = 0; z < nb; ++z) kmax = fmax(kmax, ksh[z]);
+    const int64_t nn = n * n;
+    const int64_t j0 = (int64_t)blockIdx.y * cols, i0 = (int64_t)blockIdx.x * kTW;
+    if (threadIdx.x == 0) count = 0;
+    stage(sp, geom, n, j0, cols);
+    stage_t(tp, tgeom, n, j0, cols);
+    for (int c = 0; c < 6; ++c) {  // G_CX .. G_NZ
+        xs[c][threadIdx.x] = geom[c * n + min(i0 + threadIdx.x, n - 1)];
+        xs[6 + c][threadIdx.x] = tgeom[c * n + min(i0 + threadIdx.x, n - 1)];
+    }
+    __syncthreads();
+    ring_list<kTW, q>(ksh, nb, kmax, cols, list, &count, fall, [&](int row, int c) {
+        const Panel& p = sp[c];
+        const double dx = xs[0][row] - p.c[0], dy = xs[1][row] - p.c[1], zs = xs[2][row] + p.c[2];
+        if (i0 + row >= n || j0 + c >= n) return -2.0;
+        const double d = sqrt(dx * dx + dy * dy + zs * zs);
+        return -zs >= 0.0 && d > 0.0 ? d : -1.0;
+    });
+    __syncthreads();
+    const int total = count;
+    constexpr int kZP = 2;  // frequencies per Horner pass
+    for (int t0 = 0; t0 < total; t0 += kTW) {
+        const bool mine = t0 + (int)threadIdx.x < total;
+        const int item = list[min(t0 + (int)threadIdx.x, total - 1)], row = item % kTW, c = item / kTW;
+        const Panel& p = sp[c];
+        const int64_t o = (j0 + c) * n + i0 + row;
+        const double x[3] = {xs[0][row], xs[1][row], xs[2][row]}, ni[3] = {xs[3][row], xs[4][row], xs[5][row]};
+        const double tx[3] = {xs[6][row], xs[7][row], xs[8][row]}, tni[3] = {xs[9][row], xs[10][row], xs[11][row]};
+        const double* nD = direct ? p.n : ni;
+        const WaveGeom wg = wave_geom(x, p);
+        const double az1 = -wg.zs, rho = hypot(wg.dis, wg.zs);
+        ring_contract<kTW, q>(4.0 * atan2(wg.dis, az1) / kPi - 1.0, w);
+        const double lp = log(0.5 * (rho + az1)), gp = wg.dis / (rho * (rho + az1));
+        const double2 sR = dSR[o], dR_ = dDR[o];
+        for (int z0 = 0; z0 < nb; z0 += kZP) {
+            double R[kZP], val[kZP][4];
+            bool in[kZP], any = false;
+#pragma unroll
+            for (int t = 0; t < kZP; ++t) {
+                R[t] = ksh[min(z0 + t, nb - 1)] * rho;
+                in[t] = mine && z0 + t < nb && ring_in(q, R[t]);
+                any |= in[t];
+            }
+            if (!__any_sync(0xffffffffu, any)) continue;
+            ring_values<kTW, kZP, q>(w, R, val);
+#pragma unroll
+            for (int t = 0; t < kZP; ++t) {
+                if (!in[t]) continue;
+                const int z = z0 + t;
+                const double k = ksh[z];
+                GDer o3;
+                delh_tangent_values(val[t][0], val[t][1], val[t][2], val[t][3], logk[z] + lp, gp * iksh[z], R[t], k, wg,
+                                    o3);
+                cplx ds, dDn;
+                wave_tangent(o3, wg, k, p.area, !direct, nD, pair_tan(tx, tni, tp[c], direct, dksh[z]), ds, dDn);
+                dS[(int64_t)z * nn + o] = make_double2(sR.x - kI4P * ds.re, sR.y - kI4P * ds.im);
+                dD[(int64_t)z * nn + o] = make_double2(dR_.x - kI4P * dDn.re, dR_.y - kI4P * dDn.im);
+            }
+        }
+    }
+}
+
+// The (pair, frequency) tangents the rings do not reach either (pairs above
+// the free surface or at R = k d >= 16), by the full table and the quadrature;
+// exits at once when none was flagged.
 __global__ void __launch_bounds__(kTW)
 k_wave_tangent_allw_rest(const int* __restrict__ fall, const double* __restrict__ geom,
                          const double* __restrict__ tgeom, int64_t n, int direct, const double* __restrict__ tab,
@@ -306,7 +406,7 @@ k_wave_tangent_allw_rest(const int* __restrict__ fall, const double* __restrict_
                          const double2* __restrict__ dSR, const double2* __restrict__ dDR, double2* __restrict__ dS,
                          double2* __restrict__ dD)
 {
-    if (*fall == 0) return;
+    if (fall[kRings] == 0) return;
     __shared__ Panel sp[kGradCols], tp[kGradCols];
     const int64_t j0 = (int64_t)blockIdx.y * kGradCols;
     stage(sp, geom, n, j0);
@@ -334,7 +434,7 @@ k_wave_tangent_allw_rest(const int* __restrict__ fall, const double* __restrict_
 #pragma unroll 1
         for (int z = 0; z < nb; ++z) {
             const double k = kvec[z];
-            if (polar_ok && k * rho < kTabRPolar * (1.0 - 1e-12)) continue;
+            if (polar_ok && k * rho < kRingMax * (1.0 - 1e-12)) continue;
             const WaveTan t = pair_tan(tx, tni, tp[jj], direct, dkvec[z]);
             GDer o3;
             delh_point_grad(tab, k * wg.dis, k * wg.zs, &o3);
@@ -496,18 +596,28 @@ int tangent_matrices(const Batch& bt, const Jvp& jv, const double* d_k, const do
     const int64_t n = bt.n;
     if (jv.wave_kind == 2 && tab && nb >= kJvpAllwMinFreqs) {
         const size_t smem = tan_allw_smem(nb);
-        auto* fall = (int*)ws_get(ctx, WS_FALL, sizeof(int));
+        auto* fall = (int*)ws_get(ctx, WS_FALL, (kRings + 1) * sizeof(int));
         if (!fall) return MH_ERR_OOM;
         MH_CUDA_TRY(ctx, raise_smem_cap((const void*)k_wave_tangent_allw, smem));
-        MH_CUDA_TRY(ctx, cudaMemcpyToSymbolAsync(c_polar_cheb, tab, sizeof(c_polar_cheb), 0, cudaMemcpyDeviceToDevice,
-                                                 ctx->stream));
-        MH_CUDA_TRY(ctx, cudaMemsetAsync(fall, 0, sizeof(int), ctx->stream));
-        const dim3 g2(nblk(n, kTW), nblk(n, kGradCols));
-        k_wave_tangent_allw<<<g2, kTW, smem, ctx->stream>>>(bt.m->geom, jv.tgeom, n, bt.direct, d_k, d_dk, nb,
+        MH_CUDA_TRY(ctx, cudaMemsetAsync(fall, 0, (kRings + 1) * sizeof(int), ctx->stream));
+        const int cols = wave_cols(n, kGradCols);
+        const dim3 gw(nblk(n, kTW), nblk(n, cols)), g2(nblk(n, kTW), nblk(n, kGradCols));
+        k_wave_tangent_allw<<<gw, kTW, smem, ctx->stream>>>(bt.m->geom, jv.tgeom, n, bt.direct, cols, d_k, d_dk, nb,
                                                             jv.dSR, jv.dDR, dS, dD, fall);
+        auto ring = [&](auto kern, int q) -> cudaError_t {
+            const cudaError_t e = raise_smem_cap((const void*)kern, tan_ring_smem(q, nb));
+            if (e != cudaSuccess) return e;
+            const int rc = ring_cols(n);
+            kern<<<dim3(nblk(n, kTW), nblk(n, rc)), kTW, tan_ring_smem(q, nb), ctx->stream>>>(
+                fall, bt.m->geom, jv.tgeom, n, bt.direct, rc, d_k, d_dk, nb, jv.dSR, jv.dDR, dS, dD);
+            return cudaGetLastError();
+        };
+        MH_CUDA_TRY(ctx, ring(k_wave_tangent_ring<0>, 0));
+        MH_CUDA_TRY(ctx, ring(k_wave_tangent_ring<1>, 1));
+        MH_CUDA_TRY(ctx, ring(k_wave_tangent_ring<2>, 2));
         k_wave_tangent_allw_rest<<<g2, kTW, 0, ctx->stream>>>(fall, bt.m->geom, jv.tgeom, n, bt.direct, tab, d_k,
                                                              d_dk, nb, jv.dSR, jv.dDR, dS, dD);
-        ctx->launches += 1;
+        ctx->launches += 4;
     } else {
         k_wave_tangent<<<dim3(nblk(n, kJR), nblk(n, kGradCols), (unsigned)nb), kJR, 0, ctx->stream>>>(
             jv.wave_kind, bt.m->geom, jv.tgeom, n, bt.direct, jv.wave_kind == 2 ? tab : nullptr, d_k, d_dk, jv.dSR,
@@ -760,6 +870,15 @@ int hydro_batch_jvp(mh_ctx* ctx, const mh_mesh* m, int64_t nomega, const double*
     }
     if (info) *info = local;
     return MH_OK;
+}
+
+cudaError_t upload_tangent_constants(mh_ctx* ctx, const double* cheb, const RingTable& rings)
+{
+    cudaError_t e = cudaMemcpyToSymbolAsync(c_polar_cheb, cheb, sizeof(c_polar_cheb), 0, cudaMemcpyHostToDevice,
+                                            ctx->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyToSymbolAsync(c_rings, &rings, sizeof(rings), 0, cudaMemcpyHostToDevice, ctx->stream);
+    return e == cudaSuccess ? cudaStreamSynchronize(ctx->stream) : e;
 }
 
 }  // namespace mh

@@ -2,11 +2,14 @@
 // and the point-evaluation hook mh_wave_term.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
+#include <memory>
 #include <vector>
 
 #include "mh_internal.h"
 #include "mh_device.cuh"
+#include "mh_rings.cuh"
 
 namespace mh {
 namespace {
@@ -54,25 +57,41 @@ void cheb_nodes(int n, double a, double b, std::vector<double>& x)
         x[k] = 0.5 * (a + b) + 0.5 * (b - a) * std::cos(M_PI * (k + 0.5) / n);
 }
 
-// Chebyshev coefficients of an n x n block of node values (row = first coord).
-void cheb_coeffs(int n, const double* vals, double* coef)
+// Chebyshev coefficients of an n x m block of node values (row = first coord).
+void cheb_coeffs(int n, int m, const double* vals, double* coef)
 {
-    std::vector<double> T((size_t)n * n), tmp((size_t)n * n);
+    auto basis = [](int k) {
+        std::vector<double> T((size_t)k * k);
+        for (int i = 0; i < k; ++i)
+            for (int l = 0; l < k; ++l) T[(size_t)i * k + l] = (i == 0 ? 1.0 : 2.0) / k * std::cos(M_PI * i * (l + 0.5) / k);
+        return T;
+    };
+    const std::vector<double> Tn = basis(n), Tm = basis(m);
+    std::vector<double> tmp((size_t)n * m);
     for (int i = 0; i < n; ++i)
-        for (int k = 0; k < n; ++k)
-            T[i * n + k] = (i == 0 ? 1.0 : 2.0) / n * std::cos(M_PI * i * (k + 0.5) / n);
-    for (int i = 0; i < n; ++i)
-        for (int l = 0; l < n; ++l) {
+        for (int l = 0; l < m; ++l) {
             double s = 0.0;
-            for (int k = 0; k < n; ++k) s += T[i * n + k] * vals[k * n + l];
-            tmp[i * n + l] = s;
+            for (int k = 0; k < n; ++k) s += Tn[(size_t)i * n + k] * vals[(size_t)k * m + l];
+            tmp[(size_t)i * m + l] = s;
         }
     for (int i = 0; i < n; ++i)
-        for (int j = 0; j < n; ++j) {
+        for (int j = 0; j < m; ++j) {
             double s = 0.0;
-            for (int l = 0; l < n; ++l) s += tmp[i * n + l] * T[j * n + l];
-            coef[i * n + j] = s;
+            for (int l = 0; l < m; ++l) s += tmp[(size_t)i * m + l] * Tm[(size_t)j * m + l];
+            coef[(size_t)i * m + j] = s;
         }
+}
+
+// P[i * n + m]: coefficient of u^m in T_i(u), i, m < n.
+std::vector<double> cheb_to_powers(int n)
+{
+    std::vector<double> P((size_t)n * n, 0.0);
+    P[0] = 1.0;
+    if (n > 1) P[(size_t)n + 1] = 1.0;
+    for (int i = 2; i < n; ++i)  // T_i = 2 u T_{i-1} - T_{i-2}
+        for (int m = 0; m < n; ++m)
+            P[(size_t)i * n + m] = (m > 0 ? 2.0 * P[(size_t)(i - 1) * n + m - 1] : 0.0) - P[(size_t)(i - 2) * n + m];
+    return P;
 }
 
 }  // namespace
@@ -100,6 +119,15 @@ int ensure_delh_table(mh_ctx* ctx)
                     z.push_back(-xb[l]);
                 }
         }
+    for (int q = 0; q < kRings; ++q) {
+        cheb_nodes(ring_fit_r(q), 2.0 * (1 << q), 4.0 * (1 << q), xa);
+        cheb_nodes(ring_fit_a(q), 0.0, 0.5 * M_PI, xb);
+        for (int k = 0; k < ring_fit_r(q); ++k)
+            for (int l = 0; l < ring_fit_a(q); ++l) {
+                r.push_back(xa[k] * std::sin(xb[l]));
+                z.push_back(-xa[k] * std::cos(xb[l]));
+            }
+    }
     const int n = (int)r.size();
     double *d_r = nullptr, *d_z = nullptr, *d_B = nullptr, *d_C = nullptr, *d_E0 = nullptr,
            *d_E1 = nullptr, *d_tab = nullptr;
@@ -144,16 +172,10 @@ int ensure_delh_table(mh_ctx* ctx)
     // monomial basis of u: T_i(u) = sum_m P[i][m] u^m
     {
         std::vector<double> full((size_t)kTabNP * kTabNP);
-        std::vector<double> P((size_t)kTabNU * kTabNU, 0.0);  // P[i][m]
-        P[0] = 1.0;
-        if (kTabNU > 1) P[1 * kTabNU + 1] = 1.0;
-        for (int i = 2; i < kTabNU; ++i)  // T_i = 2 u T_{i-1} - T_{i-2}
-            for (int m = 0; m < kTabNU; ++m)
-                P[(size_t)i * kTabNU + m] = (m > 0 ? 2.0 * P[(size_t)(i - 1) * kTabNU + m - 1] : 0.0) -
-                                            P[(size_t)(i - 2) * kTabNU + m];
+        const std::vector<double> P = cheb_to_powers(kTabNU);
         const double* src[4] = {hB.data(), hC.data(), hE0.data(), hE1.data()};
         for (int q = 0; q < 4; ++q) {
-            cheb_coeffs(kTabNP, src[q], full.data());
+            cheb_coeffs(kTabNP, kTabNP, src[q], full.data());
             for (int i = 0; i < kTabNU; ++i)
                 for (int j = 0; j < kTabNV; ++j)
                     tab[(size_t)q * kTabPolarFn + i * kTabNV + j] = full[(size_t)i * kTabNP + j];
@@ -169,8 +191,36 @@ int ensure_delh_table(mh_ctx* ctx)
     const int np = kTabNP * kTabNP, nc = kTabNC * kTabNC;
     for (int c = 0; c < kTabNCell * kTabNCell; ++c) {
         double* dst = tab.data() + kTabPolarWords + (size_t)c * kTabCellWords;
-        cheb_coeffs(kTabNC, hB.data() + np + (size_t)c * nc, dst);
-        cheb_coeffs(kTabNC, hC.data() + np + (size_t)c * nc, dst + nc);
+        cheb_coeffs(kTabNC, kTabNC, hB.data() + np + (size_t)c * nc, dst);
+        cheb_coeffs(kTabNC, kTabNC, hC.data() + np + (size_t)c * nc, dst + nc);
+    }
+    // rings: the same four functions, rows in powers of u, packed
+    auto rings = std::make_unique<RingTable>();
+    size_t at = (size_t)np + (size_t)kTabNCell * kTabNCell * nc;
+    for (int q = 0; q < kRings; ++q) {
+        const int fr = ring_fit_r(q), fa = ring_fit_a(q), nu = ring_nu(q);
+        const double* src[4] = {hB.data() + at, hC.data() + at, hE0.data() + at, hE1.data() + at};
+        at += (size_t)fr * fa;
+        const std::vector<double> P = cheb_to_powers(nu);
+        std::vector<double> full((size_t)fr * fa);
+        for (int f = 0; f < 4; ++f) {
+            cheb_coeffs(fr, fa, src[f], full.data());
+            for (int m = 0; m < nu; ++m)
+                for (int j = 0; j < ring_nv(q, m >= ring_head(q)); ++j) {
+                    double a = 0.0;
+                    for (int i = m; i < nu; ++i)
+                        if (j < ring_nv(q, i >= ring_head(q))) a += P[(size_t)i * nu + m] * full[(size_t)i * fa + j];
+                    rings->coef[4 * (size_t)(ring_at(q, m) + j) + f] = a;
+                }
+        }
+    }
+    const double* mono = tab.data() + kTabMonoOff;
+    if (e == cudaSuccess) e = upload_wave_constants(ctx, mono, *rings);
+    if (e == cudaSuccess) e = upload_tangent_constants(ctx, tab.data(), *rings);
+    if (e != cudaSuccess) {
+        cleanup();
+        cudaFree(d_tab);
+        return set_err(ctx, MH_ERR_CUDA, "Delhommeau constants: %s", cudaGetErrorString(e));
     }
     e = cudaMemcpyAsync(d_tab, tab.data(), sizeof(double) * kTabWords, cudaMemcpyHostToDevice,
                         ctx->stream);

@@ -23,8 +23,14 @@
 //     frequency).  Degree 14 in R and 21 in alpha are kept: the fitted
 //     coefficients beyond them are at the rounding level (|c| < 5e-15 for
 //     all four functions);
+//   - three rings R in [2, 4), [4, 8), [8, 16) in the same polar coordinates
+//     and functions, for the frequency-batched evaluation past the patch: a
+//     panel pair keeps its alpha at every frequency, so its alpha direction is
+//     contracted once per ring (every thread reads the same coefficient) and
+//     each frequency is four polynomials in R again (mh_rings.cuh);
 //   - Cartesian cells of 0.5 x 0.5 over r, |z| in [0, 16), degree 12 x 12,
-//     for R >= 2 (every cell touching R < 1 lies inside the polar patch).
+//     for single points at R >= 2 (every cell touching R < 1 lies inside the
+//     polar patch).
 // Points outside the table fall back to the adaptive quadrature.  The node
 // values are computed on the device with the FP64 quadrature; the table's
 // error against it is ~1e-12 absolute.
