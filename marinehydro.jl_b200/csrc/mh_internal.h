@@ -224,6 +224,13 @@ cudaError_t launch_lu_solve_persist(mh_ctx* ctx, int backend, bool conj_trans, c
                                     int64_t stride, int nbatch, const float2* Dinv, float2* X, int64_t xstride,
                                     int nrhs, int* bad = nullptr, const int* done = nullptr,
                                     cudaStream_t stream = nullptr, int flags_slot = WS_FLAGS);
+// The tensor-core backend's part of it (mh_lu_solve.cu): bad is required;
+// unset_flag (may be null): failure injection, a flag that nothing publishes.
+// lu_solve_cluster_fits: whether the solution fits a CTA's shared memory.
+bool lu_solve_cluster_fits(int64_t n);
+cudaError_t launch_lu_solve_cluster(mh_ctx* ctx, bool conj_trans, const float2* A, int64_t n, int64_t stride,
+                                    int nbatch, const float2* Dinv, int64_t dstride, float2* X, int64_t xstride,
+                                    int nrhs, int* bad, const int* done, const int* unset_flag, cudaStream_t stream);
 // Conjugate-transposed solve D^H X = X with the factors of launch_lu_tc
 // (backend MH_LU_TCGEN05_F16) or launch_lu_f32 (MH_LU_SIMT_F32).
 cudaError_t launch_lu_solve_ct(mh_ctx* ctx, int backend, const float2* A, int64_t n, int64_t stride,
