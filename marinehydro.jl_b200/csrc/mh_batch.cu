@@ -119,6 +119,12 @@ constexpr size_t kWaveAllwSmem = wave_allw_smem<double>();
 __device__ __forceinline__ double hfma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float hfma(float a, float b, float c) { return fmaf(a, b, c); }
 
+// The four functions' coefficients of one row, side by side for 16-byte accesses.
+template <typename HT>
+struct alignas(16) Quad {
+    HT f[4];
+};
+
 // HT: the type of the per-frequency Horner series in R; CT: the type of the
 // alpha contraction (double, or float in the reduced-precision levels of the
 // mixed path, mh_ctx_set_wave_series_fp32).  The pair geometry, the log
@@ -134,7 +140,8 @@ k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, int col
     double* logk = wsm;                            // [nb]
     double* invk = logk + kAllwMaxFreqs;           // [nb], nb <= kAllwMaxFreqs
     double* ksm = invk + kAllwMaxFreqs;            // [nb]
-    HT* w = reinterpret_cast<HT*>(ksm + kAllwMaxFreqs);  // [4 * NU][kWT]
+    const int tid = threadIdx.x;
+    Quad<HT>* w = reinterpret_cast<Quad<HT>*>(ksm + kAllwMaxFreqs) + tid;  // [NU][kWT]
     __shared__ Panel sp[kCols];
     const int64_t j0 = (int64_t)blockIdx.y * cols;
     stage_panels(sp, geom, n, j0, cols);
@@ -144,13 +151,11 @@ k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, int col
         invk[t] = 1.0 / kvec[t];
     }
     __syncthreads();
-    const int tid = threadIdx.x;
     const int64_t i = (int64_t)blockIdx.x * kWT + tid;
     if (i >= n) return;
     const int64_t nn = n * n;
     const double x[3] = {geom[G_CX * n + i], geom[G_CY * n + i], geom[G_CZ * n + i]};
     const double ni[3] = {geom[G_NX * n + i], geom[G_NY * n + i], geom[G_NZ * n + i]};
-    const bool wrt_first = !direct;
     const int jend = (int)min((int64_t)cols, n - j0);
     for (int jj = 0; jj < jend; ++jj) {
         const Panel& p = sp[jj];
@@ -168,33 +173,30 @@ k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, int col
         const double v = 4.0 * atan2(rho, az) / kPi - 1.0;
         const double lp = log(0.5 * (d + az));
         const double gp = rho / (d * (d + az));
-        const double inv_d = 1.0 / d, inv_rho = rho > 0.0 ? 1.0 / rho : 0.0;
+        const double inv_d2 = 2.0 / d;
         const double sr = SR[o], dr = DR[o];
-        // contract alpha: w_q[row] = sum_j c_q[row][j] T_j(v), the four
-        // functions' Clenshaw recurrences interleaved (four independent
-        // dependency chains per row)
+        // contract alpha: w_q[row] = sum_j c_q[row][j] T_j(v).  The T_j are held
+        // in registers for all rows, so a term is one FMA whose constant operand
+        // is a factor; with the constant as the addend (Clenshaw's recurrence, two
+        // operations a term, or Horner's rule) its load bounds the loop, and two or
+        // three rows at a time lose more in occupancy.  2048 panels x 64
+        // frequencies, us: Clenshaw 2376, Horner 2871, this 2164 (three rows at a
+        // time 2743), with the pair's factors multiplied out (allw_pair) 1957.
         if (polar_ok) {
-            const CT vc = (CT)v, v2 = (CT)(2.0 * v);
+            CT T[kTabNV];
+            cheb_values<kTabNV>((CT)v, T);
 #pragma unroll 1
             for (int row = 0; row < kTabNU; ++row) {
-                const int cr = row * kTabNV;
-                CT b1[4] = {0, 0, 0, 0}, b2[4] = {0, 0, 0, 0};
+                CT b[4] = {0, 0, 0, 0};
 #pragma unroll
-                for (int col = kTabNV - 1; col >= 1; --col) {
+                for (int col = 0; col < kTabNV; ++col)
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const CT t = hfma(v2, b1[q], polar_coef<CT>(cr + q * kTabPolarFn + col) - b2[q]);
-                        b2[q] = b1[q];
-                        b1[q] = t;
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    w[(q * kTabNU + row) * kWT + tid] = (HT)hfma(vc, b1[q], polar_coef<CT>(cr + q * kTabPolarFn) - b2[q]);
+                    for (int q = 0; q < 4; ++q) b[q] = hfma(polar_coef<CT>(4 * (row * kTabNV + col) + q), T[col], b[q]);
+                w[row * kWT] = Quad<HT>{{(HT)b[0], (HT)b[1], (HT)b[2], (HT)b[3]}};
             }
         }
-        const AllwPair q{dx, dy, rho, inv_rho, p.area, sr, dr, direct ? p.n[0] : ni[0], direct ? p.n[1] : ni[1],
-                         direct ? p.n[2] : ni[2], o, wrt_first};
+        const AllwPair q = allw_pair(dx, dy, rho, p.area, sr, dr, direct ? p.n[0] : ni[0], direct ? p.n[1] : ni[1],
+                                     direct ? p.n[2] : ni[2], direct, o);
         // four frequencies per Horner pass: each coefficient read from shared
         // memory feeds four recurrences.  Frequencies off the polar patch are
         // only noted here: k_wave_delh_ring evaluates them with the
@@ -218,20 +220,18 @@ k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, int col
             }
             HT val[kZP][4];
             if (anyp) {
+                const Quad<HT> c0 = w[(kTabNU - 1) * kWT];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const HT c = w[(q * kTabNU + kTabNU - 1) * kWT + tid];
+                for (int t = 0; t < kZP; ++t)
 #pragma unroll
-                    for (int t = 0; t < kZP; ++t) val[t][q] = c;
-                }
+                    for (int q = 0; q < 4; ++q) val[t][q] = c0.f[q];
 #pragma unroll
                 for (int row = kTabNU - 2; row >= 0; --row) {
+                    const Quad<HT> c = w[row * kWT];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const HT c = w[(q * kTabNU + row) * kWT + tid];
+                    for (int t = 0; t < kZP; ++t)
 #pragma unroll
-                        for (int t = 0; t < kZP; ++t) val[t][q] = hfma(val[t][q], uz[t], c);
-                    }
+                        for (int q = 0; q < 4; ++q) val[t][q] = hfma(val[t][q], uz[t], c.f[q]);
                 }
             }
 #pragma unroll
@@ -246,11 +246,12 @@ k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, int col
                 const double B = (double)val[t][0], C = (double)val[t][1], E0 = (double)val[t][2],
                              E1 = (double)val[t][3];
                 const double L = logk[z] + lp;
-                const double G_re = -2.0 * E0 * L + B, G_im = 2.0 * kPi * E0;
+                const double e0 = -2.0 * E0, e1 = 2.0 * E1;
+                const double G_re = e0 * L + B, G_im = 2.0 * kPi * E0;
                 cplx o3[3];
                 o3[0] = mk(G_re, G_im);
-                o3[1] = mk(2.0 * E1 * L - 2.0 * E0 * gp * ik + C, -2.0 * kPi * E1);
-                o3[2] = mk(G_re + 2.0 * inv_d * ik, G_im);  // 2 / R, R = k d
+                o3[1] = mk(fma(e1, L, fma(e0, gp * ik, C)), -2.0 * kPi * E1);
+                o3[2] = mk(fma(inv_d2, ik, G_re), G_im);  // 2 / R, R = k d
                 allw_emit(q, z, kz[t], o3, nn, S64, D64, Dlo, tape);
             }
         }
@@ -290,8 +291,7 @@ k_wave_delh_allw_rest(const int* __restrict__ fall, const double* __restrict__ g
             const double d = hypot(rho, zeta);
             const bool polar_ok = -zeta >= 0.0;
             const double* nn3 = direct ? p.n : ni;
-            const AllwPair q{dx, dy, rho, rho > 0.0 ? 1.0 / rho : 0.0, p.area, SR[o], DR[o], nn3[0], nn3[1], nn3[2], o,
-                             !direct};
+            const AllwPair q = allw_pair(dx, dy, rho, p.area, SR[o], DR[o], nn3[0], nn3[1], nn3[2], direct, o);
     #pragma unroll 1
             for (int z = 0; z < nb; ++z) {
                 const double k = kvec[z];

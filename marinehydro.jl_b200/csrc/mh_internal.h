@@ -376,12 +376,12 @@ int hydro_batch_jvp(mh_ctx* ctx, const mh_mesh* m, int64_t nomega, const double*
 int ensure_delh_table(mh_ctx* ctx);
 // The table's constant-memory copies of the frequency-batched passes, written
 // on the ctx stream when a context builds its table (host sources, waited
-// for by the caller): polar functions in powers of u (mono) or as Chebyshev
-// series (cheb), and the rings.  Every context on a device writes the same bytes.
+// for by the caller): the polar functions in powers of u (mono: [row][column]
+// [function]) and the rings.  Every context on a device writes the same bytes.
 struct RingTable;
 cudaError_t upload_wave_constants(mh_ctx* ctx, const double* mono, const RingTable& rings);   // mh_batch.cu
 cudaError_t upload_ring_constants(mh_ctx* ctx, const RingTable& rings);                       // mh_rings.cu
-cudaError_t upload_tangent_constants(mh_ctx* ctx, const double* cheb, const RingTable& rings);  // mh_jvp.cu
+cudaError_t upload_tangent_constants(mh_ctx* ctx, const double* mono, const RingTable& rings);  // mh_jvp.cu
 // Table to use for `mask` on this ctx (null: no Delhommeau term or exact quadrature).
 const double* delh_table_for(mh_ctx* ctx, uint32_t mask, int* status);
 cudaError_t launch_wave_term(mh_ctx* ctx, const double* tab, uint32_t which, int64_t n,

@@ -174,7 +174,7 @@ k_wave_tangent(int kind, const double* __restrict__ geom, const double* __restri
 
 // Frequency-batched tangent of the tabulated Delhommeau term (the tangent of
 // the forward's frequency-batched pass): the alpha contraction of the four
-// polar tables once per pair, 1-D Clenshaw in R per frequency, derivatives
+// polar tables once per pair, a polynomial in R per frequency, derivatives
 // from the identities.
 constexpr int kTW = 64;  // rows (threads) per CTA
 constexpr int kTS = 4;   // series: B, C, E0, E1
@@ -182,10 +182,10 @@ constexpr int kTS = 4;   // series: B, C, E0, E1
 // contracted series of every row, then k, 1/k, log k and dk/d(direction) per frequency
 size_t tan_allw_smem(int nb) { return sizeof(double) * ((size_t)kTS * kTabNU * kTW + 4 * (size_t)nb); }
 
-// The four polar functions' Chebyshev coefficients in constant memory (every
-// lane of the alpha contraction reads the same one); written when a context
+// The four polar functions (powers of u, Chebyshev series in v) in constant
+// memory (every lane of the alpha contraction reads the same one); written when a context
 // builds its table (every context builds the same one).
-__constant__ double c_polar_cheb[kTS * kTabPolarFn];
+__constant__ double c_polar_mono[kTS * kTabPolarFn];
 
 // G and its derivatives from the four functions' values, L = log((R + |z|) / 2),
 // gpk = r / (R (R + |z|)), R = k rho.
@@ -248,23 +248,19 @@ k_wave_tangent_allw(const double* __restrict__ geom, const double* __restrict__ 
         const double lp = log(0.5 * (rho + az1));
         const double gp = wg.dis / (rho * (rho + az1));
         const double2 sR = dSR[o], dR_ = dDR[o];
-        if (polar_ok) {  // the four functions' recurrences interleaved
-            const double v = 4.0 * atan2(wg.dis, az1) / kPi - 1.0, v2 = 2.0 * v;
+        if (polar_ok) {
+            double T[kTabNV];
+            cheb_values(4.0 * atan2(wg.dis, az1) / kPi - 1.0, T);
 #pragma unroll 1
             for (int row = 0; row < kTabNU; ++row) {
-                const double* cr = c_polar_cheb + row * kTabNV;
-                double b1[kTS] = {0.0, 0.0, 0.0, 0.0}, b2[kTS] = {0.0, 0.0, 0.0, 0.0};
+                const double* cr = c_polar_mono + 4 * row * kTabNV;
+                double b[kTS] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-                for (int col = kTabNV - 1; col >= 1; --col) {
+                for (int col = 0; col < kTabNV; ++col)
 #pragma unroll
-                    for (int q = 0; q < kTS; ++q) {
-                        const double t = fma(v2, b1[q], cr[q * kTabPolarFn + col] - b2[q]);
-                        b2[q] = b1[q];
-                        b1[q] = t;
-                    }
-                }
+                    for (int q = 0; q < kTS; ++q) b[q] = fma(cr[4 * col + q], T[col], b[q]);
 #pragma unroll
-                for (int q = 0; q < kTS; ++q) wt[(q * kTabNU + row) * kTW] = fma(v, b1[q], cr[q * kTabPolarFn] - b2[q]);
+                for (int q = 0; q < kTS; ++q) wt[(q * kTabNU + row) * kTW] = b[q];
             }
         }
         bool nfall = false;
@@ -278,21 +274,14 @@ k_wave_tangent_allw(const double* __restrict__ geom, const double* __restrict__ 
             const WaveTan t = pair_tan(tx, tni, tp[jj], direct, dksh[z]);
             GDer o3;
             {
-                const double u = 2.0 * R / kTabRPolar - 1.0, u2 = 2.0 * u;
-                double b1[kTS], b2[kTS];
-#pragma unroll
-                for (int q = 0; q < kTS; ++q) b1[q] = b2[q] = 0.0;
-#pragma unroll 4
-                for (int row = kTabNU - 1; row >= 1; --row)
-#pragma unroll
-                    for (int q = 0; q < kTS; ++q) {
-                        const double nt = fma(u2, b1[q], wt[(q * kTabNU + row) * kTW] - b2[q]);
-                        b2[q] = b1[q];
-                        b1[q] = nt;
-                    }
+                const double u = 2.0 * R / kTabRPolar - 1.0;
                 double sv[kTS];
 #pragma unroll
-                for (int q = 0; q < kTS; ++q) sv[q] = fma(u, b1[q], wt[q * kTabNU * kTW] - b2[q]);
+                for (int q = 0; q < kTS; ++q) sv[q] = wt[(q * kTabNU + kTabNU - 1) * kTW];
+#pragma unroll 7
+                for (int row = kTabNU - 2; row >= 0; --row)
+#pragma unroll
+                    for (int q = 0; q < kTS; ++q) sv[q] = fma(sv[q], u, wt[(q * kTabNU + row) * kTW]);
                 delh_tangent_values(sv[0], sv[1], sv[2], sv[3], logk[z] + lp, gp * iksh[z], R, k, wg, o3);
             }
             cplx ds, dDn;
@@ -872,9 +861,9 @@ int hydro_batch_jvp(mh_ctx* ctx, const mh_mesh* m, int64_t nomega, const double*
     return MH_OK;
 }
 
-cudaError_t upload_tangent_constants(mh_ctx* ctx, const double* cheb, const RingTable& rings)
+cudaError_t upload_tangent_constants(mh_ctx* ctx, const double* mono, const RingTable& rings)
 {
-    cudaError_t e = cudaMemcpyToSymbolAsync(c_polar_cheb, cheb, sizeof(c_polar_cheb), 0, cudaMemcpyHostToDevice,
+    cudaError_t e = cudaMemcpyToSymbolAsync(c_polar_mono, mono, sizeof(c_polar_mono), 0, cudaMemcpyHostToDevice,
                                             ctx->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyToSymbolAsync(c_rings, &rings, sizeof(rings), 0, cudaMemcpyHostToDevice, ctx->stream);

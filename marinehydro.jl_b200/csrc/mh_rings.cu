@@ -19,9 +19,8 @@ namespace {
 // Evaluating each point from the Cartesian cells instead (what this replaces)
 // gathers 288 coefficients per thread from cells that differ between the
 // threads of a warp, on top of exp, log, J0 and J1 per point.  Measured, us:
-// cells -> this, N 2997, 24 frequencies, R below 3.4: 5806 -> 2414; two bodies,
-// N 1456, 32 frequencies, R below 7: 2049 -> 1064; N 870, 16 frequencies, R below
-// 2.7: 258 -> 231, and its tangent (mh_jvp.cu) 424 -> 263.
+// cells -> this, N 2997, 24 frequencies, R below 3.4: 5806 -> 2232; N 870, 16
+// frequencies, R below 2.7: 258 -> 215, and its tangent (mh_jvp.cu) 424 -> 258.
 constexpr int kRT = 64;  // threads (rows) per CTA
 constexpr size_t ring_smem(int q) { return sizeof(double) * (3 * kAllwMaxFreqs + 4 * ring_nu(q) * kRT); }
 
@@ -79,10 +78,10 @@ k_wave_delh_ring(int* __restrict__ fall, const double* __restrict__ geom, int64_
         ring_contract<kRT, q>(4.0 * atan2(rho, az) / kPi - 1.0, w);
         const double lp = log(0.5 * (d + az));
         const double gp = rho / (d * (d + az));
-        const double inv_d = 1.0 / d;
-        const AllwPair pair{dx, dy, rho, rho > 0.0 ? 1.0 / rho : 0.0, p.area, SR[o], DR[o],
-                            direct ? p.n[0] : xs[3][row], direct ? p.n[1] : xs[4][row], direct ? p.n[2] : xs[5][row],
-                            o, !direct};
+        const double inv_d2 = 2.0 / d;
+        const AllwPair pair =
+            allw_pair(dx, dy, rho, p.area, SR[o], DR[o], direct ? p.n[0] : xs[3][row], direct ? p.n[1] : xs[4][row],
+                      direct ? p.n[2] : xs[5][row], direct, o);
         for (int z0 = 0; z0 < nb; z0 += kZP) {
             double R[kZP], val[kZP][4];
             bool in[kZP], any = false;
@@ -100,11 +99,12 @@ k_wave_delh_ring(int* __restrict__ fall, const double* __restrict__ geom, int64_
                 const int z = z0 + t;
                 const double ik = invk[z], L = logk[z] + lp;
                 const double B = val[t][0], C = val[t][1], E0 = val[t][2], E1 = val[t][3];
-                const double G_re = -2.0 * E0 * L + B, G_im = 2.0 * kPi * E0;
+                const double e0 = -2.0 * E0, e1 = 2.0 * E1;
+                const double G_re = e0 * L + B, G_im = 2.0 * kPi * E0;
                 cplx o3[3];
                 o3[0] = mk(G_re, G_im);
-                o3[1] = mk(2.0 * E1 * L - 2.0 * E0 * gp * ik + C, -2.0 * kPi * E1);
-                o3[2] = mk(G_re + 2.0 * inv_d * ik, G_im);
+                o3[1] = mk(fma(e1, L, fma(e0, gp * ik, C)), -2.0 * kPi * E1);
+                o3[2] = mk(fma(inv_d2, ik, G_re), G_im);
                 allw_emit(pair, z, ksm[z], o3, nn, S64, D64, Dlo, tape);
             }
         }

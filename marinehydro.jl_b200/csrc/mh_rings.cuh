@@ -11,8 +11,9 @@
 // written when a context builds its table (every context writes the same).
 // 2997 panels x 24 frequencies, us: 7265 with the coefficients read from global
 // memory (two 16-byte loads per column bound it), 4294 from constant memory
-// with a loop of its own length for every row, 4004 with these fixed lengths (2414
-// with the pairs listed first, mh_rings.cu).
+// with a loop of its own length for every row, 4004 with these fixed lengths, 2414
+// with the pairs listed first (mh_rings.cu), 2232 with the Chebyshev values in
+// registers instead of Clenshaw's recurrence.
 #pragma once
 #include "mh_internal.h"
 #include "mh_device.cuh"
@@ -53,37 +54,32 @@ __device__ __forceinline__ bool ring_in(int q, double R)
     return R >= lo * (1.0 - 1e-12) && R < 2.0 * lo * (1.0 + 1e-12);
 }
 
-// Rows m0 .. m1 - 1 of ring q (of NV columns each) contracted at v.
-template <int T, int q, int NV, int m0, int m1>
-__device__ __forceinline__ void ring_contract_rows(double v, double* __restrict__ w)
+// Rows m0 .. m1 - 1 of ring q (of NV columns each) contracted with t[j] = T_j(v).
+template <int T, int q, int NV, int m0, int m1, int N>
+__device__ __forceinline__ void ring_contract_rows(const double (&t)[N], double* __restrict__ w)
 {
-    const double v2 = 2.0 * v;
 #pragma unroll 1
     for (int row = m0; row < m1; ++row) {
         const int c = 4 * (ring_at(q, m0) + (row - m0) * NV);
-        double b1[4] = {0.0, 0.0, 0.0, 0.0}, b2[4] = {0.0, 0.0, 0.0, 0.0};
+        double b[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-        for (int col = NV - 1; col >= 1; --col) {
+        for (int col = 0; col < NV; ++col)
 #pragma unroll
-            for (int f = 0; f < 4; ++f) {
-                const double t = fma(v2, b1[f], c_rings.coef[c + 4 * col + f] - b2[f]);
-                b2[f] = b1[f];
-                b1[f] = t;
-            }
-        }
+            for (int f = 0; f < 4; ++f) b[f] = fma(c_rings.coef[c + 4 * col + f], t[col], b[f]);
 #pragma unroll
-        for (int f = 0; f < 4; ++f) w[(4 * row + f) * T] = fma(v, b1[f], c_rings.coef[c + f] - b2[f]);
+        for (int f = 0; f < 4; ++f) w[(4 * row + f) * T] = b[f];
     }
 }
 
 // The alpha direction of ring q contracted at v: w[(4 row + f) T], f = B, C,
-// E0, E1, the coefficients of u^row (T threads' columns side by side), the four
-// functions' Clenshaw recurrences interleaved.
+// E0, E1, the coefficients of u^row (T threads' columns side by side).
 template <int T, int q>
 __device__ __forceinline__ void ring_contract(double v, double* __restrict__ w)
 {
-    ring_contract_rows<T, q, ring_nv(q, 0), 0, ring_head(q)>(v, w);
-    ring_contract_rows<T, q, ring_nv(q, 1), ring_head(q), ring_nu(q)>(v, w);
+    double t[ring_nv(q, 0)];
+    cheb_values(v, t);
+    ring_contract_rows<T, q, ring_nv(q, 0), 0, ring_head(q)>(t, w);
+    ring_contract_rows<T, q, ring_nv(q, 1), ring_head(q), ring_nu(q)>(t, w);
 }
 
 // The four functions at Z values of R in ring q, from its contraction.

@@ -214,9 +214,11 @@ int ensure_delh_table(mh_ctx* ctx)
                 }
         }
     }
-    const double* mono = tab.data() + kTabMonoOff;
-    if (e == cudaSuccess) e = upload_wave_constants(ctx, mono, *rings);
-    if (e == cudaSuccess) e = upload_tangent_constants(ctx, tab.data(), *rings);
+    std::vector<double> mono(4 * kTabPolarFn);  // the functions of a (row, column) side by side
+    for (int i = 0; i < kTabPolarFn; ++i)
+        for (int q = 0; q < 4; ++q) mono[4 * i + q] = tab[kTabMonoOff + q * kTabPolarFn + i];
+    if (e == cudaSuccess) e = upload_wave_constants(ctx, mono.data(), *rings);
+    if (e == cudaSuccess) e = upload_tangent_constants(ctx, mono.data(), *rings);
     if (e != cudaSuccess) {
         cleanup();
         cudaFree(d_tab);

@@ -128,4 +128,14 @@ __device__ __noinline__ static void delh_dimless_table(const double* __restrict_
     out[2] = mk(G_re + 2.0 / R, G_im);
 }
 
+// T_0(v) .. T_{N-1}(v).
+template <int N, class T>
+__device__ __forceinline__ void cheb_values(T v, T (&t)[N])
+{
+    t[0] = 1;
+    t[1] = v;
+#pragma unroll
+    for (int j = 2; j < N; ++j) t[j] = 2 * v * t[j - 1] - t[j - 2];
+}
+
 }  // namespace mh

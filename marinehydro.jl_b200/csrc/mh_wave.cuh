@@ -33,31 +33,30 @@ __device__ __forceinline__ void stage_panels(Panel* sp, const double* __restrict
 
 // One pair of the frequency-batched pass and its output: S, D (FP64 and the
 // FP32 copy of D) and the tape of frequency z from the dimensionless
-// (G, G_r, G_z) in o3.
+// (G, G_r, G_z) in o3.  What does not depend on the frequency is multiplied out
+// once per pair: S = sr + s0 k G, D = dr + k^2 (a G_r + c G_z).
 struct AllwPair {
-    double dx, dy, rho, inv_rho, area, sr, dr;
-    double n0, n1, n2;  // the normal of D (source panel when direct), held in registers
-    int64_t o;          // pair offset j * n + i
-    bool wrt_first;
+    double rho, sr, dr, s0, a, c;
+    int64_t o;  // pair offset j * n + i
 };
+
+// nx, ny, nz: the normal of D, the source panel's when direct (whose derivative
+// is by the second argument).
+__device__ __forceinline__ AllwPair allw_pair(double dx, double dy, double rho, double area, double sr, double dr,
+                                              double nx, double ny, double nz, bool direct, int64_t o)
+{
+    const double s0 = -kInv4Pi * area, h = rho > 0.0 ? s0 / rho * (nx * dx + ny * dy) : 0.0;
+    return AllwPair{rho, sr, dr, s0, direct ? -h : h, s0 * nz, o};
+}
 
 __device__ __forceinline__ void allw_emit(const AllwPair& q, int z, double k, const cplx o3[3], int64_t nn,
                                           double2* __restrict__ S64, double2* __restrict__ D64,
                                           float2* __restrict__ Dlo, double2* __restrict__ tape)
 {
-    const double r = k * q.rho;
-    double d1 = 0.0, d2 = 0.0;
-    if (fabs(r) > 1e-6) {
-        const double f = k * q.inv_rho;  // k^2 / r
-        d1 = q.wrt_first ? f * q.dx : -f * q.dx;
-        d2 = q.wrt_first ? f * q.dy : -f * q.dy;
-    }
-    const double ka = k * q.area;
-    const cplx s = ka * o3[0];
-    const cplx g0 = (ka * d1) * o3[1], g1 = (ka * d2) * o3[1], g2 = (ka * k) * o3[2];
-    const double Sr = q.sr - kInv4Pi * s.re, Si = -kInv4Pi * s.im;
-    const double Dr = q.dr - kInv4Pi * (q.n0 * g0.re + q.n1 * g1.re + q.n2 * g2.re);
-    const double Di = -kInv4Pi * (q.n0 * g0.im + q.n1 * g1.im + q.n2 * g2.im);
+    const double ks = k * q.s0, k2 = k * k, a = k * q.rho > 1e-6 ? q.a : 0.0;
+    const double Sr = fma(ks, o3[0].re, q.sr), Si = ks * o3[0].im;
+    const double Dr = fma(k2, fma(a, o3[1].re, q.c * o3[2].re), q.dr);
+    const double Di = k2 * fma(a, o3[1].im, q.c * o3[2].im);
     const int64_t m = (int64_t)z * nn + q.o;
     S64[m] = make_double2(Sr, Si);
     D64[m] = make_double2(Dr, Di);
