@@ -84,35 +84,25 @@ k_wave_batch(const double* __restrict__ geom, int64_t n, int direct, int cols, c
 // R = k d moves: the alpha direction of the four polar tables (B, C,
 // E0 = e^z J0(r), E1 = e^z J1(r)) is contracted once per pair into
 // w_q[i] = sum_j c_q[i][j] T_j(v(alpha)) (shared memory), and each frequency
-// then evaluates four 1-D Chebyshev series in R (Clenshaw) with no
-// transcendental calls; the log term splits as log(k) + log((d + |zeta|)/2).
-// The series in R use the table's monomial-in-u copy (Horner's rule, four
-// frequencies per pass).
+// then evaluates four polynomials in R (Horner's rule, four frequencies per
+// pass) with no transcendental calls; the log term splits as log(k) +
+// log((d + |zeta|)/2).
 // Frequencies at which the pair leaves the polar patch use the table's rings.
 // Same arithmetic as wave_pair<true> up to reassociation (~1e-16).
-// The four polar functions' monomial-in-u coefficients in constant memory:
-// every lane of the alpha contraction reads the same coefficient, which the
-// constant cache broadcasts.  Written when a context builds its table; every
-// context builds the same one, so a later copy writes identical bytes.
-__constant__ double c_polar_mono[4 * kTabPolarFn];
-// The same coefficients rounded to FP32 (the FP32 alpha contraction).
-__constant__ float c_polar_mono_f[4 * kTabPolarFn];
-
-template <typename CT>
-__device__ __forceinline__ CT polar_coef(int i);
-template <>
-__device__ __forceinline__ double polar_coef<double>(int i) { return c_polar_mono[i]; }
-template <>
-__device__ __forceinline__ float polar_coef<float>(int i) { return c_polar_mono_f[i]; }
+// The polar coefficients of the FP32 contraction, [row][column][function]: every
+// lane reads the same one, which the constant cache broadcasts.  Written when a
+// context builds its table; every context builds the same one, so a later copy
+// writes identical bytes.
+__constant__ float c_polar_f[4 * kTabPolarFn];
 
 constexpr int kWT = 128;  // threads (rows) per CTA of k_wave_delh_allw
 // k, log k and 1/k per frequency, then the contracted series of every row
-// in the type HT of the per-frequency Horner pass (the polar coefficients
-// are read from constant memory)
+// in the type HT of the per-frequency Horner pass; one column of padding, so
+// that contract_tiles' stores meet no bank twice in FP32
 template <typename HT>
 constexpr size_t wave_allw_smem()
 {
-    return sizeof(double) * 3 * kAllwMaxFreqs + sizeof(HT) * 4 * kTabNU * kWT;
+    return sizeof(double) * 3 * kAllwMaxFreqs + sizeof(HT) * 4 * kTabNU * (kWT + 1);
 }
 constexpr size_t kWaveAllwSmem = wave_allw_smem<double>();
 
@@ -130,7 +120,7 @@ struct alignas(16) Quad {
 // mixed path, mh_ctx_set_wave_series_fp32).  The pair geometry, the log
 // terms and everything after the series stay in FP64.
 template <typename HT, typename CT>
-__global__ void __launch_bounds__(kWT, 3)
+__global__ void __launch_bounds__(kWT, sizeof(HT) == 4 ? 4 : 3)
 k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, int cols, const double* __restrict__ tab,
                  const double* __restrict__ kvec, int nb, const double* __restrict__ SR,
                  const double* __restrict__ DR, double2* __restrict__ S64, double2* __restrict__ D64,
@@ -141,7 +131,7 @@ k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, int col
     double* invk = logk + kAllwMaxFreqs;           // [nb], nb <= kAllwMaxFreqs
     double* ksm = invk + kAllwMaxFreqs;            // [nb]
     const int tid = threadIdx.x;
-    Quad<HT>* w = reinterpret_cast<Quad<HT>*>(ksm + kAllwMaxFreqs) + tid;  // [NU][kWT]
+    Quad<HT>* w = reinterpret_cast<Quad<HT>*>(ksm + kAllwMaxFreqs);  // [NU][kWT + 1]
     __shared__ Panel sp[kCols];
     const int64_t j0 = (int64_t)blockIdx.y * cols;
     stage_panels(sp, geom, n, j0, cols);
@@ -151,8 +141,8 @@ k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, int col
         invk[t] = 1.0 / kvec[t];
     }
     __syncthreads();
-    const int64_t i = (int64_t)blockIdx.x * kWT + tid;
-    if (i >= n) return;
+    const bool inside = (int64_t)blockIdx.x * kWT + tid < n;  // the others take part in the contractions
+    const int64_t i = min((int64_t)blockIdx.x * kWT + tid, n - 1);
     const int64_t nn = n * n;
     const double x[3] = {geom[G_CX * n + i], geom[G_CY * n + i], geom[G_CZ * n + i]};
     const double ni[3] = {geom[G_NX * n + i], geom[G_NY * n + i], geom[G_NZ * n + i]};
@@ -175,26 +165,38 @@ k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, int col
         const double gp = rho / (d * (d + az));
         const double inv_d2 = 2.0 / d;
         const double sr = SR[o], dr = DR[o];
-        // contract alpha: w_q[row] = sum_j c_q[row][j] T_j(v).  The T_j are held
-        // in registers for all rows, so a term is one FMA whose constant operand
-        // is a factor; with the constant as the addend (Clenshaw's recurrence, two
-        // operations a term, or Horner's rule) its load bounds the loop, and two or
-        // three rows at a time lose more in occupancy.  2048 panels x 64
-        // frequencies, us: Clenshaw 2376, Horner 2871, this 2164 (three rows at a
-        // time 2743), with the pair's factors multiplied out (allw_pair) 1957.
-        if (polar_ok) {
+        // contract alpha: w[row].f[q] = sum_j c_q[row][j] T_j(v).  In FP32 a term is
+        // one FMA, the T_j in registers for all rows; in FP64 the warp's pairs
+        // together by the matrix instruction (mh_contract.cuh).
+        if constexpr (sizeof(CT) == 4) {
             CT T[kTabNV];
-            cheb_values<kTabNV>((CT)v, T);
+            cheb_values((CT)v, T);
 #pragma unroll 1
             for (int row = 0; row < kTabNU; ++row) {
                 CT b[4] = {0, 0, 0, 0};
 #pragma unroll
                 for (int col = 0; col < kTabNV; ++col)
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) b[q] = hfma(polar_coef<CT>(4 * (row * kTabNV + col) + q), T[col], b[q]);
-                w[row * kWT] = Quad<HT>{{(HT)b[0], (HT)b[1], (HT)b[2], (HT)b[3]}};
+                    for (int q = 0; q < 4; ++q) b[q] = hfma(c_polar_f[4 * (row * kTabNV + col) + q], T[col], b[q]);
+                w[row * (kWT + 1) + tid] = Quad<HT>{{(HT)b[0], (HT)b[1], (HT)b[2], (HT)b[3]}};
             }
+        } else {
+            __syncwarp();  // the last pairs' columns are read
+#pragma unroll 1
+            for (int g = 0; g < 4; ++g) {
+                double t[1][frag_steps(kTabNV)];
+                cheb_frags(v, g, t);
+                contract_tiles<frag_tiles(kTabNU), frag_steps(kTabNV)>(
+                    tab + kFragPolar, g, t, [&](int m, int pr, double a, double b) {
+                        if (m >= 4 * kTabNU) return;
+                        Quad<HT>* to = w + (m >> 2) * (kWT + 1) + (tid & ~31) + pr;
+                        to[0].f[m & 3] = (HT)a;
+                        to[1].f[m & 3] = (HT)b;
+                    });
+            }
+            __syncwarp();
         }
+        if (!inside) continue;
         const AllwPair q = allw_pair(dx, dy, rho, p.area, sr, dr, direct ? p.n[0] : ni[0], direct ? p.n[1] : ni[1],
                                      direct ? p.n[2] : ni[2], direct, o);
         // four frequencies per Horner pass: each coefficient read from shared
@@ -220,14 +222,14 @@ k_wave_delh_allw(const double* __restrict__ geom, int64_t n, int direct, int col
             }
             HT val[kZP][4];
             if (anyp) {
-                const Quad<HT> c0 = w[(kTabNU - 1) * kWT];
+                const Quad<HT> c0 = w[(kTabNU - 1) * (kWT + 1) + tid];
 #pragma unroll
                 for (int t = 0; t < kZP; ++t)
 #pragma unroll
                     for (int q = 0; q < 4; ++q) val[t][q] = c0.f[q];
 #pragma unroll
                 for (int row = kTabNU - 2; row >= 0; --row) {
-                    const Quad<HT> c = w[row * kWT];
+                    const Quad<HT> c = w[row * (kWT + 1) + tid];
 #pragma unroll
                     for (int t = 0; t < kZP; ++t)
 #pragma unroll
@@ -854,7 +856,7 @@ int run_mixed_chunk(const Batch& bt, const double* d_omegas, const double* d_k, 
             MH_CUDA_TRY(ctx, cudaMemsetAsync(d_fall, 0, (kRings + 1) * sizeof(int), ctx->stream));
             wk<<<g2, kWT, wsm, ctx->stream>>>(bt.m->geom, n, bt.direct, cols, tab, d_k + z, m, SR, DR, S64 + off,
                                               D64 + off, Dlo + off, tp, d_fall);
-            MH_CUDA_TRY(ctx, launch_wave_rings(bt, d_k + z, m, SR, DR, S64 + off, D64 + off, Dlo + off, tp, d_fall));
+            MH_CUDA_TRY(ctx, launch_wave_rings(bt, tab, d_k + z, m, SR, DR, S64 + off, D64 + off, Dlo + off, tp, d_fall));
             k_wave_delh_allw_rest<<<dim3(g2.x, std::min(g2.y, 64u)), kWT, 0, ctx->stream>>>(d_fall, bt.m->geom, n, bt.direct, cols, tab, d_k + z, m,
                                                               SR, DR, S64 + off, D64 + off, Dlo + off, tp);
             ctx->launches += 1 + (z > 0);
@@ -975,7 +977,7 @@ int run_fp64_chunk(const Batch& bt, const double* d_omegas, const double* d_k, i
             double2* tp = bt.tape ? bt.tape + 2 * off : nullptr;
             k_wave_delh_allw<double, double><<<g2, kWT, kWaveAllwSmem, ctx->stream>>>(
                 bt.m->geom, n, bt.direct, cols, tab, d_k + z, m, SR, DR, S64 + off, D64 + off, Dlo + off, tp, d_fall);
-            MH_CUDA_TRY(ctx, launch_wave_rings(bt, d_k + z, m, SR, DR, S64 + off, D64 + off, Dlo + off, tp, d_fall));
+            MH_CUDA_TRY(ctx, launch_wave_rings(bt, tab, d_k + z, m, SR, DR, S64 + off, D64 + off, Dlo + off, tp, d_fall));
             k_wave_delh_allw_rest<<<dim3(g2.x, std::min(g2.y, 64u)), kWT, 0, ctx->stream>>>(d_fall, bt.m->geom, n, bt.direct, cols, tab, d_k + z, m,
                                                               SR, DR, S64 + off, D64 + off, Dlo + off, tp);
             ctx->launches += 2;
@@ -1215,15 +1217,10 @@ int fallback_factor(mh_ctx* ctx, FallbackStore* fb, int64_t n, int nb, int z, co
     return fp64_lu_factor(ctx, n, fb->lu + (int64_t)z * nn, fb->piv + (int64_t)z * n);
 }
 
-cudaError_t upload_wave_constants(mh_ctx* ctx, const double* mono, const RingTable& rings)
+cudaError_t upload_wave_constants(mh_ctx* ctx, const float* mono)
 {
-    std::vector<float> f(mono, mono + 4 * kTabPolarFn);
-    cudaError_t e = cudaMemcpyToSymbolAsync(c_polar_mono, mono, sizeof(c_polar_mono), 0, cudaMemcpyHostToDevice,
-                                            ctx->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyToSymbolAsync(c_polar_mono_f, f.data(), sizeof(c_polar_mono_f), 0, cudaMemcpyHostToDevice,
-                                    ctx->stream);
-    if (e == cudaSuccess) e = upload_ring_constants(ctx, rings);
+    const cudaError_t e = cudaMemcpyToSymbolAsync(c_polar_f, mono, sizeof(c_polar_f), 0, cudaMemcpyHostToDevice,
+                                                  ctx->stream);
     return e == cudaSuccess ? cudaStreamSynchronize(ctx->stream) : e;
 }
 

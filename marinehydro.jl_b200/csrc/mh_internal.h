@@ -257,8 +257,8 @@ struct Batch {
 // the pass before sets when it left any pair and frequency.  Sets fall[1] and
 // fall[2] for the rings past the first, and fall[3] when a pair lies outside
 // the rings too.
-cudaError_t launch_wave_rings(const Batch& bt, const double* d_k, int m, const double* SR, const double* DR,
-                              double2* S64, double2* D64, float2* Dlo, double2* tape, int* fall);
+cudaError_t launch_wave_rings(const Batch& bt, const double* tab, const double* d_k, int m, const double* SR,
+                              const double* DR, double2* S64, double2* D64, float2* Dlo, double2* tape, int* fall);
 // FP64 factors of the problems of a chunk that left the mixed path, kept for
 // the adjoint solve (lu: nb matrices, piv: nb x n, used[z] != 0 when set).
 struct FallbackStore {
@@ -374,14 +374,11 @@ int hydro_batch_jvp(mh_ctx* ctx, const mh_mesh* m, int64_t nomega, const double*
 
 // ---- Delhommeau table (mh_table.cu) ----
 int ensure_delh_table(mh_ctx* ctx);
-// The table's constant-memory copies of the frequency-batched passes, written
-// on the ctx stream when a context builds its table (host sources, waited
-// for by the caller): the polar functions in powers of u (mono: [row][column]
-// [function]) and the rings.  Every context on a device writes the same bytes.
-struct RingTable;
-cudaError_t upload_wave_constants(mh_ctx* ctx, const double* mono, const RingTable& rings);   // mh_batch.cu
-cudaError_t upload_ring_constants(mh_ctx* ctx, const RingTable& rings);                       // mh_rings.cu
-cudaError_t upload_tangent_constants(mh_ctx* ctx, const double* mono, const RingTable& rings);  // mh_jvp.cu
+// The polar functions' coefficients in FP32 for k_wave_delh_allw's FP32 contraction,
+// [row][column][function], powers of u by Chebyshev series in v: copied to constant
+// memory on the ctx stream and waited for.  Every context on a device writes the
+// same bytes.
+cudaError_t upload_wave_constants(mh_ctx* ctx, const float* mono);  // mh_batch.cu
 // Table to use for `mask` on this ctx (null: no Delhommeau term or exact quadrature).
 const double* delh_table_for(mh_ctx* ctx, uint32_t mask, int* status);
 cudaError_t launch_wave_term(mh_ctx* ctx, const double* tab, uint32_t which, int64_t n,

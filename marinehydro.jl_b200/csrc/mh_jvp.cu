@@ -182,11 +182,6 @@ constexpr int kTS = 4;   // series: B, C, E0, E1
 // contracted series of every row, then k, 1/k, log k and dk/d(direction) per frequency
 size_t tan_allw_smem(int nb) { return sizeof(double) * ((size_t)kTS * kTabNU * kTW + 4 * (size_t)nb); }
 
-// The four polar functions (powers of u, Chebyshev series in v) in constant
-// memory (every lane of the alpha contraction reads the same one); written when a context
-// builds its table (every context builds the same one).
-__constant__ double c_polar_mono[kTS * kTabPolarFn];
-
 // G and its derivatives from the four functions' values, L = log((R + |z|) / 2),
 // gpk = r / (R (R + |z|)), R = k rho.
 __device__ __forceinline__ void delh_tangent_values(double B, double C, double E0, double E1, double L, double gpk,
@@ -202,7 +197,7 @@ __device__ __forceinline__ void delh_tangent_values(double B, double C, double E
 
 __global__ void __launch_bounds__(kTW, 5)
 k_wave_tangent_allw(const double* __restrict__ geom, const double* __restrict__ tgeom, int64_t n, int direct,
-                    int cols, const double* __restrict__ kvec,
+                    int cols, const double* __restrict__ tab, const double* __restrict__ kvec,
                     const double* __restrict__ dkvec, int nb, const double2* __restrict__ dSR,
                     const double2* __restrict__ dDR, double2* __restrict__ dS, double2* __restrict__ dD,
                     int* __restrict__ fall)
@@ -225,8 +220,8 @@ k_wave_tangent_allw(const double* __restrict__ geom, const double* __restrict__ 
     }
     __syncthreads();
     const int tid = threadIdx.x;
-    const int64_t i = (int64_t)blockIdx.x * kTW + tid;
-    if (i >= n) return;  // no block-level synchronisation below
+    const bool inside = (int64_t)blockIdx.x * kTW + tid < n;  // the others take part in the contractions
+    const int64_t i = min((int64_t)blockIdx.x * kTW + tid, n - 1);
     double x[3], ni[3], tx[3], tni[3];
     for (int c = 0; c < 3; ++c) {
         x[c] = geom[(G_CX + c) * n + i];
@@ -236,7 +231,6 @@ k_wave_tangent_allw(const double* __restrict__ geom, const double* __restrict__ 
     }
     const int jend = (int)min((int64_t)cols, n - j0);
     const int64_t nn = n * n;
-    double* wt = w + tid;
     for (int jj = 0; jj < jend; ++jj) {
         const Panel& p = sp[jj];
         const int64_t o = (j0 + jj) * n + i;
@@ -248,21 +242,20 @@ k_wave_tangent_allw(const double* __restrict__ geom, const double* __restrict__ 
         const double lp = log(0.5 * (rho + az1));
         const double gp = wg.dis / (rho * (rho + az1));
         const double2 sR = dSR[o], dR_ = dDR[o];
-        if (polar_ok) {
-            double T[kTabNV];
-            cheb_values(4.0 * atan2(wg.dis, az1) / kPi - 1.0, T);
+        const double v = 4.0 * atan2(wg.dis, az1) / kPi - 1.0;
+        __syncwarp();  // the last pairs' columns are read
 #pragma unroll 1
-            for (int row = 0; row < kTabNU; ++row) {
-                const double* cr = c_polar_mono + 4 * row * kTabNV;
-                double b[kTS] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-                for (int col = 0; col < kTabNV; ++col)
-#pragma unroll
-                    for (int q = 0; q < kTS; ++q) b[q] = fma(cr[4 * col + q], T[col], b[q]);
-#pragma unroll
-                for (int q = 0; q < kTS; ++q) wt[(q * kTabNU + row) * kTW] = b[q];
-            }
+        for (int g = 0; g < 4; g += 2) {
+            double t[2][frag_steps(kTabNV)];
+            cheb_frags(v, g, t);
+            contract_tiles<frag_tiles(kTabNU), frag_steps(kTabNV)>(
+                tab + kFragPolar, g, t, [&](int m, int pr, double a, double b) {
+                    if (m < kTS * kTabNU)
+                        *reinterpret_cast<double2*>(w + w_at<kTW>(m, (tid & ~31) + pr)) = make_double2(a, b);
+                });
         }
+        __syncwarp();
+        if (!inside) continue;
         bool nfall = false;
         for (int z = 0; z < nb; ++z) {
             const double k = ksh[z];
@@ -277,11 +270,11 @@ k_wave_tangent_allw(const double* __restrict__ geom, const double* __restrict__ 
                 const double u = 2.0 * R / kTabRPolar - 1.0;
                 double sv[kTS];
 #pragma unroll
-                for (int q = 0; q < kTS; ++q) sv[q] = wt[(q * kTabNU + kTabNU - 1) * kTW];
+                for (int q = 0; q < kTS; ++q) sv[q] = w[w_at<kTW>(q, tid) + kTS * (kTabNU - 1) * kTW];
 #pragma unroll 7
                 for (int row = kTabNU - 2; row >= 0; --row)
 #pragma unroll
-                    for (int q = 0; q < kTS; ++q) sv[q] = fma(sv[q], u, wt[(q * kTabNU + row) * kTW]);
+                    for (int q = 0; q < kTS; ++q) sv[q] = fma(sv[q], u, w[w_at<kTW>(q, tid) + kTS * row * kTW]);
                 delh_tangent_values(sv[0], sv[1], sv[2], sv[3], logk[z] + lp, gp * iksh[z], R, k, wg, o3);
             }
             cplx ds, dDn;
@@ -300,13 +293,13 @@ size_t tan_ring_smem(int q, int nb) { return sizeof(double) * (4 * (size_t)ring_
 template <int q>
 __global__ void __launch_bounds__(kTW, 5)
 k_wave_tangent_ring(int* __restrict__ fall, const double* __restrict__ geom, const double* __restrict__ tgeom,
-                    int64_t n, int direct, int cols, const double* __restrict__ kvec, const double* __restrict__ dkvec,
-                    int nb, const double2* __restrict__ dSR, const double2* __restrict__ dDR, double2* __restrict__ dS,
+                    int64_t n, int direct, int cols, const double* __restrict__ tab, const double* __restrict__ kvec,
+                    const double* __restrict__ dkvec, int nb, const double2* __restrict__ dSR, const double2* __restrict__ dDR, double2* __restrict__ dS,
                     double2* __restrict__ dD)
 {
     if (fall[q] == 0) return;
     extern __shared__ double dsm[];
-    double* w = dsm + threadIdx.x;             // [4 NU][kTW]
+    double* w = dsm;                           // [4 NU][kTW]
     double* ksh = dsm + 4 * ring_nu(q) * kTW;  // [nb] k
     double* iksh = ksh + nb;                   // [nb] 1/k
     double* logk = iksh + nb;                  // [nb] log k
@@ -354,7 +347,7 @@ k_wave_tangent_ring(int* __restrict__ fall, const double* __restrict__ geom, con
         const double* nD = direct ? p.n : ni;
         const WaveGeom wg = wave_geom(x, p);
         const double az1 = -wg.zs, rho = hypot(wg.dis, wg.zs);
-        ring_contract<kTW, q>(4.0 * atan2(wg.dis, az1) / kPi - 1.0, w);
+        ring_contract<kTW, q>(tab, 4.0 * atan2(wg.dis, az1) / kPi - 1.0, w);
         const double lp = log(0.5 * (rho + az1)), gp = wg.dis / (rho * (rho + az1));
         const double2 sR = dSR[o], dR_ = dDR[o];
         for (int z0 = 0; z0 < nb; z0 += kZP) {
@@ -591,14 +584,14 @@ int tangent_matrices(const Batch& bt, const Jvp& jv, const double* d_k, const do
         MH_CUDA_TRY(ctx, cudaMemsetAsync(fall, 0, (kRings + 1) * sizeof(int), ctx->stream));
         const int cols = wave_cols(n, kGradCols);
         const dim3 gw(nblk(n, kTW), nblk(n, cols)), g2(nblk(n, kTW), nblk(n, kGradCols));
-        k_wave_tangent_allw<<<gw, kTW, smem, ctx->stream>>>(bt.m->geom, jv.tgeom, n, bt.direct, cols, d_k, d_dk, nb,
+        k_wave_tangent_allw<<<gw, kTW, smem, ctx->stream>>>(bt.m->geom, jv.tgeom, n, bt.direct, cols, tab, d_k, d_dk, nb,
                                                             jv.dSR, jv.dDR, dS, dD, fall);
         auto ring = [&](auto kern, int q) -> cudaError_t {
             const cudaError_t e = raise_smem_cap((const void*)kern, tan_ring_smem(q, nb));
             if (e != cudaSuccess) return e;
             const int rc = ring_cols(n);
             kern<<<dim3(nblk(n, kTW), nblk(n, rc)), kTW, tan_ring_smem(q, nb), ctx->stream>>>(
-                fall, bt.m->geom, jv.tgeom, n, bt.direct, rc, d_k, d_dk, nb, jv.dSR, jv.dDR, dS, dD);
+                fall, bt.m->geom, jv.tgeom, n, bt.direct, rc, tab, d_k, d_dk, nb, jv.dSR, jv.dDR, dS, dD);
             return cudaGetLastError();
         };
         MH_CUDA_TRY(ctx, ring(k_wave_tangent_ring<0>, 0));
@@ -859,15 +852,6 @@ int hydro_batch_jvp(mh_ctx* ctx, const mh_mesh* m, int64_t nomega, const double*
     }
     if (info) *info = local;
     return MH_OK;
-}
-
-cudaError_t upload_tangent_constants(mh_ctx* ctx, const double* mono, const RingTable& rings)
-{
-    cudaError_t e = cudaMemcpyToSymbolAsync(c_polar_mono, mono, sizeof(c_polar_mono), 0, cudaMemcpyHostToDevice,
-                                            ctx->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyToSymbolAsync(c_rings, &rings, sizeof(rings), 0, cudaMemcpyHostToDevice, ctx->stream);
-    return e == cudaSuccess ? cudaStreamSynchronize(ctx->stream) : e;
 }
 
 }  // namespace mh

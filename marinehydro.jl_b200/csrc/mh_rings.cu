@@ -19,16 +19,17 @@ namespace {
 // Evaluating each point from the Cartesian cells instead (what this replaces)
 // gathers 288 coefficients per thread from cells that differ between the
 // threads of a warp, on top of exp, log, J0 and J1 per point.  Measured, us:
-// cells -> this, N 2997, 24 frequencies, R below 3.4: 5806 -> 2232; N 870, 16
-// frequencies, R below 2.7: 258 -> 215, and its tangent (mh_jvp.cu) 424 -> 258.
+// cells -> this, N 2997, 24 frequencies, R below 3.4: 5806 -> 1786; two bodies,
+// N 1456, 32 frequencies, R below 7: 2049 -> 747; N 870, 16 frequencies, R below
+// 2.7: 258 -> 152, and its tangent (mh_jvp.cu) 424 -> 185.
 constexpr int kRT = 64;  // threads (rows) per CTA
 constexpr size_t ring_smem(int q) { return sizeof(double) * (3 * kAllwMaxFreqs + 4 * ring_nu(q) * kRT); }
 
 template <int q>
 __global__ void __launch_bounds__(kRT, q == 0 ? 6 : q == 1 ? 5 : 4)
 k_wave_delh_ring(int* __restrict__ fall, const double* __restrict__ geom, int64_t n, int direct, int cols,
-                 const double* __restrict__ kvec, int nb, const double* __restrict__ SR,
-                 const double* __restrict__ DR, double2* __restrict__ S64, double2* __restrict__ D64,
+                 const double* __restrict__ tab, const double* __restrict__ kvec, int nb,
+                 const double* __restrict__ SR, const double* __restrict__ DR, double2* __restrict__ S64, double2* __restrict__ D64,
                  float2* __restrict__ Dlo, double2* __restrict__ tape)
 {
     if (fall[q] == 0) return;
@@ -36,7 +37,7 @@ k_wave_delh_ring(int* __restrict__ fall, const double* __restrict__ geom, int64_
     double* logk = wsm;
     double* invk = logk + kAllwMaxFreqs;
     double* ksm = invk + kAllwMaxFreqs;
-    double* w = ksm + kAllwMaxFreqs + threadIdx.x;  // [4 * NU][kRT]
+    double* w = ksm + kAllwMaxFreqs;  // [4 * NU][kRT]
     __shared__ Panel sp[kRingCols];
     __shared__ double xs[6][kRT];  // collocation points and their normals
     __shared__ unsigned short list[kRingCols * kRT];
@@ -75,7 +76,7 @@ k_wave_delh_ring(int* __restrict__ fall, const double* __restrict__ geom, int64_
         const double rho = (dis2 == 0.0) ? sqrt(dis2 + purt * purt) - purt : sqrt(dis2);
         const double zeta = xs[2][row] + p.c[2], az = -zeta;
         const double d = hypot(rho, zeta);
-        ring_contract<kRT, q>(4.0 * atan2(rho, az) / kPi - 1.0, w);
+        ring_contract<kRT, q>(tab, 4.0 * atan2(rho, az) / kPi - 1.0, w);
         const double lp = log(0.5 * (d + az));
         const double gp = rho / (d * (d + az));
         const double inv_d2 = 2.0 / d;
@@ -112,7 +113,7 @@ k_wave_delh_ring(int* __restrict__ fall, const double* __restrict__ geom, int64_
 }
 
 template <int q>
-cudaError_t launch_ring(const Batch& bt, const double* d_k, int m, const double* SR, const double* DR,
+cudaError_t launch_ring(const Batch& bt, const double* tab, const double* d_k, int m, const double* SR, const double* DR,
                         double2* S64, double2* D64, float2* Dlo, double2* tape, int* fall)
 {
     const cudaError_t e = cudaFuncSetAttribute(k_wave_delh_ring<q>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -120,25 +121,20 @@ cudaError_t launch_ring(const Batch& bt, const double* d_k, int m, const double*
     if (e != cudaSuccess) return e;
     const int cols = ring_cols(bt.n);
     k_wave_delh_ring<q><<<dim3((unsigned)((bt.n + kRT - 1) / kRT), (unsigned)((bt.n + cols - 1) / cols)), kRT, ring_smem(q), bt.ctx->stream>>>(
-        fall, bt.m->geom, bt.n, bt.direct, cols, d_k, m, SR, DR, S64, D64, Dlo, tape);
+        fall, bt.m->geom, bt.n, bt.direct, cols, tab, d_k, m, SR, DR, S64, D64, Dlo, tape);
     bt.ctx->launches += 1;
     return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t launch_wave_rings(const Batch& bt, const double* d_k, int m, const double* SR, const double* DR,
-                              double2* S64, double2* D64, float2* Dlo, double2* tape, int* fall)
+cudaError_t launch_wave_rings(const Batch& bt, const double* tab, const double* d_k, int m, const double* SR,
+                              const double* DR, double2* S64, double2* D64, float2* Dlo, double2* tape, int* fall)
 {
-    cudaError_t e = launch_ring<0>(bt, d_k, m, SR, DR, S64, D64, Dlo, tape, fall);
-    if (e == cudaSuccess) e = launch_ring<1>(bt, d_k, m, SR, DR, S64, D64, Dlo, tape, fall);
-    if (e == cudaSuccess) e = launch_ring<2>(bt, d_k, m, SR, DR, S64, D64, Dlo, tape, fall);
+    cudaError_t e = launch_ring<0>(bt, tab, d_k, m, SR, DR, S64, D64, Dlo, tape, fall);
+    if (e == cudaSuccess) e = launch_ring<1>(bt, tab, d_k, m, SR, DR, S64, D64, Dlo, tape, fall);
+    if (e == cudaSuccess) e = launch_ring<2>(bt, tab, d_k, m, SR, DR, S64, D64, Dlo, tape, fall);
     return e;
-}
-
-cudaError_t upload_ring_constants(mh_ctx* ctx, const RingTable& rings)
-{
-    return cudaMemcpyToSymbolAsync(c_rings, &rings, sizeof(rings), 0, cudaMemcpyHostToDevice, ctx->stream);
 }
 
 }  // namespace mh

@@ -6,17 +6,21 @@
 // all four are dropped; the first ring_head rows keep ring_nv(q, 0) of them and
 // the others ring_nv(q, 1) (row lengths fall from 25 to 3 in the first ring).
 // Error against the quadrature ~5e-14.
-// The coefficients sit in constant memory, which broadcasts the one that every
-// thread of a warp reads; one copy per translation unit that includes this,
-// written when a context builds its table (every context writes the same).
 // 2997 panels x 24 frequencies, us: 7265 with the coefficients read from global
-// memory (two 16-byte loads per column bound it), 4294 from constant memory
-// with a loop of its own length for every row, 4004 with these fixed lengths, 2414
-// with the pairs listed first (mh_rings.cu), 2232 with the Chebyshev values in
-// registers instead of Clenshaw's recurrence.
+// memory a thread at a time (two 16-byte loads per column bound it), 4004 from
+// constant memory, 2414 with the pairs listed first (mh_rings.cu), 2232 with the
+// Chebyshev values in registers instead of Clenshaw's recurrence, 1786 with the
+// matrix instruction (mh_contract.cuh).
+// The polar patch has the same form for these kernels: its rows in powers of
+// u = 2 R / kTabRPolar - 1.  After the alpha contraction each function is a
+// degree-14 polynomial in u whose coefficients sum to less than 6 in absolute
+// value (the Chebyshev coefficients decay faster than the basis change grows
+// them), so Horner's rule in u is as accurate as Clenshaw's recurrence and takes
+// one FMA per term instead of two operations.
 #pragma once
 #include "mh_internal.h"
 #include "mh_device.cuh"
+#include "mh_contract.cuh"
 
 namespace mh {
 
@@ -31,20 +35,17 @@ constexpr __host__ __device__ int ring_nv(int q, int tail)                      
 {
     return tail ? (q == 0 ? 19 : q == 1 ? 24 : 29) : (q == 0 ? 25 : q == 1 ? 30 : 36);
 }
-// column of row m's first coefficient in the packed table
-constexpr __host__ __device__ int ring_at(int q, int m)
+// The fragments (mh_contract.cuh) follow the table's cells: the polar patch, then
+// each ring's tiles with a row of full length and its others.
+constexpr int kFragPolar = kTabWords;
+constexpr __host__ __device__ int ring_head_tiles(int q) { return frag_tiles(ring_head(q)); }
+constexpr __host__ __device__ int ring_frags(int q, int tail)  // first word
 {
-    const int h = ring_head(q), head = (m < h ? m : h) * ring_nv(q, 0), tail = (m > h ? m - h : 0) * ring_nv(q, 1);
-    return (q ? ring_at(q - 1, ring_nu(q - 1)) : 0) + head + tail;
+    return tail ? ring_frags(q, 0) + frag_words(ring_head(q), ring_nv(q, 0))
+         : q    ? ring_frags(q - 1, 1) + frag_words(ring_nu(q - 1) - 4 * ring_head_tiles(q - 1), ring_nv(q - 1, 1))
+                : kFragPolar + frag_words(kTabNU, kTabNV);
 }
-
-// The packed rings: coefficient (row m, column j, function f) of ring q at
-// 4 (ring_at(q, m) + j) + f.
-struct RingTable {
-    double coef[4 * ring_at(kRings - 1, ring_nu(kRings - 1))];
-};
-
-static __constant__ RingTable c_rings;
+constexpr int kTabAllWords = ring_frags(kRings, 0);
 
 // Whether R belongs to ring q, with margins of 1e-12 that let a pair on an edge
 // be written by one kernel at least, whatever the rounding of R in each.
@@ -54,35 +55,30 @@ __device__ __forceinline__ bool ring_in(int q, double R)
     return R >= lo * (1.0 - 1e-12) && R < 2.0 * lo * (1.0 + 1e-12);
 }
 
-// Rows m0 .. m1 - 1 of ring q (of NV columns each) contracted with t[j] = T_j(v).
-template <int T, int q, int NV, int m0, int m1, int N>
-__device__ __forceinline__ void ring_contract_rows(const double (&t)[N], double* __restrict__ w)
-{
-#pragma unroll 1
-    for (int row = m0; row < m1; ++row) {
-        const int c = 4 * (ring_at(q, m0) + (row - m0) * NV);
-        double b[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-        for (int col = 0; col < NV; ++col)
-#pragma unroll
-            for (int f = 0; f < 4; ++f) b[f] = fma(c_rings.coef[c + 4 * col + f], t[col], b[f]);
-#pragma unroll
-        for (int f = 0; f < 4; ++f) w[(4 * row + f) * T] = b[f];
-    }
-}
-
-// The alpha direction of ring q contracted at v: w[(4 row + f) T], f = B, C,
-// E0, E1, the coefficients of u^row (T threads' columns side by side).
+// The alpha direction of ring q contracted at the warp's 32 v: w[w_at<T>(4 row +
+// f, column)], f = B, C, E0, E1, the coefficients of u^row.  The whole warp takes
+// part; it writes the columns of its own threads only.
 template <int T, int q>
-__device__ __forceinline__ void ring_contract(double v, double* __restrict__ w)
+__device__ __forceinline__ void ring_contract(const double* __restrict__ tab, double v, double* __restrict__ w)
 {
-    double t[ring_nv(q, 0)];
-    cheb_values(v, t);
-    ring_contract_rows<T, q, ring_nv(q, 0), 0, ring_head(q)>(t, w);
-    ring_contract_rows<T, q, ring_nv(q, 1), ring_head(q), ring_nu(q)>(t, w);
+    constexpr int kHead = ring_head_tiles(q), kTail = frag_tiles(ring_nu(q) - 4 * kHead);
+    const int base = threadIdx.x & ~31;
+    const auto store = [&](int m, int p, double a, double b) {
+        if (m < 4 * ring_nu(q)) *reinterpret_cast<double2*>(w + w_at<T>(m, base + p)) = make_double2(a, b);
+    };
+    __syncwarp();  // the last pairs' columns are read
+#pragma unroll 1
+    for (int g = 0; g < 4; g += 2) {
+        double t[2][frag_steps(ring_nv(q, 0))];
+        cheb_frags(v, g, t);
+        contract_tiles<kHead, frag_steps(ring_nv(q, 0))>(tab + ring_frags(q, 0), g, t, store);
+        contract_tiles<kTail, frag_steps(ring_nv(q, 1))>(
+            tab + ring_frags(q, 1), g, t, [&](int m, int p, double a, double b) { store(16 * kHead + m, p, a, b); });
+    }
+    __syncwarp();
 }
 
-// The four functions at Z values of R in ring q, from its contraction.
+// The four functions at Z values of R in ring q, from the calling thread's column.
 template <int T, int Z, int q>
 __device__ __forceinline__ void ring_values(const double* __restrict__ w, const double R[Z], double val[Z][4])
 {
@@ -90,9 +86,10 @@ __device__ __forceinline__ void ring_values(const double* __restrict__ w, const 
     double u[Z];
 #pragma unroll
     for (int t = 0; t < Z; ++t) u[t] = 2.0 * kInvLo * R[t] - 3.0;  // hi = 2 lo
+    const int tid = threadIdx.x;
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
-        const double c = w[(4 * (ring_nu(q) - 1) + f) * T];
+        const double c = w[w_at<T>(4 * (ring_nu(q) - 1) + f, tid)];
 #pragma unroll
         for (int t = 0; t < Z; ++t) val[t][f] = c;
     }
@@ -100,7 +97,7 @@ __device__ __forceinline__ void ring_values(const double* __restrict__ w, const 
     for (int row = ring_nu(q) - 2; row >= 0; --row)
 #pragma unroll
         for (int f = 0; f < 4; ++f) {
-            const double c = w[(4 * row + f) * T];
+            const double c = w[w_at<T>(f, tid) + 4 * row * T];
 #pragma unroll
             for (int t = 0; t < Z; ++t) val[t][f] = fma(val[t][f], u[t], c);
         }

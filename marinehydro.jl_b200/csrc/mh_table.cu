@@ -94,6 +94,13 @@ std::vector<double> cheb_to_powers(int n)
     return P;
 }
 
+// Where A[m][j] of the fragments that start at word `first` belongs (mh_contract.cuh).
+size_t frag_at(int first, int cols, int m, int j)
+{
+    const int lane = 4 * (m % 8) + j % 4;
+    return (size_t)first + 64 * ((m / 16) * frag_steps(cols) + j / 4) + 2 * lane + (m % 16) / 8;
+}
+
 }  // namespace
 
 int ensure_delh_table(mh_ctx* ctx)
@@ -143,13 +150,13 @@ int ensure_delh_table(mh_ctx* ctx)
     if (cudaMalloc(&d_r, bytes) != cudaSuccess || cudaMalloc(&d_z, bytes) != cudaSuccess ||
         cudaMalloc(&d_B, bytes) != cudaSuccess || cudaMalloc(&d_C, bytes) != cudaSuccess ||
         cudaMalloc(&d_E0, bytes) != cudaSuccess || cudaMalloc(&d_E1, bytes) != cudaSuccess ||
-        cudaMalloc(&d_tab, sizeof(double) * kTabWords) != cudaSuccess) {
+        cudaMalloc(&d_tab, sizeof(double) * kTabAllWords) != cudaSuccess) {
         cudaGetLastError();
         cleanup();
         cudaFree(d_tab);
         return set_err(ctx, MH_ERR_OOM, "allocation of the Delhommeau table failed");
     }
-    std::vector<double> hB(n), hC(n), hE0(n), hE1(n), tab(kTabWords);
+    std::vector<double> hB(n), hC(n), hE0(n), hE1(n), tab(kTabAllWords);
     cudaError_t e = cudaMemcpyAsync(d_r, r.data(), bytes, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_z, z.data(), bytes, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) {
@@ -168,8 +175,9 @@ int ensure_delh_table(mh_ctx* ctx)
         return set_err(ctx, MH_ERR_CUDA, "Delhommeau table nodes: %s", cudaGetErrorString(e));
     }
     // polar block: B, C, E0, E1, fitted on kTabNP x kTabNP nodes; the first
-    // kTabNU rows (degrees in R) are kept, and again with the rows in the
-    // monomial basis of u: T_i(u) = sum_m P[i][m] u^m
+    // kTabNU rows (degrees in R) are kept, and again as fragments with the rows
+    // in the monomial basis of u: T_i(u) = sum_m P[i][m] u^m
+    std::vector<float> mono(4 * kTabPolarFn);
     {
         std::vector<double> full((size_t)kTabNP * kTabNP);
         const std::vector<double> P = cheb_to_powers(kTabNU);
@@ -183,7 +191,8 @@ int ensure_delh_table(mh_ctx* ctx)
                 for (int j = 0; j < kTabNV; ++j) {
                     double a = 0.0;
                     for (int i = m; i < kTabNU; ++i) a += P[(size_t)i * kTabNU + m] * full[(size_t)i * kTabNP + j];
-                    tab[kTabMonoOff + (size_t)q * kTabPolarFn + m * kTabNV + j] = a;
+                    tab[frag_at(kFragPolar, kTabNV, 4 * m + q, j)] = a;
+                    mono[4 * (m * kTabNV + j) + q] = (float)a;
                 }
         }
     }
@@ -194,8 +203,7 @@ int ensure_delh_table(mh_ctx* ctx)
         cheb_coeffs(kTabNC, kTabNC, hB.data() + np + (size_t)c * nc, dst);
         cheb_coeffs(kTabNC, kTabNC, hC.data() + np + (size_t)c * nc, dst + nc);
     }
-    // rings: the same four functions, rows in powers of u, packed
-    auto rings = std::make_unique<RingTable>();
+    // rings: the same four functions, rows in powers of u
     size_t at = (size_t)np + (size_t)kTabNCell * kTabNCell * nc;
     for (int q = 0; q < kRings; ++q) {
         const int fr = ring_fit_r(q), fa = ring_fit_a(q), nu = ring_nu(q);
@@ -210,21 +218,18 @@ int ensure_delh_table(mh_ctx* ctx)
                     double a = 0.0;
                     for (int i = m; i < nu; ++i)
                         if (j < ring_nv(q, i >= ring_head(q))) a += P[(size_t)i * nu + m] * full[(size_t)i * fa + j];
-                    rings->coef[4 * (size_t)(ring_at(q, m) + j) + f] = a;
+                    const int head = 4 * ring_head_tiles(q), tail = m >= head;
+                    tab[frag_at(ring_frags(q, tail), ring_nv(q, tail), 4 * (m - (tail ? head : 0)) + f, j)] = a;
                 }
         }
     }
-    std::vector<double> mono(4 * kTabPolarFn);  // the functions of a (row, column) side by side
-    for (int i = 0; i < kTabPolarFn; ++i)
-        for (int q = 0; q < 4; ++q) mono[4 * i + q] = tab[kTabMonoOff + q * kTabPolarFn + i];
-    if (e == cudaSuccess) e = upload_wave_constants(ctx, mono.data(), *rings);
-    if (e == cudaSuccess) e = upload_tangent_constants(ctx, mono.data(), *rings);
+    e = upload_wave_constants(ctx, mono.data());
     if (e != cudaSuccess) {
         cleanup();
         cudaFree(d_tab);
         return set_err(ctx, MH_ERR_CUDA, "Delhommeau constants: %s", cudaGetErrorString(e));
     }
-    e = cudaMemcpyAsync(d_tab, tab.data(), sizeof(double) * kTabWords, cudaMemcpyHostToDevice,
+    e = cudaMemcpyAsync(d_tab, tab.data(), sizeof(double) * kTabAllWords, cudaMemcpyHostToDevice,
                         ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     cleanup();
