@@ -362,15 +362,18 @@ int mh_ctx_create(int device, mh_ctx** out)
     cublasSetStream(ctx->cublas, ctx->stream);
     cusolverDnSetStream(ctx->cusolver, ctx->stream);
     // LU schedules the autotuner chose on a B200 (mh_lu_autotune, median of
-    // three sweeps over groups 1-4 x 2-8 panels per outer step x both update
-    // kernels; ms against the default 2 x 4): 512 panels x 16 matrices, 1
-    // group x 4 panels with C staged in tensor memory (0.555 vs 0.651);
-    // 1024 x 64, 1 x 4 (1.730 vs 1.736; 1.232 vs 1.413 at 1024 x 16); 1536
-    // x 16, 1 x 4 (2.00 vs 2.20); 2048 x 64, 2 x 8 (5.67 vs 6.27).  Other
-    // sizes take the nearest entry; mh_ctx_set_lu_schedule or the autotuner
-    // replace them.
-    ctx->lu_table = {{512, LuSchedule{1, 4, 1}}, {1024, LuSchedule{1, 4, 0}}, {1536, LuSchedule{1, 4, 0}},
-                     {2048, LuSchedule{2, 8, 0}}};
+    // three to seven sweeps; ms against the next best): 512 panels x 16 matrices, 1
+    // group x 4 panels with C staged in tensor memory (0.378 vs 0.379); 1224 x 16, 1
+    // x 4 (1.09 vs 1.10); 2048 x 64, 2 x 8 (4.68; 4.88 vs 5.03 for 2 x 6 in one run).  Other sizes
+    // take the nearest entry.  The number of matrices decides between one group,
+    // whose chain of panels is the critical path, and two, which overlap each
+    // other's: the line is at kLuFewColumns columns in all.  Two for one above it:
+    // 1024 x 64 1.30 vs 1.40, 1456 x 32 1.78 vs 1.79; 1 x 4 for 2 x 8 up to it: 2048
+    // x 1 1.61 vs 1.80, x 8 1.80 vs 2.22, x 16 2.22 vs 2.41, 2997 x 8 3.30 vs 3.60,
+    // 4096 x 4 4.09 vs 4.75 (past it 2997 x 16 4.92 vs 4.64, 4096 x 12 6.89 vs 6.35).
+    // mh_ctx_set_lu_schedule or the autotuner replace them.
+    ctx->lu_table = {{512, LuSchedule{1, 4, 1}}, {1024, LuSchedule{1, 4, 0, 0, 2}}, {1536, LuSchedule{1, 4, 0, 0, 2}},
+                     {2048, LuSchedule{2, 8, 0, 4, 0}}};
     *out = ctx;
     return MH_OK;
 }

@@ -70,7 +70,10 @@ constexpr int kLuGroups = 4;
 // Schedule of the tensor-core LU: groups of matrices on their own stream
 // pairs (1 .. kLuGroups), 64-column panels per outer step (even, 2 .. 8) and
 // the trailing-update kernel (0: C through shared memory after the MMAs,
-// 1: C staged in tensor memory before them).
+// 1: C staged in tensor memory before them).  Built-in entries also say what
+// replaces them by a call's columns in all (n x matrices), if not 0: few_outer, one
+// group with that many panels per outer step up to kLuFewColumns; many_groups, that
+// many groups above it.
 // The streams and events one group of the tensor-core LU runs on.
 struct LuStreams {
     cudaStream_t main, side, strip;
@@ -81,7 +84,10 @@ struct LuSchedule {
     int groups = 2;
     int outer = 4;
     int update = 0;
+    int few_outer = 0;
+    int many_groups = 0;
 };
+constexpr int64_t kLuFewColumns = 32768;
 
 struct mh_ctx {
     int device = 0;

@@ -11,6 +11,7 @@
 //                      factors into the matrix and the FP16 operand panels of
 //                      the update, pre-packed as their shared-memory images
 //                      at absolute 128-row (column) tile slots;
+//   k_lu_block_tc      the next diagonal block's own update, for few matrices;
 //   k_lu_update_tc     A22 -= sum_p L21_p U12_p over panel pairs: the
 //                      packed panels arrive by cp.async.bulk (no register
 //                      staging), sixteen MMAs per pair accumulate in TMEM.
@@ -94,10 +95,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t phase)
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
             "selp.b32 %0, 1, 0, p;\n\t}\n"
             : "=r"(done)
-            : "r"(addr), "r"(phase), "r"(kWaitHintNs)
+            : "r"(addr), "r"(phase)
             : "memory");
         if (done) return true;
     }
@@ -184,17 +185,19 @@ __device__ __forceinline__ void mma_k128(uint32_t tmem, uint32_t a0, uint32_t lb
 // columns 128..255 as A_s B_(s+4 mod 8) (Re L Im U + Im L Re U); then commit
 // to `bar`.  The first MMAs overwrite the accumulator unless `accumulate`.
 // B holds each of Re U12, Im U12 once: 32 KB per pair instead of the 64 KB
-// of a [Re -Im; Im Re] image.
+// of a [Re -Im; Im Re] image.  N columns (the imaginary part follows them in
+// tensor memory), K chunks LBO bytes apart.
+template <uint32_t N = TC_TN, uint32_t LBO = kLboA>
 __device__ __forceinline__ void mma_cplx(uint32_t tmem, uint32_t a0, uint32_t b0, uint32_t bar, bool accumulate)
 {
-    constexpr uint32_t kNegA = 1u << 13;
+    constexpr uint32_t kNegA = 1u << 13, kIdesc = (kIdescN128 & ~(63u << 17)) | (N >> 3 << 17);
 #pragma unroll
     for (int s = 0; s < TC_KR / 16; ++s) {
-        const uint64_t da = umma_desc(a0 + 2 * s * kLboA, kLboA, kSbo);
-        const uint64_t dre = umma_desc(b0 + 2 * s * kLboB128, kLboB128, kSbo);
-        const uint64_t dim = umma_desc(b0 + 2 * ((s + 4) & 7) * kLboB128, kLboB128, kSbo);
+        const uint64_t da = umma_desc(a0 + 2 * s * LBO, LBO, kSbo);
+        const uint64_t dre = umma_desc(b0 + 2 * s * LBO, LBO, kSbo);
+        const uint64_t dim = umma_desc(b0 + 2 * ((s + 4) & 7) * LBO, LBO, kSbo);
         const uint32_t acc = (s > 0 || accumulate) ? 1u : 0u;
-        const uint32_t idre = kIdescN128 | (s >= 4 ? kNegA : 0u);
+        const uint32_t idre = kIdesc | (s >= 4 ? kNegA : 0u);
         asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n"
@@ -202,7 +205,7 @@ __device__ __forceinline__ void mma_cplx(uint32_t tmem, uint32_t a0, uint32_t b0
         asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n"
-            :: "r"(tmem + (uint32_t)TC_TN), "l"(da), "l"(dim), "r"(kIdescN128), "r"(acc), "r"(0u), "r"(0u),
+            :: "r"(tmem + N), "l"(da), "l"(dim), "r"(kIdesc), "r"(acc), "r"(0u), "r"(0u),
                "r"(0u), "r"(0u));
     }
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
@@ -457,11 +460,12 @@ __device__ __forceinline__ bool epilogue_bulk(float2* M, int64_t n, int64_t r0, 
 // mode 1: the first w tile rows and tile columns (an L of width w; w (2 ntile
 // - w) tiles, the part the next panels depend on; tile x of the L is
 // blockIdx.x + xoff, tile 0 being the diagonal tile (t0, t0)); mode 2: the
-// tiles past them (grid (ntile - w)^2).
+// tiles past them (grid (ntile - w)^2).  Entries with both indices below skip are
+// not written (k_lu_block_tc updates them meanwhile).
 __global__ void __launch_bounds__(128, 2)
 k_lu_update_tc(float2* __restrict__ Ab, int64_t n, int64_t stride, int t0, int ntile, int mode, int w,
                PanelPairs pp, int npair, int64_t pstride, int64_t lo, int* __restrict__ bad,
-               int xoff)
+               int xoff, int64_t skip)
 {
     extern __shared__ __align__(1024) unsigned char tc_smem[];
     __shared__ uint64_t mbar[2 + kCBufs];
@@ -499,11 +503,13 @@ k_lu_update_tc(float2* __restrict__ Ab, int64_t n, int64_t stride, int t0, int n
     // a tile wholly inside the trailing matrix (and n even, so every column
     // of it starts on a 16-byte boundary) goes through shared memory by bulk
     // copies after the MMAs; other tiles use per-thread loads and stores
-    const bool full = r0 >= lo && c0 >= lo && r0 + TC_TM <= n && c0 + TC_TN <= n && (n & 1) == 0;
+    const bool full = r0 >= lo && c0 >= lo && (r0 >= skip || c0 >= skip) && r0 + TC_TM <= n &&
+                      c0 + TC_TN <= n && (n & 1) == 0;
     // this thread's row of C does not depend on the products: its first 16
     // columns are loaded while the panel copies and the MMAs run
     const int64_t gi = r0 + warp * 32 + lane;
     const bool row_ok = gi >= lo && gi < n;
+    const int64_t col0 = gi >= skip ? lo : skip;  // first column stored in this row
     constexpr int kEc = 16;  // columns per epilogue chunk
     float2 cv[kEc];
     if (!full) {
@@ -572,7 +578,7 @@ k_lu_update_tc(float2* __restrict__ Ab, int64_t n, int64_t stride, int t0, int n
 #pragma unroll
                 for (int q = 0; q < kEc; ++q, pc += n) {
                     const int64_t gj = c0 + cc * kEc + q;
-                    if (gj >= lo && gj < n)
+                    if (gj >= col0 && gj < n)
                         *pc = make_float2(cv[q].x - __uint_as_float(re[q]), cv[q].y - __uint_as_float(im[q]));
                 }
             }
@@ -601,7 +607,7 @@ k_lu_update_tc(float2* __restrict__ Ab, int64_t n, int64_t stride, int t0, int n
 __global__ void __launch_bounds__(128, 2)
 k_lu_update_tc_acc(float2* __restrict__ Ab, int64_t n, int64_t stride, int t0, int ntile, int mode, int w,
                    PanelPairs pp, int npair, int64_t pstride, int64_t lo, int* __restrict__ bad,
-               int xoff)
+               int xoff, int64_t skip)
 {
     extern __shared__ __align__(1024) unsigned char tc_smem[];
     __shared__ uint64_t mbar[2];
@@ -659,6 +665,7 @@ k_lu_update_tc_acc(float2* __restrict__ Ab, int64_t n, int64_t stride, int t0, i
     // [lo, n) as zeros; they are not stored back)
     const int64_t gi = r0 + warp * 32 + lane;
     const bool row_ok = gi >= lo && gi < n;
+    const int64_t col0 = gi >= skip ? lo : skip;  // first column stored in this row
     constexpr int kEc = 16;
 #pragma unroll 2
     for (int cc = 0; cc < TC_TN / kEc; ++cc) {
@@ -707,7 +714,7 @@ k_lu_update_tc_acc(float2* __restrict__ Ab, int64_t n, int64_t stride, int t0, i
 #pragma unroll
                 for (int q = 0; q < kEc; ++q) {
                     const int64_t gj = c0 + cc * kEc + q;
-                    if (gj >= lo && gj < n)
+                    if (gj >= col0 && gj < n)
                         pc[(int64_t)q * n] = make_float2(-__uint_as_float(re[q]), -__uint_as_float(im[q]));
                 }
             }
@@ -721,6 +728,115 @@ k_lu_update_tc_acc(float2* __restrict__ Ab, int64_t n, int64_t stride, int t0, i
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, kTmemCols);
+}
+
+// The next diagonal block alone, rows and columns lo .. lo + 63 (lo a multiple of
+// 64): the part of the update that the next factorisation waits for, on the
+// critical path of a call with few matrices.  The products of the block's 64
+// rows of L and 64 columns of U, a quarter of a tile's: kBlkStages pairs' operands
+// (16 KB each, 1 KB pieces of the packed images, one per lane of warp 0) are in
+// flight at once, the block of C is in registers before the products are done,
+// and there is no staging of C.  The MMAs keep M = 128; their rows 64 .. 127 read
+// whatever follows in shared memory and are not used.  One matrix of 2048, us: 6.5
+// for one pair and 16.7 for ten (k_lu_update_tc on the block's tile: 10.3 and 18.9,
+// the same a pair: the copies' latency).
+constexpr int kBlkStages = 3;
+constexpr uint32_t kBlkImage = TC_NB * TC_KR * 2;  // 16 KB: 64 rows, K = 128
+constexpr uint32_t kBlkSmem = kBlkStages * 2 * kBlkImage;
+constexpr uint32_t kBlkLbo = (TC_NB / 8) * 128;
+
+__global__ void __launch_bounds__(64)
+k_lu_block_tc(float2* __restrict__ Ab, int64_t n, int64_t stride, PanelPairs pp, int npair, int64_t pstride,
+              int64_t lo, int* __restrict__ bad)
+{
+    extern __shared__ __align__(1024) unsigned char tc_smem[];
+    __shared__ uint64_t full_bar[kBlkStages], used_bar[kBlkStages];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int done;
+    const int b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float2* C = Ab + (int64_t)b * stride + lo * n + lo;
+    if (warp == 0) tmem_alloc(&tmem_slot, 2 * TC_NB);
+    if (tid == 0)
+        for (int q = 0; q < kBlkStages; ++q) {
+            mbar_init(&full_bar[q]);
+            mbar_init(&used_bar[q]);
+        }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    // chunk `lane % 16` of the pair's L (lanes 0 .. 15) or U image
+    const int64_t src = (int64_t)b * pstride + (lo / TC_TM) * (int64_t)(lane < 16 ? kPanelL : kPanelU) +
+                        (lane & 15) * kLboA + (lo % TC_TM) / 8 * 128;
+    const auto copy = [&](int p) {
+        const uint32_t bar = smem_u32(&full_bar[p % kBlkStages]);
+        if (lane == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                         :: "r"(bar), "r"(2 * kBlkImage) : "memory");
+        __syncwarp();
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     :: "r"(smem_u32(tc_smem) + (p % kBlkStages) * 2 * kBlkImage + lane * kBlkLbo),
+                        "l"((lane < 16 ? pp.L[p] : pp.U[p]) + src), "r"(kBlkLbo), "r"(bar) : "memory");
+    };
+    if (warp == 0)
+        for (int p = 0; p < min(npair, kBlkStages); ++p) copy(p);
+    float2 c[TC_NB];
+#pragma unroll
+    for (int j = 0; j < TC_NB; ++j)
+        c[j] = lo + tid < n && lo + j < n ? C[j * n + tid] : make_float2(0.f, 0.f);
+    if (warp == 0) {
+        bool ok = true;
+        int p = 0;      // pairs whose MMAs are issued
+        int sent = min(npair, kBlkStages);
+        for (; p < npair; ++p) {
+            const int q = p % kBlkStages;
+            const uint32_t ph = (uint32_t)(p / kBlkStages & 1);
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&full_bar[q]), ph));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a0 = smem_u32(tc_smem) + q * 2 * kBlkImage;
+            if (lane == 0)
+                mma_cplx<TC_NB, kBlkLbo>(tmem, a0, a0 + kBlkImage, smem_u32(&used_bar[q]), p > 0);
+            __syncwarp();
+            if (sent < npair) {  // this buffer takes the pair kBlkStages on
+                ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&used_bar[q]), ph));
+                if (!ok) {
+                    ++p;
+                    break;
+                }
+                copy(sent++);
+            }
+        }
+        if (p > 0) {  // the last MMAs issued are done after all before them
+            const bool last = mbar_wait(smem_u32(&used_bar[(p - 1) % kBlkStages]), (uint32_t)((p - 1) / kBlkStages & 1));
+            ok = __all_sync(0xffffffffu, last) && ok;
+        }
+        for (int r = p; r < sent; ++r)  // not ok: bounded, for what is in flight
+            mbar_wait(smem_u32(&full_bar[r % kBlkStages]), (uint32_t)(r / kBlkStages & 1));
+        if (lane == 0) done = ok;
+    }
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (done) {
+        const uint32_t base = tmem + ((uint32_t)(warp * 32) << 16);
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            uint32_t re[16], im[16];
+            tmem_ld16(base + 16 * h, re);
+            tmem_ld16(base + TC_NB + 16 * h, im);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                if (lo + tid < n && lo + 16 * h + j < n)
+                    C[(16 * h + j) * n + tid] = make_float2(c[16 * h + j].x - __uint_as_float(re[j]),
+                                                            c[16 * h + j].y - __uint_as_float(im[j]));
+        }
+    } else if (lane == 0) {
+        atomicExch(bad + b, 2);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem, 2 * TC_NB);
 }
 
 // ---------------------------------------------------------------------------
@@ -1569,7 +1685,8 @@ namespace {
 // The schedule above for nbatch matrices on one (main, side) stream pair;
 // panels: lu_panel_bytes_tc(n) * nbatch bytes for these matrices.
 cudaError_t lu_tc_group(mh_ctx* ctx, float2* A, int64_t n, int64_t stride, int nbatch, float2* Dinv,
-                        unsigned char* panels, int* bad, const LuStreams& st, const int op, const int update)
+                        unsigned char* panels, int* bad, const LuStreams& st, const int op, const int update,
+                        const bool alone)
 {
     auto* upd = update ? k_lu_update_tc_acc : k_lu_update_tc;
     cudaError_t e;
@@ -1584,20 +1701,33 @@ cudaError_t lu_tc_group(mh_ctx* ctx, float2* A, int64_t n, int64_t stride, int n
     if ((e = cudaEventRecord(st.ev_side, side_s)) != cudaSuccess) return e;
     if ((e = cudaEventRecord(st.ev_strip_done, strip_s)) != cudaSuccess) return e;
     // An L of the trailing matrix (mode 1 at tile t0, width w) updated with
-    // the panel pairs q: its diagonal tile (t0, t0), which holds the next
-    // diagonal block, on the main stream; the rest on the strip stream,
-    // concurrently with the next diagonal-block factorisation; the next panel
-    // solve waits for it (strip_join).
+    // the panel pairs q: the part with the next diagonal block, at lo, on the
+    // main stream; the rest on the strip stream, concurrently with the next
+    // diagonal-block factorisation; the next panel solve waits for it
+    // (strip_join).  Where these matrices have the device to themselves (alone: one
+    // group) and the rest is one wave of its CTAs, so that the main stream is the
+    // critical path, that part is the block alone (k_lu_block_tc), else the whole
+    // diagonal tile, which is then passed over once: LU ms, block and tile, 1224 x
+    // 16 matrices 1.087 and 1.158, 870 x 16 0.714 and 0.769, 2048 x 8 1.785 and
+    // 1.932, but in two groups 2048 x 64 5.054 and 4.836, 2997 x 24 5.88 and 5.73.
+    // (The rest could start beside the block already, but then it holds the SMs
+    // first and the factorisations, one CTA each, share theirs with it: 38 us for 27.)
     auto strip = [&](int t0, int nt, int w, const PanelPairs& q, int np, int64_t lo) -> cudaError_t {
         cudaError_t e2;
-        upd<<<dim3(1, 1, nbz), 128, kTcSmemBytes, main_s>>>(A, n, stride, t0, nt, 1, w, q, np, pstride, lo, bad, 0);
+        const bool block = alone && (int64_t)(w * (2 * nt - w) - 1) * nbatch <= 2 * 148;
+        const int own = block && lo % TC_TM == 0 && n > lo + TC_NB;  // the block's tile holds more than the block
+        if (block)
+            k_lu_block_tc<<<nbz, 64, kBlkSmem, main_s>>>(A, n, stride, q, np, pstride, lo, bad);
+        else
+            upd<<<dim3(1, 1, nbz), 128, kTcSmemBytes, main_s>>>(A, n, stride, t0, nt, 1, w, q, np, pstride, lo, bad, 0,
+                                                                lo);
         ctx->launches += 1;
-        const int rest = w * (2 * nt - w) - 1;
+        const int rest = w * (2 * nt - w) - 1 + own;
         if (rest > 0) {
             if ((e2 = cudaEventRecord(st.ev_strip_go, main_s)) != cudaSuccess) return e2;
             if ((e2 = cudaStreamWaitEvent(strip_s, st.ev_strip_go, 0)) != cudaSuccess) return e2;
             upd<<<dim3(rest, 1, nbz), 128, kTcSmemBytes, strip_s>>>(A, n, stride, t0, nt, 1, w, q, np, pstride, lo,
-                                                                    bad, 1);
+                                                                    bad, 1 - own, own ? lo + TC_NB : lo);
             ctx->launches += 1;
             if ((e2 = cudaEventRecord(st.ev_strip_done, strip_s)) != cudaSuccess) return e2;
         }
@@ -1674,7 +1804,7 @@ cudaError_t lu_tc_group(mh_ctx* ctx, float2* A, int64_t n, int64_t stride, int n
         const int w = std::min(kW, nt);
         if (nt > w) {
             upd<<<dim3(nt - w, nt - w, nbz), 128, kTcSmemBytes, side_s>>>(
-                A, n, stride, t0, nt, 2, w, pp, op, pstride, lo, bad, 0);
+                A, n, stride, t0, nt, 2, w, pp, op, pstride, lo, bad, 0, lo);
             ctx->launches += 1;
         }
         if ((e = cudaEventRecord(st.ev_side, side_s)) != cudaSuccess) return e;
@@ -1707,7 +1837,13 @@ cudaError_t launch_lu_tc(mh_ctx* ctx, float2* A, int64_t n, int64_t stride, int 
     cudaError_t e;
     static_assert(TC_NB == 64, "the diagonal blocks are factored by k_lu_diag64");
     static_assert(TC_TM == 2 * TC_NB && TC_TN == TC_TM, "two panels per 128-wide tile");
-    const LuSchedule sched = ctx->lu_schedule(n);
+    LuSchedule sched = ctx->lu_schedule(n);
+    const bool few = n * nbatch <= kLuFewColumns;
+    if (sched.few_outer && few) {
+        sched.groups = 1;
+        sched.outer = sched.few_outer;
+    }
+    if (sched.many_groups && !few) sched.groups = sched.many_groups;
     if (sched.groups < 1 || sched.groups > kLuGroups || sched.outer < 2 || sched.outer > kOuterMax ||
         (sched.outer & 1) || sched.update < 0 || sched.update > 1)
         return cudaErrorInvalidValue;
@@ -1716,6 +1852,9 @@ cudaError_t launch_lu_tc(mh_ctx* ctx, float2* A, int64_t n, int64_t stride, int 
         return e;
     if ((e = cudaFuncSetAttribute(k_lu_update_tc_acc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(kSmemA + kSmemB))) != cudaSuccess)
+        return e;
+    if ((e = cudaFuncSetAttribute(k_lu_block_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlkSmem)) !=
+        cudaSuccess)
         return e;
     if ((e = cudaFuncSetAttribute(k_lu_trsm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(kSmemA + kSmemA))) != cudaSuccess)
@@ -1740,7 +1879,8 @@ cudaError_t launch_lu_tc(mh_ctx* ctx, float2* A, int64_t n, int64_t stride, int 
         st.ev_strip_go = ctx->lu_ev_strip_go[g];
         st.ev_strip_done = ctx->lu_ev_strip_done[g];
         if ((e = lu_tc_group(ctx, A + (int64_t)b0 * stride, n, stride, nbg, Dinv + (int64_t)b0 * dstride,
-                             panels + (int64_t)b0 * pbytes, bad + b0, st, sched.outer, sched.update)) != cudaSuccess)
+                             panels + (int64_t)b0 * pbytes, bad + b0, st, sched.outer, sched.update, groups == 1)) !=
+            cudaSuccess)
             return e;
         b0 += nbg;
     }
