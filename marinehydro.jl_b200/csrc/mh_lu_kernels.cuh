@@ -175,10 +175,10 @@ __device__ __forceinline__ void pack_trsm_b(const __half2 (*x)[LD], unsigned cha
 // right what inv(U) needs; what it makes of the entries that have left is never
 // read.  The pivot block is factored and inverted by the same elimination, one
 // pivot at a time.
-// Thread (ti, tj) of 16 x 16 holds the entries (ti + 16 a, tj + 16 b); a ninth
-// warp does the pivot blocks (two entries per lane, exchanged by shuffles), the
-// next panel's while the others run this panel's update: they hand its eight
-// rows and columns over first.  What bounds it: the 64 dependent pivot steps (a
+// Thread (ti, tj) of 16 x 16 holds the entries (ti + 16 a, tj + 16 b); a warp of
+// its own, with a scheduler of its own, does the pivot blocks (two entries per lane,
+// exchanged by shuffles), the next panel's while the others run this panel's
+// update: they hand its eight rows and columns over first.  What bounds it: the 64 dependent pivot steps (a
 // shuffle, a reciprocal and three products each), one CTA per matrix.
 // The panel loop is not unrolled: with the panel as a compile-time index the
 // code, run once, missed the instruction cache for a third of the time.
@@ -186,9 +186,10 @@ __device__ __forceinline__ void pack_trsm_b(const __half2 (*x)[LD], unsigned cha
 // Same outputs as k_lu_diag.  28 KB of shared memory, so that a CTA fits beside
 // two CTAs of the trailing update on an SM.
 // Measured on a B200: 44 us (panels of eight by one warp, then the inverses by
-// recursive doubling: 36 barriers) -> 26 us a block; 64 matrices of 2048 beside
-// their updates, 60 -> 39 us.
-constexpr int kDiag64Threads = 288;
+// recursive doubling: 36 barriers) -> 25 us a block (26 with the pivot warp on a
+// scheduler that two others use); 64 matrices of 2048 beside their updates, 60 -> 37
+// us.
+constexpr int kDiag64Threads = 320;
 
 __global__ void __launch_bounds__(kDiag64Threads)
 k_lu_diag64(float2* __restrict__ A, int64_t n, int64_t stride, int64_t k0, float2* __restrict__ Dinv,
@@ -207,8 +208,11 @@ k_lu_diag64(float2* __restrict__ A, int64_t n, int64_t stride, int64_t k0, float
     float2* invL = Dinv + b0 * dstride + (k0 / NB) * 2 * NB * NB;
     float2* invU = invL + NB * NB;
     const int kb = (int)min((int64_t)NB, n - k0);
-    const int tid = threadIdx.x, ti = tid & 15, tj = tid >> 4, lane = tid & 31;
-    const bool pivots = tid >= 256;  // the ninth warp
+    // warps 0, 1, 2, 4, 5, 6, 8, 9 hold the block, warp 3 does the pivot blocks with
+    // a scheduler of its own, warp 7 is not used
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tid = 32 * (warp - warp / 4) + lane, ti = tid & 15, tj = tid >> 4;
+    const bool pivots = (warp & 3) == 3;
     const float2 z = make_float2(0.f, 0.f), one = make_float2(1.f, 0.f);
     float2 X[4][4];
     if (!pivots) {
@@ -229,7 +233,7 @@ k_lu_diag64(float2* __restrict__ A, int64_t n, int64_t stride, int64_t k0, float
     for (int K = -8; K < NB; K += 8) {
         if (pivots) {
             const int N = K + 8;  // the panel after K
-            if (N < NB) {
+            if (warp == 3 && N < NB) {
                 // lane (i, g) holds the entries (i, g) and (i, g + 4) of the pivot block
                 const int i = lane & 7, g = lane >> 3;
                 float2 x[2] = {pv[i][g], pv[i][4 + g]};

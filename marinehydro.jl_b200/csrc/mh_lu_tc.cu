@@ -95,10 +95,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t phase)
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
             "selp.b32 %0, 1, 0, p;\n\t}\n"
             : "=r"(done)
-            : "r"(addr), "r"(phase)
+            : "r"(addr), "r"(phase), "r"(kWaitHintNs)
             : "memory");
         if (done) return true;
     }
