@@ -216,6 +216,9 @@ k_adj_wave(int kind, const double* __restrict__ geom, int64_t n, int direct, con
 // warp's VB/VD slot and retires the slot that the next copies overwrite;
 // there is no CTA barrier in the loop.  NQ = 0 takes any count up to
 // kMaxRhs and loads VA, VC directly.
+// FP64 operations a pair and frequency, three right-hand sides: about 70 (105 with
+// every complex derivative formed before its product); 2048 panels x 64
+// frequencies 3306 -> 3186 us, so the loads still bound it.
 // rowpart[colblock][kRowF][n], colpart[rowblock][kWaveF][n],
 // kpart[z][block]: deterministic partial sums.
 constexpr int kTJ = 2;
@@ -347,10 +350,10 @@ k_adj_delh_tape(const double* __restrict__ geom, int64_t n, int direct, const do
 #pragma unroll
                 for (int u = 0; u < kTJ; ++u) {
                     const double2 b = vcol[(q * kTJ + u) * 2], d = vcol[(q * kTJ + u) * 2 + 1];
-                    sr[u] += a.x * b.x + a.y * b.y;
-                    si[u] += a.y * b.x - a.x * b.y;
-                    dr[u] -= c.x * d.x + c.y * d.y;
-                    di[u] -= c.y * d.x - c.x * d.y;
+                    sr[u] = fma(a.x, b.x, fma(a.y, b.y, sr[u]));
+                    si[u] = fma(a.y, b.x, fma(-a.x, b.y, si[u]));
+                    dr[u] = fma(-c.x, d.x, fma(-c.y, d.y, dr[u]));
+                    di[u] = fma(-c.y, d.x, fma(c.x, d.y, di[u]));
                 }
             };
             if constexpr (NQ > 0) {
@@ -368,54 +371,45 @@ k_adj_delh_tape(const double* __restrict__ geom, int64_t n, int direct, const do
                 if (!live) continue;
                 const Panel& p = sp[jj];
                 const double* nD = direct ? p.n : ni;
-                // cs = conj(-S-bar / 4pi), cw = conj(-D-bar / 4pi)
-                const double csr = -kI4P * sr[u], csi = kI4P * si[u];
-                const double cwr = -kI4P * dr[u], cwi = kI4P * di[u];
-                // dimensionless G, G_r from the tape; G_z = G + 2/R, second
-                // derivatives from the identities (as gder_identities)
-                const double iR = ik * irho[u], iR3 = iR * iR * iR;  // 1 / R, R = k rho
+                // the coefficients conj(-S-bar / 4pi), conj(-D-bar / 4pi) enter
+                // linearly: here s = S-bar and d = D-bar, the factor -1/4pi
+                // follows with the sums.  Dimensionless G, G_r from the tape;
+                // G_z = G + 2/R, second derivatives from the identities (as
+                // gder_identities), of which only the real products are formed
+                const double iR = ik * irho[u], h1 = 2.0 * iR, h3 = h1 * iR * iR;  // 1 / R, R = k rho; 2 / R^3
                 const double r = k * wg[u].dis, zz = k * wg[u].zs;
                 const double2 g0 = mine[(2 * u) * kAR], g1 = mine[(2 * u + 1) * kAR];
-                const double G2r = g0.x + 2.0 * iR, G2i = g0.y;
-                const double Gzzr = G2r - 2.0 * zz * iR3, Gzzi = G2i;
-                const double Grzr = g1.x - 2.0 * r * iR3, Grzi = g1.y;
-                double Grrr, Grri;
-                if (r > 1e-3) {
-                    const double ir = ik * wg[u].invd;
-                    Grrr = -g1.x * ir - Gzzr;
-                    Grri = -g1.y * ir - Gzzi;
-                } else {
-                    Grrr = -0.5 * Gzzr;
-                    Grri = -0.5 * Gzzi;
-                }
-                const double va = csr * g1.x - csi * g1.y;  // re(cs G_r)
-                const double vb = cwr * Grrr - cwi * Grri;  // re(cw G_rr)
-                const double vc = cwr * Grzr - cwi * Grzi;  // re(cw G_rz)
-                const double vd = cwr * g1.x - cwi * g1.y;  // re(cw G_r)
-                const double ve = csr * G2r - csi * G2i;    // re(cs G_z)
-                const double vf = cwr * Gzzr - cwi * Gzzi;  // re(cw G_zz)
-                const double vg = csr * g0.x - csi * g0.y;  // re(cs G)
-                const double vh = cwr * G2r - cwi * G2i;    // re(cw G_z)
+                const double va = fma(sr[u], g1.x, si[u] * g1.y);        // re(conj(s) G_r)
+                const double vg = fma(sr[u], g0.x, si[u] * g0.y);        // re(conj(s) G)
+                const double ve = fma(sr[u], h1, vg);                    // re(conj(s) G_z)
+                const double vd = fma(dr[u], g1.x, di[u] * g1.y);        // re(conj(d) G_r)
+                const double vh = fma(dr[u], g0.x + h1, di[u] * g0.y);   // re(conj(d) G_z)
+                const double vf = fma(-dr[u], zz * h3, vh);              // re(conj(d) G_zz)
+                const double vc = fma(-dr[u], r * h3, vd);               // re(conj(d) G_rz)
+                const double vb = r > 1e-3 ? fma(-vd, ik * wg[u].invd, -vf) : -0.5 * vf;  // re(conj(d) G_rr)
                 const bool rad = fabs(r) > 1e-6;
-                Sa2[u] += k2 * va;
-                Sc3[u] += k3 * vc;
-                Se2[u] += k2 * ve;
-                Sf3[u] += k3 * vf;
-                Sg1[u] += k * vg;
-                Sh2[u] += k2 * vh;
+                Sa2[u] = fma(k2, va, Sa2[u]);
+                Sc3[u] = fma(k3, vc, Sc3[u]);
+                Se2[u] = fma(k2, ve, Se2[u]);
+                Sf3[u] = fma(k3, vf, Sf3[u]);
+                Sg1[u] = fma(k, vg, Sg1[u]);
+                Sh2[u] = fma(k2, vh, Sh2[u]);
                 if (rad) {
-                    Sb3r[u] += k3 * vb;
-                    Sc3r[u] += k3 * vc;
-                    Sd2r[u] += k2 * vd;
+                    Sb3r[u] = fma(k3, vb, Sb3r[u]);
+                    Sc3r[u] = fma(k3, vc, Sc3r[u]);
+                    Sd2r[u] = fma(k2, vd, Sd2r[u]);
                 }
-                // dL/dk of this pair and frequency (wave_chain's k term)
-                const double A = p.area, rs = rad ? s01[u] : 0.0;
-                const double Lr = A * (k * va + rs * k2 * vb + nD[2] * k2 * vc);
-                const double Lz = A * (k * ve + rs * k2 * vc + nD[2] * k2 * vf);
-                bk += Lr * wg[u].dis + Lz * wg[u].zs + A * vg + 2.0 * k * A * (rs * vd + nD[2] * vh);
+                // dL/dk of this pair and frequency (wave_chain's k term):
+                // L_r dis + L_z zs + A s G + 2 k A (rs d G_r + n_z d G_z) with
+                // L_r = A (k s G_r + k^2 (rs d G_rr + n_z d G_rz)), L_z alike
+                const double rs = rad ? s01[u] : 0.0, dis = wg[u].dis, zs = wg[u].zs;
+                const double q1 = fma(va, dis, ve * zs);
+                const double q2 = fma(rs, fma(vb, dis, vc * zs), nD[2] * fma(vc, dis, vf * zs));
+                const double q3 = fma(rs, vd, nD[2] * vh);
+                bk = fma(p.area, fma(k, fma(k, q2, fma(2.0, q3, q1)), vg), bk);
             }
             bk = warp_sum(bk);
-            if (lane == 0) ksm[warp * nb + z] += bk;
+            if (lane == 0) ksm[warp * nb + z] -= kI4P * bk;
         }
         // the chain of wave_chain summed over the frequencies: per pair
         // dx, dy, z, area and the normal, from the moments
@@ -426,12 +420,12 @@ k_adj_delh_tape(const double* __restrict__ geom, int64_t n, int direct, const do
             if (live) {
                 const Panel& p = sp[jb + u];
                 const double* nD = direct ? p.n : ni;
-                const double A = p.area, u0 = wg[u].u0, u1 = wg[u].u1, invd = wg[u].invd;
+                const double A = -kI4P * p.area, u0 = wg[u].u0, u1 = wg[u].u1, invd = wg[u].invd;
                 const double lin = Sa2[u] + s01[u] * Sb3r[u] + nD[2] * Sc3[u];
                 const double dx = A * u0 * lin + sg * A * invd * (nD[0] * (1.0 - u0 * u0) - nD[1] * u0 * u1) * Sd2r[u];
                 const double dy = A * u1 * lin + sg * A * invd * (nD[1] * (1.0 - u1 * u1) - nD[0] * u0 * u1) * Sd2r[u];
                 const double zs = A * (Se2[u] + s01[u] * Sc3r[u] + nD[2] * Sf3[u]);
-                const double area = Sg1[u] + s01[u] * Sd2r[u] + nD[2] * Sh2[u];
+                const double area = -kI4P * (Sg1[u] + s01[u] * Sd2r[u] + nD[2] * Sh2[u]);
                 const double nb0 = sg * A * u0 * Sd2r[u], nb1 = sg * A * u1 * Sd2r[u], nb2 = A * Sh2[u];
                 xb[0] += dx;
                 xb[1] += dy;
