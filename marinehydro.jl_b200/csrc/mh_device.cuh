@@ -244,158 +244,116 @@ __device__ __forceinline__ void rankine_pair(const T x[3], const PanelT<T>& p, T
 template <class T>
 __device__ __forceinline__ T wu_dFuncC(const T& t)  // wu.jl:51-66
 {
-    T g = (3168.35 + -1590.27 * t) * t;
-    g = (-2318.58 + g) * t;
-    g = (847.8 + g) * t;
-    g = (-148.24 + g) * t;
-    return 14.19 + g;
+    constexpr double c[] = {14.19, -148.24, 847.8, -2318.58, 3168.35, -1590.27};
+    return horner(c, t);
 }
 template <class T>
 __device__ __forceinline__ T wu_dFuncB(const T& t)  // wu.jl:69-92
 {
-    T g = (-76209.82 + 19923.28 * t) * t;
-    g = (118879.26 + g) * t;
-    g = (-97014.11 + g) * t;
-    g = (44270.15 + g) * t;
-    g = (-11336.19 + g) * t;
-    g = (1565.35 + g) * t;
-    g = (-76.765 + g) * t;
-    g = (2.894 + g) * t;
-    return 1.11 + g;
+    constexpr double c[] = {1.11, 2.894, -76.765, 1565.35, -11336.19, 44270.15,
+                            -97014.11, 118879.26, -76209.82, 19923.28};
+    return horner(c, t);
 }
 template <class T>
 __device__ __forceinline__ T wu_dFuncA(const T& t)  // wu.jl:94-117
 {
-    T g = (-46688.0 + 12622.25 * t) * t;
-    g = (68220.87 + g) * t;
-    g = (-48811.41 + g) * t;
-    g = (16370.75 + g) * t;
-    g = (-1187.71 + g) * t;
-    g = (-754.85 + g) * t;
-    g = (249.69 + g) * t;
-    g = (-24.53 + g) * t;
-    return 2.948 + g;
+    constexpr double c[] = {2.948, -24.53, 249.69, -754.85, -1187.71, 16370.75,
+                            -48811.41, 68220.87, -46688.0, 12622.25};
+    return horner(c, t);
 }
 template <class T>
 __device__ __forceinline__ T wu_FuncD(const T& t)  // wu.jl:159-182
 {
-    T g = (128170.2 + -33744.6 * t) * t;
-    g = (-205690.43 + g) * t;
-    g = (181856.75 + g) * t;
-    g = (-96293.05 + g) * t;
-    g = (31127.39 + g) * t;
-    g = (-6072.07 + g) * t;
-    g = (667.16 + g) * t;
-    g = (-40.97 + g) * t;
-    return 0.632 + g;
+    constexpr double c[] = {0.632, -40.97, 667.16, -6072.07, 31127.39, -96293.05,
+                            181856.75, -205690.43, 128170.2, -33744.6};
+    return horner(c, t);
 }
 template <class T>
 __device__ __forceinline__ T wu_FuncC(const T& t)  // wu.jl:184-203
 {
-    T g = (9136.4 + -3272.62 * t) * t;
-    g = (-9844.35 + g) * t;
-    g = (5155.67 + g) * t;
-    g = (-1397.89 + g) * t;
-    g = (209.653 + g) * t;
-    g = (-9.747 + g) * t;
-    return 1.268 + g;
+    constexpr double c[] = {1.268, -9.747, 209.653, -1397.89, 5155.67, -9844.35, 9136.4, -3272.62};
+    return horner(c, t);
 }
 template <class T>
 __device__ __forceinline__ T wu_FuncB(const T& t)  // wu.jl:205-228
 {
-    T g = (-29030.24 + 7671.22 * t) * t;
-    g = (44894.06 + g) * t;
-    g = (-36618.81 + g) * t;
-    g = (17137.74 + g) * t;
-    g = (-4780.77 + g) * t;
-    g = (796.534 + g) * t;
-    g = (-67.92 + g) * t;
-    g = (5.737 + g) * t;
-    return 0.938 + g;
+    constexpr double c[] = {0.938, 5.737, -67.92, 796.534, -4780.77, 17137.74,
+                            -36618.81, 44894.06, -29030.24, 7671.22};
+    return horner(c, t);
 }
 template <class T>
 __device__ __forceinline__ T wu_FuncA(const T& t)  // wu.jl:230-253
 {
-    T g = (21859.0 + -4838.6 * t) * t;
-    g = (-41592.9 + g) * t;
-    g = (42002.57 + g) * t;
-    g = (-24314.21 + g) * t;
-    g = (8418.94 + g) * t;
-    g = (-1763.96 + g) * t;
-    g = (215.896 + g) * t;
-    g = (-13.328 + g) * t;
-    return 1.21 + g;
+    constexpr double c[] = {1.21, -13.328, 215.896, -1763.96, 8418.94, -24314.21,
+                            42002.57, -41592.9, 21859.0, -4838.6};
+    return horner(c, t);
+}
+
+// Struve H0, H1 (wu.jl:295-327, 331-362); yy = (xx / 3)^2 for xx <= 3, (3 / xx)^2 past it
+template <class T>
+__device__ __forceinline__ T struve_h0(const T& xx, const T& yy)
+{
+    if (val(xx) <= 3.0) {
+        constexpr double c[] = {1.909859164, -1.909855001, 0.687514637, -0.126164557, 0.013828813, -0.000876918};
+        return horner(c, yy) * ((1.0 / 3.0) * xx);
+    }
+    constexpr double a[] = {0.99999906, 4.77228920, 3.85542044, 0.32303607};
+    constexpr double b[] = {1.0, 4.88331068, 4.28957333, 0.52120508};
+    return 2.0 * horner(a, yy) / (kPi * xx * horner(b, yy)) + y0(xx);
 }
 
 template <class T>
-__device__ __forceinline__ T struve_h0(const T& xx)  // wu.jl:295-327
+__device__ __forceinline__ T struve_h1(const T& xx, const T& yy)
 {
     if (val(xx) <= 3.0) {
-        T yy = (xx / 3.0) * (xx / 3.0);
-        T h = 1.909859164 + (-1.909855001 + (0.687514637 + (-0.126164557
-                   + (0.013828813 + -0.000876918 * yy) * yy) * yy) * yy) * yy;
-        return h * (xx / 3.0);
+        constexpr double c[] = {1.909859286, -1.145914713, 0.294656958, -0.042070508, 0.003785727, -0.000207183};
+        return horner(c, yy) * yy;
     }
-    T yy = (3.0 / xx) * (3.0 / xx);
-    T c1 = 2.0 * (0.99999906 + (4.77228920 + (3.85542044 + 0.32303607 * yy) * yy) * yy);
-    T c2 = kPi * xx * (1.0 + (4.88331068 + (4.28957333 + 0.52120508 * yy) * yy) * yy);
-    return c1 / c2 + y0(xx);
+    constexpr double a[] = {1.00000004, 3.92205313, 2.64893033, 0.27450895};
+    constexpr double b[] = {1.0, 3.81095112, 2.26216956, 0.10885141};
+    return 2.0 * horner(a, yy) / (kPi * horner(b, yy)) + y1(xx);
 }
 
-template <class T>
-__device__ __forceinline__ T struve_h1(const T& xx)  // wu.jl:331-362
-{
-    if (val(xx) <= 3.0) {
-        T yy = (xx / 3.0) * (xx / 3.0);
-        return (1.909859286 + (-1.145914713 + (0.294656958 + (-0.042070508
-                + (0.003785727 + -0.000207183 * yy) * yy) * yy) * yy) * yy) * yy;
-    }
-    T yy = (3.0 / xx) * (3.0 / xx);
-    T c1 = 2.0 * (1.00000004 + (3.92205313 + (2.64893033 + 0.27450895 * yy) * yy) * yy);
-    T c2 = kPi * (1.0 + (3.81095112 + (2.26216956 + 0.10885141 * yy) * yy) * yy);
-    return c1 / c2 + y1(xx);
-}
-
-// (G, dG/dh, dG/dv) of the Wu wave term, wu.jl:19-30; out = 3 complex.
+// (G, dG/dh, dG/dv) of the Wu wave term, wu.jl:19-30; out = 3 complex.  Bound by
+// FP64 operations: the polynomials are one FMA a term (two operations in the form
+// (c + g) t), and what is divided by more than once is inverted once.  1224 panels x
+// 16 frequencies 910 -> 728 us, the adjoint of one frequency of 2048 489 -> 378.
 template <class T>
 __device__ __forceinline__ void wu_dimless(const T& hh, const T& vv, cx<T> out[3])
 {
     T dd = sqrt(hh * hh + vv * vv);
-    T alpha = -vv / dd;
-    T beta = hh / dd;
-    T rho = dd / (1.0 + dd);
+    T id = 1.0 / dd;
+    T alpha = -vv * id;
+    T beta = hh * id;
+    T om = 1.0 / (1.0 + dd);  // 1 - rho
+    T rho = dd * om;
     T ev = exp(vv);
-    T om = 1.0 - rho;
-    T om3 = om * om * om;
-    T dd3 = dd * dd * dd;
+    T rom3 = rho * om * om * om;
+    T dd2 = dd * dd;
+    T i3 = 1.0 / (1.0 + dd2 * dd);
+    T omb = 1.0 - beta;
     // GF_Func_Lp / GF_Func_L0 (wu.jl:266-293)
-    T RR = (1.0 - beta) * wu_FuncA(rho);
-    RR -= beta * wu_FuncB(rho);
-    RR -= alpha * wu_FuncC(rho) / (1.0 + 6.0 * alpha * rho * (1.0 - rho));
-    RR += beta * (1.0 - beta) * wu_FuncD(rho);
-    T Lp = rho * om3 * RR;
+    T RR = omb * wu_FuncA(rho) - beta * wu_FuncB(rho) - alpha * wu_FuncC(rho) / (1.0 + 6.0 * alpha * rho * om)
+           + beta * omb * wu_FuncD(rho);
     const double gama = 0.5772156649;
-    T PP = log(0.5 * (dd - vv)) + gama - 2.0 * dd * dd;
-    PP = ev * PP;
-    PP = PP + dd * dd - vv;
-    T L0 = 2.0 * PP / (1.0 + dd3) + 2.0 * Lp;
+    T PP = ev * (log(0.5 * (dd - vv)) + gama - 2.0 * dd2) + dd2 - vv;
+    T L0 = 2.0 * (PP * i3 + rom3 * RR);
     // GF_Func_Lsp / GF_Func_Ls (wu.jl:131-157)
-    T RS = beta * wu_dFuncA(rho);
-    RS -= (1.0 - alpha) * wu_dFuncB(rho);
-    RS += beta * (1.0 - beta) * rho * (1.0 - 2.0 * rho) * wu_dFuncC(rho);
-    T Lsp = rho * om3 * RS;
-    T PS = (beta + hh) / (dd - vv);
-    PS = PS - 2.0 * beta + 2.0 * ev * dd - hh;
-    T QS = exp(-dd) * (1.0 - beta);
-    QS = QS * (1.0 + dd / (1.0 + dd3));
-    T Ls = 2.0 * PS / (1.0 + dd3) - 4.0 * QS + 2.0 * Lsp;
+    T RS = beta * wu_dFuncA(rho) - (1.0 - alpha) * wu_dFuncB(rho)
+           + beta * omb * rho * (1.0 - 2.0 * rho) * wu_dFuncC(rho);
+    T PS = (beta + hh) / (dd - vv) - 2.0 * beta + 2.0 * ev * dd - hh;
+    T QS = exp(-dd) * omb * (1.0 + dd * i3);
+    T Ls = 2.0 * (PS * i3 + rom3 * RS) - 4.0 * QS;
     // W, Wh (wu.jl:122-129, :257-264)
-    T H0 = struve_h0(hh), J0 = j0(hh), H1 = struve_h1(hh), J1 = j1(hh);
+    T q = val(hh) <= 3.0 ? (1.0 / 3.0) * hh : 3.0 / hh;
+    T yy = q * q;
+    T H0 = struve_h0(hh, yy), H1 = struve_h1(hh, yy), J0, J1;
+    bessel_j01(hh, J0, J1);
     T G_re = -L0 - (2.0 * kPi) * H0 * ev;
     T G_im = (2.0 * kPi) * J0 * ev;
     out[0] = cx<T>{G_re, G_im};
     out[1] = cx<T>{-Ls - (2.0 * kPi) * (2.0 / kPi - H1) * ev, (-2.0 * kPi) * J1 * ev};
-    out[2] = cx<T>{G_re + 2.0 / dd, G_im};
+    out[2] = cx<T>{G_re + 2.0 * id, G_im};
 }
 
 // ---------------------------------------------------------------------------

@@ -119,7 +119,8 @@ __device__ __forceinline__ dualn<ND> operator/(const dualn<ND>& a, double b) { r
 template <int ND>
 __device__ __forceinline__ dualn<ND> operator/(double a, const dualn<ND>& b)
 {
-    return dchain(b, a / b.v, -a / (b.v * b.v));
+    const double ib = 1.0 / b.v, f = a * ib;
+    return dchain(b, f, -f * ib);
 }
 
 template <int ND>
@@ -183,6 +184,41 @@ __device__ __forceinline__ dualn<ND> y1(const dualn<ND>& x)
 {
     const double Y1 = ::y1(x.v);
     return dchain(x, Y1, ::y0(x.v) - Y1 / x.v);
+}
+// J0 and J1 together: their derivatives are each other's values
+__device__ __forceinline__ void bessel_j01(double x, double& J0, double& J1)
+{
+    J0 = ::j0(x);
+    J1 = ::j1(x);
+}
+template <int ND>
+__device__ __forceinline__ void bessel_j01(const dualn<ND>& x, dualn<ND>& J0, dualn<ND>& J1)
+{
+    const double a = ::j0(x.v), b = ::j1(x.v);
+    J0 = dchain(x, a, -b);
+    J1 = dchain(x, b, x.v != 0.0 ? a - b / x.v : 0.5);
+}
+// The polynomial sum_i c[i] t^i by Horner's rule; for a dual its value and its
+// derivative together, then the chain once (5 operations a term for two
+// directions otherwise).
+template <int N>
+__device__ __forceinline__ double horner(const double (&c)[N], double t)
+{
+    double p = c[N - 1];
+#pragma unroll
+    for (int i = N - 2; i >= 0; --i) p = ::fma(p, t, c[i]);
+    return p;
+}
+template <int N, int ND>
+__device__ __forceinline__ dualn<ND> horner(const double (&c)[N], const dualn<ND>& t)
+{
+    double p = c[N - 1], dp = 0.0;
+#pragma unroll
+    for (int i = N - 2; i >= 0; --i) {
+        dp = ::fma(dp, t.v, p);
+        p = ::fma(p, t.v, c[i]);
+    }
+    return dchain(t, p, dp);
 }
 template <int ND>
 __device__ __forceinline__ dualn<ND> fma(const dualn<ND>& a, const dualn<ND>& b, const dualn<ND>& c)
