@@ -1,0 +1,321 @@
+// FP64 complex solve A X = B with partial pivoting for one matrix of moderate
+// order: the calls for one frequency (forces, solve).  The FP64 batches and their
+// adjoints keep cuSOLVER, whose factors the adjoint solves with again.  B rides along as further
+// columns: panels of kW columns, and per panel
+//   k_lu64_panel   one CTA factors the panel in shared memory and records the row
+//                  exchanges as a gather;
+//   k_lu64_update  a CTA takes kC columns to the right (of A, then of B): gathers
+//                  the exchanged rows, U12 = inv(L11) A12 by shuffles, A22 -= L21 U12;
+// then k_lu64_back, a CTA per column of B, substitutes back.  The pivot is the
+// entry of largest |re| + |im|, as in LAPACK's zgetrf; left of a panel nothing is
+// exchanged, since L is not used again.
+// What bounds it: n dependent pivot searches (about 1 us each with the update of
+// the panel's other columns in one CTA, 2 with 800 rows).  Measured, us, cuSOLVER's
+// zgetrf and zgetrs -> this, one right-hand side: n 50 174 -> 113, 100 272 -> 218, 200
+// 513 -> 442, 400 1104 -> 962, 800 2673 -> 2421; equal at 1000.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "mh_internal.h"
+
+namespace mh {
+namespace {
+
+constexpr int kW = 16;              // panel columns
+constexpr int kC = 8;               // columns per CTA of the update
+constexpr int kPanelThreads = 512;
+constexpr int kUpdThreads = 256;
+constexpr int kBackThreads = 512;
+constexpr int kBlk = 32;            // rows per step of the back substitution
+
+__device__ __forceinline__ double2 cmul(double2 a, double2 b)
+{
+    return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
+}
+// c - a b
+__device__ __forceinline__ double2 cfms(double2 c, double2 a, double2 b)
+{
+    return make_double2(fma(-a.x, b.x, fma(a.y, b.y, c.x)), fma(-a.x, b.y, fma(-a.y, b.x, c.y)));
+}
+// 1 / a, scaled by a power of two near 1 / |a|: no overflow or underflow of |a|^2
+__device__ __forceinline__ double2 cinv(double2 a)
+{
+    const int e = __double2hiint(fmax(fabs(a.x), fabs(a.y))) >> 20;  // biased exponent
+    const double s = __hiloint2double((2046 - max(1, min(2045, e))) << 20, 0);
+    const double x = a.x * s, y = a.y * s, d = s / fma(x, x, y * y);
+    return make_double2(x * d, -y * d);
+}
+
+// Shared memory: the panel by columns, rows k0 .. n - 1, then which row of it
+// stands in each; and the panel's width, fewer columns where the rows are many.
+size_t panel_smem(int64_t rows, int w) { return (size_t)rows * (w * sizeof(double2) + sizeof(int)); }
+constexpr size_t kPanelSmemMax = 226 * 1024;
+int panel_width(int64_t rows)
+{
+    int w = (int)std::min<int64_t>(kW, rows);
+    while (w > 4 && panel_smem(rows, w) > kPanelSmemMax) --w;
+    return w;
+}
+
+// The largest of the warp's big >= 0 (its bits as an integer's, in two halves; -1
+// where a lane has none) and a lane that has it.
+__device__ __forceinline__ int warp_best(double& big)
+{
+    const unsigned hi = big < 0.0 ? 0u : (unsigned)__double2hiint(big) + 1u;
+    const unsigned top = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned lo = hi == top ? (unsigned)__double2loint(big) : 0u;
+    const unsigned low = __reduce_max_sync(0xffffffffu, lo);
+    big = top ? __hiloint2double((int)(top - 1u), (int)low) : -1.0;
+    return __ffs(__ballot_sync(0xffffffffu, hi == top && lo == low)) - 1;
+}
+
+// gather: 2 kW pairs (to, from), rows of the matrix: where every row that moved,
+// or is at the panel's top, comes from.  Two barriers per column: the pivot row is
+// set aside, then every row is updated (old row j into the pivot's place) and
+// looks for the next column's pivot on the way.
+__global__ void __launch_bounds__(kPanelThreads)
+k_lu64_panel(double2* __restrict__ A, int n, int k0, int w, int2* __restrict__ gather, int* __restrict__ info)
+{
+    extern __shared__ double2 p[];
+    const int rows = n - k0, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+    int* perm = reinterpret_cast<int*>(p + (size_t)rows * w);
+    __shared__ double best[kPanelThreads / 32];
+    __shared__ int where[kPanelThreads / 32];
+    __shared__ int moved[kW];
+    __shared__ double2 u[kW + 3];  // the pivot row (read past its end in fours, not used)
+    double2* M = A + (int64_t)k0 * n + k0;
+    double big = -1.0;
+    int at = 0;
+    for (int r = tid; r < rows; r += blockDim.x) {
+        perm[r] = r;
+#pragma unroll 4
+        for (int c = 0; c < w; ++c) p[c * rows + r] = M[(int64_t)c * n + r];
+        const double m = fabs(p[r].x) + fabs(p[r].y);
+        if (m > big) {
+            big = m;
+            at = r;
+        }
+    }
+    for (int j = 0; j < w; ++j) {
+        {
+            const int from = warp_best(big);
+            if (lane == from) {
+                best[warp] = big;
+                where[warp] = at;
+            }
+        }
+        __syncthreads();  // also: the rows are updated
+        big = lane < warps ? best[lane] : -1.0;
+        at = lane < warps ? where[lane] : j;
+        at = __shfl_sync(0xffffffffu, at, warp_best(big));
+        if (!(big >= 0.0)) at = j;  // no number in the column
+        const double2 piv = p[j * rows + at], ip = cinv(piv);
+        if (tid < w) {
+            u[tid] = p[tid * rows + at];
+            if (tid < j) {  // L is exchanged whole
+                p[tid * rows + at] = p[tid * rows + j];
+                p[tid * rows + j] = u[tid];
+            }
+        }
+        if (tid == 0) {
+            const int t = perm[j];
+            perm[j] = perm[at];
+            perm[at] = t;
+            moved[j] = at;
+            if (piv.x == 0.0 && piv.y == 0.0) atomicCAS(info, 0, k0 + j + 1);
+        }
+        __syncthreads();
+        const int pr = at;
+        big = -1.0;
+        at = rows;
+        for (int r = tid; r < rows; r += blockDim.x) {
+            if (r < j || r == pr) continue;
+            const int to = r == j ? pr : r;
+            const double2 l = cmul(p[j * rows + r], ip);
+            p[j * rows + to] = l;
+            for (int c = j + 1; c < w; c += 4) {
+                double2 a[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (c + i < w) a[i] = p[(c + i) * rows + r];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a[i] = cfms(a[i], l, u[c + i]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (c + i < w) p[(c + i) * rows + to] = a[i];
+                if (c == j + 1) {
+                    const double m = fabs(a[0].x) + fabs(a[0].y);
+                    if (m > big) {
+                        big = m;
+                        at = to;
+                    }
+                }
+            }
+            if (r == j)
+                for (int c = j; c < w; ++c) p[c * rows + j] = u[c];
+        }
+        if (big < 0.0) at = j + 1;
+    }
+    __syncthreads();
+    for (int r = tid; r < rows; r += blockDim.x)
+#pragma unroll 4
+        for (int c = 0; c < w; ++c) M[(int64_t)c * n + r] = p[c * rows + r];
+    if (tid < w) {
+        gather[tid] = make_int2(k0 + tid, k0 + perm[tid]);
+        gather[kW + tid] = make_int2(k0 + moved[tid], k0 + perm[moved[tid]]);
+    }
+}
+
+__global__ void __launch_bounds__(kUpdThreads)
+k_lu64_update(double2* __restrict__ A, double2* __restrict__ B, int n, int nrhs, int k0, int w,
+              const int2* __restrict__ gather)
+{
+    __shared__ double2 top[kW][kC], l11[kW][kW + 1];
+    const int right = n - k0 - w, tid = threadIdx.x;
+    const auto column = [&](int c) {  // column c right of the panel, null past the last
+        const int q = (int)blockIdx.x * kC + c;
+        return q < right ? A + (int64_t)(k0 + w + q) * n : q < right + nrhs ? B + (int64_t)(q - right) * n : nullptr;
+    };
+    static_assert(kUpdThreads == 2 * kW * kC && kW * kW == kUpdThreads, "one gathered entry and one of L11 per thread");
+    {
+        const int e = tid % (2 * kW), c = tid / (2 * kW);
+        double2* col = column(c);
+        const bool live = col && e % kW < w;
+        const int2 g = live ? gather[e] : make_int2(0, 0);
+        const double2 v = live ? col[g.y] : make_double2(0.0, 0.0);
+        const int i = tid % kW, m = tid / kW;
+        l11[i][m] = m < i && i < w ? A[(int64_t)(k0 + m) * n + k0 + i] : make_double2(0.0, 0.0);
+        __syncthreads();  // every gathered row is read
+        if (e < kW) top[e][c] = v;
+        else if (live && g.x >= k0 + w) col[g.x] = v;
+    }
+    __syncthreads();
+    if (tid < kW * kC) {  // U12: a column per half warp, a row per lane
+        const int i = tid % kW, c = tid / kW, base = tid & 16;
+        double2 t = top[i][c];
+#pragma unroll
+        for (int m = 0; m < kW - 1; ++m) {
+            const double2 u = make_double2(__shfl_sync(0xffffffffu, t.x, base + m), __shfl_sync(0xffffffffu, t.y, base + m));
+            t = cfms(t, l11[i][m], u);  // zero for i <= m
+        }
+        top[i][c] = t;
+        double2* col = column(c);
+        if (col && i < w) col[k0 + i] = t;
+    }
+    __syncthreads();
+    for (int r = k0 + w + tid; r < n; r += kUpdThreads) {
+        double2 l[kW];
+#pragma unroll
+        for (int m = 0; m < kW; ++m) l[m] = m < w ? A[(int64_t)(k0 + m) * n + r] : make_double2(0.0, 0.0);
+        double2 a[kC];
+#pragma unroll
+        for (int c = 0; c < kC; ++c) {
+            const double2* col = column(c);
+            a[c] = col ? col[r] : make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int m = 0; m < kW; ++m)
+#pragma unroll
+            for (int c = 0; c < kC; ++c) a[c] = cfms(a[c], l[m], top[m][c]);
+#pragma unroll
+        for (int c = 0; c < kC; ++c) {
+            double2* col = column(c);
+            if (col) col[r] = a[c];
+        }
+    }
+}
+
+// U x = y in place, a CTA per column of B.  The next diagonal block is fetched
+// while this one is solved.
+__global__ void __launch_bounds__(kBackThreads)
+k_lu64_back(const double2* __restrict__ A, double2* __restrict__ B, int n)
+{
+    extern __shared__ double2 x[];  // [n]
+    __shared__ double2 u[kBlk][kBlk + 1];
+    double2* col = B + (int64_t)blockIdx.x * n;
+    const int tid = threadIdx.x;
+    constexpr int kE = kBlk * kBlk / kBackThreads;
+    double2 f[kE];
+    const auto fetch = [&](int k) {
+#pragma unroll
+        for (int e = 0; e < kE; ++e) {
+            const int i = (e * kBackThreads + tid) % kBlk, j = (e * kBackThreads + tid) / kBlk;
+            f[e] = k >= 0 && k + j < n && i <= j ? A[(int64_t)(k + j) * n + k + i]
+                                                 : make_double2(i == j ? 1.0 : 0.0, 0.0);
+        }
+    };
+    int k = (n - 1) / kBlk * kBlk;
+    fetch(k);
+    for (int r = tid; r < n; r += kBackThreads) x[r] = col[r];
+    for (; k >= 0; k -= kBlk) {
+        const int w = min(kBlk, n - k);
+#pragma unroll
+        for (int e = 0; e < kE; ++e) u[(e * kBackThreads + tid) % kBlk][(e * kBackThreads + tid) / kBlk] = f[e];
+        __syncthreads();  // also x
+        fetch(k - kBlk);
+        if (tid < kBlk) {
+            double2 t = tid < w ? x[k + tid] : make_double2(0.0, 0.0);
+            const double2 inv = cinv(u[tid][tid]);
+#pragma unroll 4
+            for (int j = kBlk - 1; j >= 0; --j) {
+                double2 v = cmul(t, inv);
+                v = make_double2(__shfl_sync(0xffffffffu, v.x, j), __shfl_sync(0xffffffffu, v.y, j));
+                t = tid == j ? v : tid < j ? cfms(t, u[tid][j], v) : t;
+            }
+            if (tid < w) x[k + tid] = t;
+        }
+        __syncthreads();
+        for (int r = tid; r < k; r += kBackThreads) {
+            double2 t = x[r];
+            for (int j0 = 0; j0 < w; j0 += 16) {
+                double2 a[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    a[j] = j0 + j < w ? A[(int64_t)(k + j0 + j) * n + r] : make_double2(0.0, 0.0);
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    if (j0 + j < w) t = cfms(t, a[j], x[k + j0 + j]);
+            }
+            x[r] = t;
+        }
+        __syncthreads();
+    }
+    for (int r = tid; r < n; r += kBackThreads) col[r] = x[r];
+}
+
+}  // namespace
+
+// The orders it takes: where it beats cuSOLVER (figures above).
+bool lu64_takes(int64_t n) { return n <= 896; }
+
+// A X = B, A overwritten, X in place of B; MH_ERR_SINGULAR at a zero pivot.
+int lu64_solve(mh_ctx* ctx, int64_t n, double2* A, double2* B, int nrhs)
+{
+    auto* gather = (int2*)ws_get(ctx, WS_PIV, sizeof(int2) * 2 * kW);
+    auto* info = (int*)ws_get(ctx, WS_INFO, sizeof(int) * 2);
+    if (!gather || !info) return MH_ERR_OOM;
+    MH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_lu64_panel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)kPanelSmemMax));
+    MH_CUDA_TRY(ctx, cudaMemsetAsync(info, 0, sizeof(int), ctx->stream));
+    for (int64_t k0 = 0; k0 < n;) {
+        const int w = panel_width(n - k0);
+        const int threads = (int)std::min<int64_t>(kPanelThreads, (n - k0 + 31) / 32 * 32);
+        k_lu64_panel<<<1, threads, panel_smem(n - k0, w), ctx->stream>>>(A, (int)n, (int)k0, w, gather, info);
+        const int64_t cols = n - k0 - w + nrhs;
+        k_lu64_update<<<(unsigned)((cols + kC - 1) / kC), kUpdThreads, 0, ctx->stream>>>(A, B, (int)n, nrhs, (int)k0, w,
+                                                                                       gather);
+        ctx->launches += 2;
+        k0 += w;
+    }
+    k_lu64_back<<<nrhs, kBackThreads, sizeof(double2) * (size_t)n, ctx->stream>>>(A, B, (int)n);
+    ctx->launches += 1;
+    MH_CUDA_TRY(ctx, cudaGetLastError());
+    int h = 0;
+    MH_CUDA_TRY(ctx, cudaMemcpyAsync(&h, info, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    MH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    if (h > 0) return set_err(ctx, MH_ERR_SINGULAR, "zero pivot at column %d", h);
+    return MH_OK;
+}
+
+}  // namespace mh
