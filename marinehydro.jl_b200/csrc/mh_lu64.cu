@@ -1,7 +1,8 @@
 // FP64 complex solve A X = B with partial pivoting for one matrix of moderate
 // order: the calls for one frequency (forces, solve).  The FP64 batches and their
-// adjoints keep cuSOLVER, whose factors the adjoint solves with again.  B rides along as further
-// columns: panels of kW columns, and per panel
+// adjoints keep cuSOLVER, whose factors the adjoint solves with again.  B rides
+// along as further columns.  Up to kWholeMax panels k_lu64_whole does all of it in
+// one CTA; else panels of kW columns, and per panel
 //   k_lu64_panel   one CTA factors the panel in shared memory and records the row
 //                  exchanges as a gather;
 //   k_lu64_update  a CTA takes kC columns to the right (of A, then of B): gathers
@@ -11,8 +12,8 @@
 // exchanged, since L is not used again.
 // What bounds it: n dependent pivot searches (about 1 us each with the update of
 // the panel's other columns in one CTA, 2 with 800 rows).  Measured, us, cuSOLVER's
-// zgetrf and zgetrs -> this, one right-hand side: n 50 174 -> 113, 100 272 -> 218, 200
-// 513 -> 442, 400 1104 -> 962, 800 2673 -> 2421; equal at 1000.
+// zgetrf and zgetrs -> this, one right-hand side: n 24 118 -> 29, 50 157 -> 69, 100 263
+// -> 218, 200 505 -> 442, 400 1104 -> 962, 800 2673 -> 2421; equal at 1000.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,6 +29,9 @@ constexpr int kPanelThreads = 512;
 constexpr int kUpdThreads = 256;
 constexpr int kBackThreads = 512;
 constexpr int kBlk = 32;            // rows per step of the back substitution
+// One CTA for everything up to here: us, it and the panels, n 50 69 and 113, 80 139
+// and about 170, 100 227 and 218, 112 273 and about 245.
+constexpr int kWholeMax = 96;
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b)
 {
@@ -167,6 +171,89 @@ k_lu64_panel(double2* __restrict__ A, int n, int k0, int w, int2* __restrict__ g
     }
 }
 
+// The whole solve in one CTA: the columns of A and B as one panel (ld n), the rows
+// on `rows` threads (a multiple of 32, at least n) times blockDim / rows groups,
+// each with every such group's fours of columns.  As k_lu64_panel otherwise, but
+// neither L nor the exchanges are kept; then U x = y, a barrier a column.
+__global__ void __launch_bounds__(kPanelThreads)
+k_lu64_whole(const double2* __restrict__ A, double2* __restrict__ B, int n, int nrhs, int rows, int* __restrict__ info)
+{
+    extern __shared__ double2 p[];  // [n + nrhs][n]
+    const int W = n + nrhs, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+    const int r = tid % rows, group = tid / rows, groups = blockDim.x / rows;
+    double2* u = p + (size_t)W * n;  // the pivot row, [W + 3]
+    double2* dinv = u + W + 3;       // 1 / u_jj, [n]
+    __shared__ double best[kPanelThreads / 32];
+    __shared__ int where[kPanelThreads / 32];
+    if (r < n)
+        for (int c = group; c < W; c += groups)
+            p[c * n + r] = c < n ? A[(int64_t)c * n + r] : B[(int64_t)(c - n) * n + r];
+    __syncthreads();
+    double big = r < n && group == 0 ? fabs(p[r].x) + fabs(p[r].y) : -1.0;
+    if (!(big >= 0.0)) big = -1.0;
+    int at = r;
+    for (int j = 0; j < n; ++j) {
+        {
+            const int from = warp_best(big);
+            if (lane == from) {
+                best[warp] = big;
+                where[warp] = at;
+            }
+        }
+        __syncthreads();  // also: the rows are updated
+        big = lane < warps ? best[lane] : -1.0;
+        at = lane < warps ? where[lane] : j;
+        at = __shfl_sync(0xffffffffu, at, warp_best(big));
+        if (!(big >= 0.0)) at = j;  // no number in the column
+        const double2 piv = p[j * n + at], ip = cinv(piv);
+        for (int c = j + tid; c < W; c += blockDim.x) u[c] = p[c * n + at];
+        if (tid == 0 && piv.x == 0.0 && piv.y == 0.0) atomicCAS(info, 0, j + 1);
+        __syncthreads();
+        const int pr = at;
+        big = -1.0;
+        at = j + 1;
+        if (r >= j && r < n) {
+            const int to = r == j ? pr : r;
+            const double2 l = cmul(p[j * n + r], ip);
+            for (int c = j + 1 + 4 * group; c < W; c += 4 * groups) {
+                if (r != pr) {
+                    double2 a[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (c + i < W) a[i] = p[(c + i) * n + r];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) a[i] = cfms(a[i], l, u[c + i]);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (c + i < W) p[(c + i) * n + to] = a[i];
+                    if (c == j + 1) {
+                        const double m = fabs(a[0].x) + fabs(a[0].y);
+                        if (m >= 0.0) {
+                            big = m;
+                            at = to;
+                        }
+                    }
+                }
+                if (r == j)
+                    for (int i = 0; i < 4; ++i)
+                        if (c + i < W) p[(c + i) * n + j] = u[c + i];
+            }
+        }
+        if (tid == 0) dinv[j] = ip;
+    }
+    __syncthreads();
+    for (int j = n - 1; j >= 0; --j) {
+        const double2 inv = dinv[j];
+        for (int q = group; q < nrhs; q += groups) {
+            double2* y = p + (n + q) * n;
+            const double2 x = cmul(y[j], inv);
+            if (r < j) y[r] = cfms(y[r], p[j * n + r], x);
+            if (r == j) B[(int64_t)q * n + j] = x;
+        }
+        __syncthreads();
+    }
+}
+
 __global__ void __launch_bounds__(kUpdThreads)
 k_lu64_update(double2* __restrict__ A, double2* __restrict__ B, int n, int nrhs, int k0, int w,
               const int2* __restrict__ gather)
@@ -289,15 +376,34 @@ k_lu64_back(const double2* __restrict__ A, double2* __restrict__ B, int n)
 // The orders it takes: where it beats cuSOLVER (figures above).
 bool lu64_takes(int64_t n) { return n <= 896; }
 
+static int lu64_status(mh_ctx* ctx, const int* info)
+{
+    MH_CUDA_TRY(ctx, cudaGetLastError());
+    int h = 0;
+    MH_CUDA_TRY(ctx, cudaMemcpyAsync(&h, info, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    MH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    if (h > 0) return set_err(ctx, MH_ERR_SINGULAR, "zero pivot at column %d", h);
+    return MH_OK;
+}
+
 // A X = B, A overwritten, X in place of B; MH_ERR_SINGULAR at a zero pivot.
 int lu64_solve(mh_ctx* ctx, int64_t n, double2* A, double2* B, int nrhs)
 {
+    const size_t whole = sizeof(double2) * ((size_t)(n + nrhs) * (size_t)n + (size_t)(2 * n + nrhs + 3));
     auto* gather = (int2*)ws_get(ctx, WS_PIV, sizeof(int2) * 2 * kW);
     auto* info = (int*)ws_get(ctx, WS_INFO, sizeof(int) * 2);
     if (!gather || !info) return MH_ERR_OOM;
     MH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_lu64_panel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)kPanelSmemMax));
     MH_CUDA_TRY(ctx, cudaMemsetAsync(info, 0, sizeof(int), ctx->stream));
+    if (n <= kWholeMax && whole <= kPanelSmemMax) {
+        MH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_lu64_whole, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)kPanelSmemMax));
+        const int rows = (int)(n + 31) / 32 * 32, groups = kPanelThreads / rows;
+        k_lu64_whole<<<1, rows * groups, whole, ctx->stream>>>(A, B, (int)n, nrhs, rows, info);
+        ctx->launches += 1;
+        return lu64_status(ctx, info);
+    }
     for (int64_t k0 = 0; k0 < n;) {
         const int w = panel_width(n - k0);
         const int threads = (int)std::min<int64_t>(kPanelThreads, (n - k0 + 31) / 32 * 32);
@@ -310,12 +416,7 @@ int lu64_solve(mh_ctx* ctx, int64_t n, double2* A, double2* B, int nrhs)
     }
     k_lu64_back<<<nrhs, kBackThreads, sizeof(double2) * (size_t)n, ctx->stream>>>(A, B, (int)n);
     ctx->launches += 1;
-    MH_CUDA_TRY(ctx, cudaGetLastError());
-    int h = 0;
-    MH_CUDA_TRY(ctx, cudaMemcpyAsync(&h, info, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    MH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-    if (h > 0) return set_err(ctx, MH_ERR_SINGULAR, "zero pivot at column %d", h);
-    return MH_OK;
+    return lu64_status(ctx, info);
 }
 
 }  // namespace mh

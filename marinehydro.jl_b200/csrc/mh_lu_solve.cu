@@ -8,17 +8,22 @@
 // The owner's threads store y_i straight into the y table of every CTA of the
 // cluster (st.async), and each store counts on that CTA's mbarrier of block i, so
 // a CTA waits for a block on its own shared memory and reads it there: a step of
-// the chain is one tile product, one inverse product and one hand-off of about
-// half a microsecond.  (Published through global memory, with a flag per block
-// and a copy of y_j back into shared memory, a step took 5.3 us, and 8 to 13 us
-// for odd n or more than four right-hand sides.)
+// the chain is one tile product, one inverse product and one hand-off, 2 us in
+// all.  (Published through global memory, with a flag per block and a copy of y_j
+// back into shared memory, a step took 5.3 us, and 8 to 13 us for odd n or more
+// than four right-hand sides.)  With many matrices the shared-memory bandwidth of
+// a tile bounds it (written, read and multiplied from there, 512 of some 700
+// cycles).  us a solve, through global memory -> this: 2048 x 64 matrices with 3
+// right-hand sides 498 -> 419, 2997 x 24 with 2 778 -> 615, 1456 x 32 with 3 214 -> 141,
+// 2048 x 1 with 3 342 -> 138, 1224 x 16 with 8 513 -> 314.
 // Every operand a CTA reads is known in advance (its blocks' tiles in order, each
 // block followed by its inverse diagonal block), so four producer warps stream them
 // through a ring of shared-memory stages with cp.async (16 bytes a copy where n is
 // even, 8 otherwise; entries past the matrix are zero-filled) while eight consumer
 // warps multiply, and the tile stream runs ahead of the chain.
 // Cluster size: the CTAs that fill the chip with one per SM (8, 6, 4, 2 or 1 per
-// matrix), at most one per row block.
+// matrix), at most one per row block: a CTA's ring takes an SM's shared memory, so
+// a second wave of clusters would double the chain.
 //
 // Every wait is bounded: a stage wait that runs out marks the matrix in `bad` (2),
 // a wait for a block marks it (3) and later blocks are not waited for; every block

@@ -1,5 +1,6 @@
-"""FP64 solve with partial pivoting (panels in one CTA's shared memory): orders at
-the edges of a panel (16 columns, fewer where the rows are many), of the update's
+"""FP64 solve with partial pivoting (one CTA up to 96 while the right-hand sides fit
+its shared memory, else panels): orders on both sides of that line, at the edges of
+a panel (16 columns, fewer where the rows are many), of the update's
 column blocks (8) and of the back substitution's blocks (32), several right-hand
 sides, matrices that need row exchanges at every column.
 
@@ -21,7 +22,8 @@ def _check(A, X, B):
 
 
 @pytest.mark.parametrize("n,nrhs", [(1, 1), (2, 3), (7, 1), (8, 2), (15, 1), (16, 1), (17, 2), (31, 1), (32, 9), (33, 1),
-                                    (48, 1), (50, 1), (64, 8), (65, 1), (100, 6), (257, 2), (700, 1), (870, 1),
+                                    (48, 1), (50, 1), (64, 8), (65, 1), (96, 1), (96, 60), (97, 1),
+                                    (100, 6), (257, 2), (700, 1), (870, 1),
                                     (896, 3), (897, 1)])
 def test_solve(mh, gpu, n, nrhs):
     rng = np.random.default_rng(n + nrhs)
