@@ -653,20 +653,20 @@ def _peaks():
 # processes, so it is scaled by them.
 WAVE_DRAM_BYTES_PER_PAIR_FREQ = 39.4
 # FP64 operations of k_wave_delh_allw counted from its source (an FMA is 2,
-# any other arithmetic operation or library call 1): per pair, the geometry
-# (20) and the alpha contraction of the four polar functions (15 rows x 21
-# Clenshaw steps x 4 functions x (FMA + subtraction) = 3780, plus the 15 x 4
-# closing steps, 180); per pair and frequency, R and u (3), the four degree-14
-# Horner series (14 x 4 FMAs = 112), G, G_r, G_z from them (16) and the
-# scaling into S and D (32).
-WAVE_FLOPS_PER_PAIR = 3980.0
-WAVE_FLOPS_PER_PAIR_FREQ = 163.0
+# any other arithmetic operation or library call 1): per pair, the geometry and
+# the factors of S and D (36), the Chebyshev values (24) and the alpha contraction
+# of the four polar functions (15 rows x 22 terms x 4 functions FMAs = 2640; the
+# matrix instruction's padding is not counted); per pair and frequency, R and u
+# (3), the four degree-14 Horner series (14 x 4 FMAs = 112), G, G_r, G_z from
+# them (14) and the scaling into S and D (15).
+WAVE_FLOPS_PER_PAIR = 2700.0
+WAVE_FLOPS_PER_PAIR_FREQ = 144.0
 # Nominal FP64 and FP32 (CUDA-core) peaks of a B200: 148 SMs x 64 FP64 or
 # 128 FP32 FMA per clock x 2 x 1.965 GHz; neither is measured on this pool.
 FP64_PEAK_TFLOPS = 37.2
 FP32_PEAK_TFLOPS = 74.5
 # Of the per pair-frequency operations, the Horner series (112) runs in FP32
-# at the mixed path's default series level (1), the rest (51) in FP64.
+# at the mixed path's default series level (1), the rest (32) in FP64.
 WAVE_FP32_FLOPS_PER_PAIR_FREQ = 112.0
 # DRAM bytes of the LU phase per matrix of 2048, from an ncu capture of the
 # three LU kernels over one factorisation of 16 matrices of 2048 with the
