@@ -11,9 +11,10 @@
 // entry of largest |re| + |im|, as in LAPACK's zgetrf; left of a panel nothing is
 // exchanged, since L is not used again.
 // What bounds it: n dependent pivot searches (about 1 us each with the update of
-// the panel's other columns in one CTA, 2 with 800 rows).  Measured, us, cuSOLVER's
+// the panel's other columns in one CTA, 1.7 with 800 rows).  Measured, us, cuSOLVER's
 // zgetrf and zgetrs -> this, one right-hand side: n 24 118 -> 29, 50 157 -> 69, 100 263
-// -> 218, 200 505 -> 442, 400 1104 -> 962, 800 2673 -> 2421; equal at 1000.
+// -> 192, 200 505 -> 396, 400 1104 -> 859, 800 2673 -> 2124, 1000 3344 -> 2940, 1200 4533
+// -> 3921.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -25,12 +26,13 @@ namespace {
 
 constexpr int kW = 16;              // panel columns
 constexpr int kC = 8;               // columns per CTA of the update
+constexpr int kSub = 4;             // panel columns eliminated before the others take their products
 constexpr int kPanelThreads = 512;
 constexpr int kUpdThreads = 256;
 constexpr int kBackThreads = 512;
 constexpr int kBlk = 32;            // rows per step of the back substitution
-// One CTA for everything up to here: us, it and the panels, n 50 69 and 113, 80 139
-// and about 170, 100 227 and 218, 112 273 and about 245.
+// One CTA for everything up to here: us, it and the panels, n 50 69 and about 105,
+// 96 183 and about 185, 100 227 and 192.
 constexpr int kWholeMax = 96;
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b)
@@ -75,9 +77,12 @@ __device__ __forceinline__ int warp_best(double& big)
 }
 
 // gather: 2 kW pairs (to, from), rows of the matrix: where every row that moved,
-// or is at the panel's top, comes from.  Two barriers per column: the pivot row is
-// set aside, then every row is updated (old row j into the pivot's place) and
-// looks for the next column's pivot on the way.
+// or is at the panel's top, comes from.  Steps of kSub columns, their products then
+// applied to the panel's others in one pass: tall panels are bound by their traffic
+// with shared memory (all columns updated at every step: 1630 us for 1347 at n 800,
+// 142 for 120 at 100).  In a step two barriers per column: the pivot row is set
+// aside, then every row is updated (old row j into the pivot's place) and looks for
+// the next column's pivot on the way.
 __global__ void __launch_bounds__(kPanelThreads)
 k_lu64_panel(double2* __restrict__ A, int n, int k0, int w, int2* __restrict__ gather, int* __restrict__ info)
 {
@@ -87,7 +92,7 @@ k_lu64_panel(double2* __restrict__ A, int n, int k0, int w, int2* __restrict__ g
     __shared__ double best[kPanelThreads / 32];
     __shared__ int where[kPanelThreads / 32];
     __shared__ int moved[kW];
-    __shared__ double2 u[kW + 3];  // the pivot row (read past its end in fours, not used)
+    __shared__ double2 u[kSub];  // the pivot row in the step's columns
     double2* M = A + (int64_t)k0 * n + k0;
     double big = -1.0;
     int at = 0;
@@ -101,65 +106,113 @@ k_lu64_panel(double2* __restrict__ A, int n, int k0, int w, int2* __restrict__ g
             at = r;
         }
     }
-    for (int j = 0; j < w; ++j) {
-        {
-            const int from = warp_best(big);
-            if (lane == from) {
-                best[warp] = big;
-                where[warp] = at;
+    for (int j0 = 0; j0 < w; j0 += kSub) {
+        const int e = min(j0 + kSub, w);
+        for (int j = j0; j < e; ++j) {
+            {
+                const int from = warp_best(big);
+                if (lane == from) {
+                    best[warp] = big;
+                    where[warp] = at;
+                }
             }
-        }
-        __syncthreads();  // also: the rows are updated
-        big = lane < warps ? best[lane] : -1.0;
-        at = lane < warps ? where[lane] : j;
-        at = __shfl_sync(0xffffffffu, at, warp_best(big));
-        if (!(big >= 0.0)) at = j;  // no number in the column
-        const double2 piv = p[j * rows + at], ip = cinv(piv);
-        if (tid < w) {
-            u[tid] = p[tid * rows + at];
-            if (tid < j) {  // L is exchanged whole
-                p[tid * rows + at] = p[tid * rows + j];
-                p[tid * rows + j] = u[tid];
+            __syncthreads();  // also: the rows are updated
+            big = lane < warps ? best[lane] : -1.0;
+            at = lane < warps ? where[lane] : j;
+            at = __shfl_sync(0xffffffffu, at, warp_best(big));
+            if (!(big >= 0.0)) at = j;  // no number in the column
+            const double2 piv = p[j * rows + at], ip = cinv(piv);
+            if (tid < w) {
+                const double2 t = p[tid * rows + at];
+                if (tid >= j && tid < e) {
+                    u[tid - j0] = t;
+                } else {  // L and the columns past the step's are exchanged now
+                    p[tid * rows + at] = p[tid * rows + j];
+                    p[tid * rows + j] = t;
+                }
             }
-        }
-        if (tid == 0) {
-            const int t = perm[j];
-            perm[j] = perm[at];
-            perm[at] = t;
-            moved[j] = at;
-            if (piv.x == 0.0 && piv.y == 0.0) atomicCAS(info, 0, k0 + j + 1);
-        }
-        __syncthreads();
-        const int pr = at;
-        big = -1.0;
-        at = rows;
-        for (int r = tid; r < rows; r += blockDim.x) {
-            if (r < j || r == pr) continue;
-            const int to = r == j ? pr : r;
-            const double2 l = cmul(p[j * rows + r], ip);
-            p[j * rows + to] = l;
-            for (int c = j + 1; c < w; c += 4) {
-                double2 a[4];
+            if (tid == 0) {
+                const int t = perm[j];
+                perm[j] = perm[at];
+                perm[at] = t;
+                moved[j] = at;
+                if (piv.x == 0.0 && piv.y == 0.0) atomicCAS(info, 0, k0 + j + 1);
+            }
+            __syncthreads();
+            const int pr = at;
+            big = -1.0;
+            at = j + 1;
+            for (int r = tid; r < rows; r += blockDim.x) {
+                if (r < j || r == pr) continue;
+                const int to = r == j ? pr : r;
+                const double2 l = cmul(p[j * rows + r], ip);
+                p[j * rows + to] = l;
+                double2 a[kSub];
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (c + i < w) a[i] = p[(c + i) * rows + r];
+                for (int i = 1; i < kSub; ++i)
+                    if (j + i < e) a[i] = p[(j + i) * rows + r];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) a[i] = cfms(a[i], l, u[c + i]);
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (c + i < w) p[(c + i) * rows + to] = a[i];
-                if (c == j + 1) {
-                    const double m = fabs(a[0].x) + fabs(a[0].y);
+                for (int i = 1; i < kSub; ++i)
+                    if (j + i < e) {
+                        a[i] = cfms(a[i], l, u[j + i - j0]);
+                        p[(j + i) * rows + to] = a[i];
+                    }
+                if (j + 1 < e) {
+                    const double m = fabs(a[1].x) + fabs(a[1].y);
                     if (m > big) {
                         big = m;
                         at = to;
                     }
                 }
+                if (r == j)
+                    for (int c = j; c < e; ++c) p[c * rows + j] = u[c - j0];
             }
-            if (r == j)
-                for (int c = j; c < w; ++c) p[c * rows + j] = u[c];
         }
-        if (big < 0.0) at = j + 1;
+        if (e == w) break;
+        __syncthreads();  // the step's columns are final
+        if (tid >= e && tid < w) {  // its rows of U, a thread per column
+            double2* col = p + tid * rows + j0;
+#pragma unroll
+            for (int i = 1; i < kSub; ++i) {
+                double2 t = col[i];
+                for (int m = 0; m < i; ++m) t = cfms(t, p[(j0 + m) * rows + j0 + i], col[m]);
+                col[i] = t;
+            }
+        }
+        __syncthreads();
+        big = -1.0;
+        at = e;
+        for (int r = tid; r < rows; r += blockDim.x) {
+            if (r < e) continue;
+            double2 l[kSub];
+#pragma unroll
+            for (int m = 0; m < kSub; ++m) l[m] = p[(j0 + m) * rows + r];
+            for (int c = e; c < w; c += 2) {
+                const bool two = c + 1 < w;
+                double2* c0 = p + c * rows;
+                double2* c1 = two ? c0 + rows : c0;
+                double2 a0 = c0[r], a1 = c1[r], u0[kSub], u1[kSub];
+#pragma unroll
+                for (int m = 0; m < kSub; ++m) {
+                    u0[m] = c0[j0 + m];
+                    u1[m] = c1[j0 + m];
+                }
+#pragma unroll
+                for (int m = 0; m < kSub; ++m) {
+                    a0 = cfms(a0, l[m], u0[m]);
+                    a1 = cfms(a1, l[m], u1[m]);
+                }
+                c0[r] = a0;
+                if (two) c1[r] = a1;
+                if (c == e) {
+                    const double m = fabs(a0.x) + fabs(a0.y);
+                    if (m > big) {
+                        big = m;
+                        at = r;
+                    }
+                }
+            }
+        }
     }
     __syncthreads();
     for (int r = tid; r < rows; r += blockDim.x)
@@ -374,7 +427,7 @@ k_lu64_back(const double2* __restrict__ A, double2* __restrict__ B, int n)
 }  // namespace
 
 // The orders it takes: where it beats cuSOLVER (figures above).
-bool lu64_takes(int64_t n) { return n <= 896; }
+bool lu64_takes(int64_t n) { return n <= 1200; }
 
 static int lu64_status(mh_ctx* ctx, const int* info)
 {

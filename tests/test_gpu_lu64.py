@@ -24,7 +24,7 @@ def _check(A, X, B):
 @pytest.mark.parametrize("n,nrhs", [(1, 1), (2, 3), (7, 1), (8, 2), (15, 1), (16, 1), (17, 2), (31, 1), (32, 9), (33, 1),
                                     (48, 1), (50, 1), (64, 8), (65, 1), (96, 1), (96, 60), (97, 1),
                                     (100, 6), (257, 2), (700, 1), (870, 1),
-                                    (896, 3), (897, 1)])
+                                    (896, 3), (1001, 1), (1200, 1), (1201, 1)])
 def test_solve(mh, gpu, n, nrhs):
     rng = np.random.default_rng(n + nrhs)
     A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
