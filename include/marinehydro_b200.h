@@ -51,7 +51,7 @@ extern "C" {
 #define MH_GF_DELHOMMEAU                 16u  /* ExactGuevelDelhommeau()    src/green_functions/exact_Guevel_Delhommeau.jl */
 
 /* precision of a solve */
-#define MH_PRECISION_FP64   0  /* FP64 assembly + FP64 LU (cuSOLVER zgetrf/zgetrs) */
+#define MH_PRECISION_FP64   0  /* FP64 assembly + pivoted FP64 LU */
 #define MH_PRECISION_MIXED  1  /* FP64-accurate matrices, low-precision LU, FP64 iterative refinement */
 /* FP64 everywhere with the batch structure of the mixed path (mh_hydro_batch
  * and mh_hydro_batch_vjp): the frequency-independent Rankine part once, the
