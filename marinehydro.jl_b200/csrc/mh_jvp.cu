@@ -179,7 +179,11 @@ k_wave_tangent(int kind, const double* __restrict__ geom, const double* __restri
 constexpr int kTW = 64;  // rows (threads) per CTA
 constexpr int kTS = 4;   // series: B, C, E0, E1
 
-// contracted series of every row, then k, 1/k, log k and dk/d(direction) per frequency
+// contracted series of every row, then k, 1/k, log k and dk/d(direction) per frequency.
+// A launch takes kTanMaxFreqs frequencies at most: 16 KB of the 227 KB a CTA may have
+// (all at once, 5553 frequencies did not fit beside the last ring's rows), and a
+// contraction repeated every 512 frequencies costs less than 2% of theirs.
+constexpr int kTanMaxFreqs = 512;
 size_t tan_allw_smem(int nb) { return sizeof(double) * ((size_t)kTS * kTabNU * kTW + 4 * (size_t)nb); }
 
 // G and its derivatives from the four functions' values, L = log((R + |z|) / 2),
@@ -577,29 +581,34 @@ int tangent_matrices(const Batch& bt, const Jvp& jv, const double* d_k, const do
     mh_ctx* ctx = bt.ctx;
     const int64_t n = bt.n;
     if (jv.wave_kind == 2 && tab && nb >= kJvpAllwMinFreqs) {
-        const size_t smem = tan_allw_smem(nb);
         auto* fall = (int*)ws_get(ctx, WS_FALL, (kRings + 1) * sizeof(int));
         if (!fall) return MH_ERR_OOM;
-        MH_CUDA_TRY(ctx, raise_smem_cap((const void*)k_wave_tangent_allw, smem));
-        MH_CUDA_TRY(ctx, cudaMemsetAsync(fall, 0, (kRings + 1) * sizeof(int), ctx->stream));
-        const int cols = wave_cols(n, kGradCols);
-        const dim3 gw(nblk(n, kTW), nblk(n, cols)), g2(nblk(n, kTW), nblk(n, kGradCols));
-        k_wave_tangent_allw<<<gw, kTW, smem, ctx->stream>>>(bt.m->geom, jv.tgeom, n, bt.direct, cols, tab, d_k, d_dk, nb,
-                                                            jv.dSR, jv.dDR, dS, dD, fall);
-        auto ring = [&](auto kern, int q) -> cudaError_t {
-            const cudaError_t e = raise_smem_cap((const void*)kern, tan_ring_smem(q, nb));
-            if (e != cudaSuccess) return e;
-            const int rc = ring_cols(n);
-            kern<<<dim3(nblk(n, kTW), nblk(n, rc)), kTW, tan_ring_smem(q, nb), ctx->stream>>>(
-                fall, bt.m->geom, jv.tgeom, n, bt.direct, rc, tab, d_k, d_dk, nb, jv.dSR, jv.dDR, dS, dD);
-            return cudaGetLastError();
-        };
-        MH_CUDA_TRY(ctx, ring(k_wave_tangent_ring<0>, 0));
-        MH_CUDA_TRY(ctx, ring(k_wave_tangent_ring<1>, 1));
-        MH_CUDA_TRY(ctx, ring(k_wave_tangent_ring<2>, 2));
-        k_wave_tangent_allw_rest<<<g2, kTW, 0, ctx->stream>>>(fall, bt.m->geom, jv.tgeom, n, bt.direct, tab, d_k,
-                                                             d_dk, nb, jv.dSR, jv.dDR, dS, dD);
-        ctx->launches += 4;
+        const int cols = wave_cols(n, kGradCols), rcols = ring_cols(n);
+        const dim3 gw(nblk(n, kTW), nblk(n, cols)), gr(nblk(n, kTW), nblk(n, rcols)), g2(nblk(n, kTW), nblk(n, kGradCols));
+        const int windows = (nb + kTanMaxFreqs - 1) / kTanMaxFreqs;
+        for (int w = 0, z = 0; w < windows; ++w) {
+            const int m = (nb - z + windows - w - 1) / (windows - w);  // even shares
+            const size_t smem = tan_allw_smem(m);
+            double2 *dSz = dS + (int64_t)z * n * n, *dDz = dD + (int64_t)z * n * n;
+            MH_CUDA_TRY(ctx, raise_smem_cap((const void*)k_wave_tangent_allw, smem));
+            MH_CUDA_TRY(ctx, cudaMemsetAsync(fall, 0, (kRings + 1) * sizeof(int), ctx->stream));
+            k_wave_tangent_allw<<<gw, kTW, smem, ctx->stream>>>(bt.m->geom, jv.tgeom, n, bt.direct, cols, tab, d_k + z,
+                                                                d_dk + z, m, jv.dSR, jv.dDR, dSz, dDz, fall);
+            auto ring = [&](auto kern, int q) -> cudaError_t {
+                const cudaError_t e = raise_smem_cap((const void*)kern, tan_ring_smem(q, m));
+                if (e != cudaSuccess) return e;
+                kern<<<gr, kTW, tan_ring_smem(q, m), ctx->stream>>>(fall, bt.m->geom, jv.tgeom, n, bt.direct, rcols, tab,
+                                                                    d_k + z, d_dk + z, m, jv.dSR, jv.dDR, dSz, dDz);
+                return cudaGetLastError();
+            };
+            MH_CUDA_TRY(ctx, ring(k_wave_tangent_ring<0>, 0));
+            MH_CUDA_TRY(ctx, ring(k_wave_tangent_ring<1>, 1));
+            MH_CUDA_TRY(ctx, ring(k_wave_tangent_ring<2>, 2));
+            k_wave_tangent_allw_rest<<<g2, kTW, 0, ctx->stream>>>(fall, bt.m->geom, jv.tgeom, n, bt.direct, tab, d_k + z,
+                                                                 d_dk + z, m, jv.dSR, jv.dDR, dSz, dDz);
+            ctx->launches += 4 + (w > 0);
+            z += m;
+        }
     } else {
         k_wave_tangent<<<dim3(nblk(n, kJR), nblk(n, kGradCols), (unsigned)nb), kJR, 0, ctx->stream>>>(
             jv.wave_kind, bt.m->geom, jv.tgeom, n, bt.direct, jv.wave_kind == 2 ? tab : nullptr, d_k, d_dk, jv.dSR,
