@@ -134,11 +134,19 @@ int mh_ctx_set_lu_backend(mh_ctx* ctx, int backend);
  * before the MMAs, which accumulate onto it).  n = 0 sets the default for
  * sizes with no entry of their own (2 groups, 4 panels, kernel 0); otherwise
  * a size uses the entry nearest to it (in log n).  A new ctx holds the
- * entries the autotuner chose on a B200: 512 -> (1, 4, 1), 1024 -> (2, 2, 0),
- * 2048 -> (2, 4, 0).  No reference counterpart
- * (the reference factors with LAPACK). */
+ * entries the autotuner chose on a B200: 512 -> (1, 4, 1), 1024 and 1536 ->
+ * (1, 4, 0), 2048 -> (2, 8, 0).  These also go by the call's columns in all
+ * (n x matrices): up to 32768 the last runs as (1, 4, 0), above it those of
+ * 1024 and 1536 run as (2, 4, 0).  An entry that is set, or found by the
+ * autotuner, runs as it stands for any number of matrices; setting the values
+ * a new ctx holds for n gives n its built-in entry back, this rule included.
+ * mh_ctx_get_lu_schedule returns the entry (n = 0: the default),
+ * mh_ctx_get_lu_schedule_for what a factorisation of nbatch matrices runs.
+ * No reference counterpart (the reference factors with LAPACK). */
 int mh_ctx_set_lu_schedule(mh_ctx* ctx, int64_t n, int groups, int outer_panels, int update_kernel);
 int mh_ctx_get_lu_schedule(mh_ctx* ctx, int64_t n, int* groups, int* outer_panels, int* update_kernel);
+int mh_ctx_get_lu_schedule_for(mh_ctx* ctx, int64_t n, int64_t nbatch, int* groups, int* outer_panels,
+                               int* update_kernel);
 
 /* Autotuner of that schedule: factors nbatch synthetic n x n diagonally
  * dominant matrices (generated on the device) with each of the ncand

@@ -82,6 +82,8 @@ SIGNATURES = {
     "mh_ctx_set_lu_schedule": (ctypes.c_int, [_P, ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_int]),
     "mh_ctx_get_lu_schedule": (ctypes.c_int, [_P, ctypes.c_int64, ctypes.POINTER(ctypes.c_int),
                                               ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]),
+    "mh_ctx_get_lu_schedule_for": (ctypes.c_int, [_P, ctypes.c_int64, ctypes.c_int64, ctypes.POINTER(ctypes.c_int),
+                                                  ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]),
     "mh_lu_autotune": (ctypes.c_int, [_P, ctypes.c_int64, ctypes.c_int64, ctypes.c_int,
                                       ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int),
                                       ctypes.POINTER(ctypes.c_int), _D, ctypes.POINTER(ctypes.c_int)]),
@@ -236,14 +238,19 @@ class Context:
                      (1, 4, 1), (2, 2, 1), (2, 4, 1), (2, 6, 1), (3, 4, 1), (4, 4, 1))
 
     def set_lu_schedule(self, n: int, groups: int, outer_panels: int, update_kernel: int = 0):
-        """Tensor-core LU schedule for matrices of n panels (n = 0: the default)."""
+        """Tensor-core LU schedule for matrices of n panels (n = 0: the default).
+        The values a new Context holds for n give n its built-in entry back."""
         check(lib().mh_ctx_set_lu_schedule(self._h, int(n), int(groups), int(outer_panels), int(update_kernel)),
               self._h)
 
-    def lu_schedule(self, n: int = 0) -> tuple:
+    def lu_schedule(self, n: int = 0, nbatch: int | None = None) -> tuple:
+        """The entry used for n, or with nbatch what that many matrices of n run."""
         g, o, u = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
-        check(lib().mh_ctx_get_lu_schedule(self._h, int(n), ctypes.byref(g), ctypes.byref(o), ctypes.byref(u)),
-              self._h)
+        to = ctypes.byref(g), ctypes.byref(o), ctypes.byref(u)
+        if nbatch is None:
+            check(lib().mh_ctx_get_lu_schedule(self._h, int(n), *to), self._h)
+        else:
+            check(lib().mh_ctx_get_lu_schedule_for(self._h, int(n), int(nbatch), *to), self._h)
         return int(g.value), int(o.value), int(u.value)
 
     def autotune_lu(self, n: int, nbatch: int, candidates=None) -> dict:

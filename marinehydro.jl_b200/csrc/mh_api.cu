@@ -243,6 +243,34 @@ int dof_upload(mh_ctx* ctx, const mh_mesh* m, const double* dof, int64_t dof_row
     return MH_OK;
 }
 
+// The LU schedules of a new ctx: those the autotuner chose on a B200 (mh_lu_autotune, median of
+// three to seven sweeps; ms against the next best): 512 panels x 16 matrices, 1
+// group x 4 panels with C staged in tensor memory (0.378 vs 0.379); 1224 x 16, 1
+// x 4 (1.09 vs 1.10); 2048 x 64, 2 x 8 (4.68; 4.88 vs 5.03 for 2 x 6 in one run).  Other sizes
+// take the nearest entry.  The number of matrices decides between one group,
+// whose chain of panels is the critical path, and two, which overlap each
+// other's: the line is at kLuFewColumns columns in all.  Two for one above it:
+// 1024 x 64 1.30 vs 1.40, 1456 x 32 1.78 vs 1.79; 1 x 4 for 2 x 8 up to it: 2048
+// x 1 1.61 vs 1.80, x 8 1.80 vs 2.22, x 16 2.22 vs 2.41, 2997 x 8 3.30 vs 3.60,
+// 4096 x 4 4.09 vs 4.75 (past it 2997 x 16 4.92 vs 4.64, 4096 x 12 6.89 vs 6.35).
+// mh_ctx_set_lu_schedule or the autotuner replace them.
+const LuTable& builtin_lu_table()
+{
+    static const LuTable t = {{512, LuSchedule{1, 4, 1}}, {1024, LuSchedule{1, 4, 0, 0, 2}},
+                              {1536, LuSchedule{1, 4, 0, 0, 2}}, {2048, LuSchedule{2, 8, 0, 4, 0}}};
+    return t;
+}
+
+void put_lu_schedule(mh_ctx* ctx, int64_t n, const LuSchedule& s)
+{
+    for (auto& e : ctx->lu_table)
+        if (e.first == n) {
+            e.second = s;
+            return;
+        }
+    ctx->lu_table.emplace_back(n, s);
+}
+
 // Shared pipeline of the two front doors: assembly, bc, solve, force.
 int front_door(mh_ctx* ctx, const mh_mesh* m, const double* dof, int64_t dof_rows, double omega,
                double rho, double g, uint32_t gf_mask, int direct, int precision, bool diffraction,
@@ -362,19 +390,7 @@ int mh_ctx_create(int device, mh_ctx** out)
     }
     cublasSetStream(ctx->cublas, ctx->stream);
     cusolverDnSetStream(ctx->cusolver, ctx->stream);
-    // LU schedules the autotuner chose on a B200 (mh_lu_autotune, median of
-    // three to seven sweeps; ms against the next best): 512 panels x 16 matrices, 1
-    // group x 4 panels with C staged in tensor memory (0.378 vs 0.379); 1224 x 16, 1
-    // x 4 (1.09 vs 1.10); 2048 x 64, 2 x 8 (4.68; 4.88 vs 5.03 for 2 x 6 in one run).  Other sizes
-    // take the nearest entry.  The number of matrices decides between one group,
-    // whose chain of panels is the critical path, and two, which overlap each
-    // other's: the line is at kLuFewColumns columns in all.  Two for one above it:
-    // 1024 x 64 1.30 vs 1.40, 1456 x 32 1.78 vs 1.79; 1 x 4 for 2 x 8 up to it: 2048
-    // x 1 1.61 vs 1.80, x 8 1.80 vs 2.22, x 16 2.22 vs 2.41, 2997 x 8 3.30 vs 3.60,
-    // 4096 x 4 4.09 vs 4.75 (past it 2997 x 16 4.92 vs 4.64, 4096 x 12 6.89 vs 6.35).
-    // mh_ctx_set_lu_schedule or the autotuner replace them.
-    ctx->lu_table = {{512, LuSchedule{1, 4, 1}}, {1024, LuSchedule{1, 4, 0, 0, 2}}, {1536, LuSchedule{1, 4, 0, 0, 2}},
-                     {2048, LuSchedule{2, 8, 0, 4, 0}}};
+    ctx->lu_table = builtin_lu_table();
     *out = ctx;
     return MH_OK;
 }
@@ -595,12 +611,14 @@ int mh_ctx_set_lu_schedule(mh_ctx* ctx, int64_t n, int groups, int outer_panels,
         ctx->lu_default = s;
         return MH_OK;
     }
-    for (auto& e : ctx->lu_table)
-        if (e.first == n) {
-            e.second = s;
-            return MH_OK;
-        }
-    ctx->lu_table.emplace_back(n, s);
+    // the values a new ctx holds for n: that entry again, with its rule by columns
+    const LuSchedule* own = lu_nearest(builtin_lu_table(), n);
+    if (s.runs_as(*own)) {
+        s = *own;
+        s.one_size = true;
+        for (const auto& e : builtin_lu_table()) s.one_size = s.one_size && e.first != n;
+    }
+    put_lu_schedule(ctx, n, s);
     return MH_OK;
 }
 
@@ -611,6 +629,20 @@ int mh_ctx_get_lu_schedule(mh_ctx* ctx, int64_t n, int* groups, int* outer_panel
     if (n < 0 || !groups || !outer_panels || !update_kernel)
         return set_err(ctx, MH_ERR_ARG, "bad arguments to mh_ctx_get_lu_schedule");
     const LuSchedule s = n == 0 ? ctx->lu_default : ctx->lu_schedule(n);
+    *groups = s.groups;
+    *outer_panels = s.outer;
+    *update_kernel = s.update;
+    return MH_OK;
+}
+
+int mh_ctx_get_lu_schedule_for(mh_ctx* ctx, int64_t n, int64_t nbatch, int* groups, int* outer_panels,
+                               int* update_kernel)
+{
+    int rc;
+    if ((rc = check_ctx(ctx))) return rc;
+    if (n < 1 || nbatch < 1 || !groups || !outer_panels || !update_kernel)
+        return set_err(ctx, MH_ERR_ARG, "bad arguments to mh_ctx_get_lu_schedule_for");
+    const LuSchedule s = ctx->lu_schedule(n, nbatch);
     *groups = s.groups;
     *outer_panels = s.outer;
     *update_kernel = s.update;
@@ -671,8 +703,11 @@ int mh_lu_autotune(mh_ctx* ctx, int64_t n, int64_t nbatch, int ncand, const int*
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (e != cudaSuccess) return set_err(ctx, MH_ERR_CUDA, "LU autotune: %s", cudaGetErrorString(e));
-    if ((rc = mh_ctx_set_lu_schedule(ctx, n, groups[fastest], outer_panels[fastest], update_kernel[fastest])))
-        return rc;
+    LuSchedule tuned;  // as it was timed: no rule by columns, also where the values are a built-in entry's
+    tuned.groups = groups[fastest];
+    tuned.outer = outer_panels[fastest];
+    tuned.update = update_kernel[fastest];
+    put_lu_schedule(ctx, n, tuned);
     if (best) *best = fastest;
     return MH_OK;
 }

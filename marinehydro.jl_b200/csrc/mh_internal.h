@@ -67,27 +67,48 @@ enum Phase : int {
 // solves) overlaps another's trailing updates: at most this many.
 constexpr int kLuGroups = 4;
 
-// Schedule of the tensor-core LU: groups of matrices on their own stream
-// pairs (1 .. kLuGroups), 64-column panels per outer step (even, 2 .. 8) and
-// the trailing-update kernel (0: C through shared memory after the MMAs,
-// 1: C staged in tensor memory before them).  Built-in entries also say what
-// replaces them by a call's columns in all (n x matrices), if not 0: few_outer, one
-// group with that many panels per outer step up to kLuFewColumns; many_groups, that
-// many groups above it.
 // The streams and events one group of the tensor-core LU runs on.
 struct LuStreams {
     cudaStream_t main, side, strip;
     cudaEvent_t ev_side, ev_panel, ev_strip_go, ev_strip_done;
 };
 
+// Schedule of the tensor-core LU: groups of matrices on their own stream
+// pairs (1 .. kLuGroups), 64-column panels per outer step (even, 2 .. 8) and
+// the trailing-update kernel (0: C through shared memory after the MMAs,
+// 1: C staged in tensor memory before them).  Built-in entries also say what
+// replaces them by a call's columns in all (n x matrices), if not 0: few_outer, one
+// group with that many panels per outer step up to kLuFewColumns; many_groups, that
+// many groups above it.  one_size: the entry serves its own n only, not the sizes
+// nearest to it (a built-in entry set again for a size without one).
 struct LuSchedule {
     int groups = 2;
     int outer = 4;
     int update = 0;
     int few_outer = 0;
     int many_groups = 0;
+    bool one_size = false;
+    bool runs_as(const LuSchedule& o) const { return groups == o.groups && outer == o.outer && update == o.update; }
 };
 constexpr int64_t kLuFewColumns = 32768;
+
+using LuTable = std::vector<std::pair<int64_t, LuSchedule>>;
+
+// The entry of a size: its own, else the nearest in log n, else none.
+inline const LuSchedule* lu_nearest(const LuTable& table, int64_t n)
+{
+    const LuSchedule* best = nullptr;
+    double gap = 1e300;
+    for (const auto& e : table) {
+        if (e.second.one_size && e.first != n) continue;
+        const double d = std::fabs(std::log((double)e.first / (double)n));
+        if (d < gap) {
+            gap = d;
+            best = &e.second;
+        }
+    }
+    return best;
+}
 
 struct mh_ctx {
     int device = 0;
@@ -123,20 +144,24 @@ struct mh_ctx {
     int wave_series_fp32 = 1;
     // LU schedules by matrix size (set by hand or by the autotuner); sizes
     // with no entry use the nearest entry in log n, else lu_default
-    std::vector<std::pair<int64_t, LuSchedule>> lu_table;
+    LuTable lu_table;
     LuSchedule lu_default;
     LuSchedule lu_schedule(int64_t n) const
     {
-        const LuSchedule* best = &lu_default;
-        double gap = 1e300;
-        for (const auto& e : lu_table) {
-            const double d = std::fabs(std::log((double)e.first / (double)n));
-            if (d < gap) {
-                gap = d;
-                best = &e.second;
-            }
+        const LuSchedule* s = lu_nearest(lu_table, n);
+        return s ? *s : lu_default;
+    }
+    // What a factorisation of nbatch matrices of n runs.
+    LuSchedule lu_schedule(int64_t n, int64_t nbatch) const
+    {
+        LuSchedule s = lu_schedule(n);
+        const bool few = n * nbatch <= kLuFewColumns;
+        if (s.few_outer && few) {
+            s.groups = 1;
+            s.outer = s.few_outer;
         }
-        return *best;
+        if (s.many_groups && !few) s.groups = s.many_groups;
+        return s;
     }
     // refinement sweeps launched before the first host check, per direction
     // (0: D x = b, 1: D^H x = b): the most any matrix needed in the last call

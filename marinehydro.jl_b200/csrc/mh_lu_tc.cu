@@ -1837,13 +1837,7 @@ cudaError_t launch_lu_tc(mh_ctx* ctx, float2* A, int64_t n, int64_t stride, int 
     cudaError_t e;
     static_assert(TC_NB == 64, "the diagonal blocks are factored by k_lu_diag64");
     static_assert(TC_TM == 2 * TC_NB && TC_TN == TC_TM, "two panels per 128-wide tile");
-    LuSchedule sched = ctx->lu_schedule(n);
-    const bool few = n * nbatch <= kLuFewColumns;
-    if (sched.few_outer && few) {
-        sched.groups = 1;
-        sched.outer = sched.few_outer;
-    }
-    if (sched.many_groups && !few) sched.groups = sched.many_groups;
+    const LuSchedule sched = ctx->lu_schedule(n, nbatch);
     if (sched.groups < 1 || sched.groups > kLuGroups || sched.outer < 2 || sched.outer > kOuterMax ||
         (sched.outer & 1) || sched.update < 0 || sched.update > 1)
         return cudaErrorInvalidValue;
