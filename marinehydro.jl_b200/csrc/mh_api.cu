@@ -173,10 +173,11 @@ int sync_status(mh_ctx* ctx, const char* what)
 }
 
 // LU-factorise A (n x n, device, overwritten) and solve A X = B in place
-// (B: n x nrhs, device): mh_lu64.cu, or cuSOLVER zgetrf/zgetrs for large orders.
+// (B: n x nrhs, device): mh_lu64.cu, or cuSOLVER zgetrf/zgetrs for large orders or
+// many right-hand sides.
 int lu_solve_fp64(mh_ctx* ctx, int64_t n, double2* A, double2* B, int64_t nrhs)
 {
-    if (mh::lu64_takes(n)) return mh::lu64_solve(ctx, n, A, B, (int)nrhs);
+    if (mh::lu64_takes(n, nrhs)) return mh::lu64_solve(ctx, n, A, B, (int)nrhs);
     int lwork = 0;
     cusolverStatus_t st = cusolverDnZgetrf_bufferSize(ctx->cusolver, (int)n, (int)n,
                                                       (cuDoubleComplex*)A, (int)n, &lwork);

@@ -264,7 +264,7 @@ cudaError_t launch_lu_solve_cluster(mh_ctx* ctx, bool conj_trans, const float2* 
                                     int nrhs, int* bad, const int* done, const int* unset_flag, cudaStream_t stream);
 // FP64 solve of one matrix with partial pivoting (mh_lu64.cu): A X = B, A
 // overwritten, X in place of B; the stream is waited for.
-bool lu64_takes(int64_t n);
+bool lu64_takes(int64_t n, int64_t nrhs);
 int lu64_solve(mh_ctx* ctx, int64_t n, double2* A, double2* B, int nrhs);
 // Conjugate-transposed solve D^H X = X with the factors of launch_lu_tc
 // (backend MH_LU_TCGEN05_F16) or launch_lu_f32 (MH_LU_SIMT_F32).

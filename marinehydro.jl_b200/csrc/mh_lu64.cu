@@ -1,8 +1,8 @@
 // FP64 complex solve A X = B with partial pivoting for one matrix of moderate
 // order: the calls for one frequency (forces, solve).  The FP64 batches and their
 // adjoints keep cuSOLVER, whose factors the adjoint solves with again.  B rides
-// along as further columns.  Up to kWholeMax panels k_lu64_whole does all of it in
-// one CTA; else panels of kW columns, and per panel
+// along as further columns.  Small orders with few of them are all k_lu64_whole's, in
+// one CTA (whole_most); else panels of kW columns, and per panel
 //   k_lu64_panel   one CTA factors the panel in shared memory and records the row
 //                  exchanges as a gather;
 //   k_lu64_update  a CTA takes kC columns to the right (of A, then of B): gathers
@@ -31,9 +31,13 @@ constexpr int kPanelThreads = 512;
 constexpr int kUpdThreads = 256;
 constexpr int kBackThreads = 512;
 constexpr int kBlk = 32;            // rows per step of the back substitution
-// One CTA for everything up to here: us, it and the panels, n 50 69 and about 105,
-// 96 183 and about 185, 100 227 and 192.
-constexpr int kWholeMax = 96;
+// Right-hand sides up to which one CTA does everything: its time grows with them (a
+// CTA's threads walk all columns), the panels' hardly does.  us for the call's
+// kernels, it and the panels: n 8, 32 right-hand sides 37 and 44; 32, 32 73 and 81, 48
+// 84 and 82; 40, 24 101 and 104, 32 112 and 105; 50, 1 84 and 117, 16 102 and 118, 32
+// 134 and 129, 64 180 and 126; 64, 12 128 and 135, 24 157 and 142; 72, 8 155 and 156;
+// 80, 1 155 and 165, 6 173 and 166; 96, 1 200 and 197, 32 329 and 205.
+constexpr int whole_most(int64_t n) { return n <= 32 ? 40 : n <= 86 ? (int)(88 - n) / 2 : n < 96; }
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b)
 {
@@ -426,8 +430,11 @@ k_lu64_back(const double2* __restrict__ A, double2* __restrict__ B, int n)
 
 }  // namespace
 
-// The orders it takes: where it beats cuSOLVER (figures above).
-bool lu64_takes(int64_t n) { return n <= 1200; }
+// What it takes: where it beats cuSOLVER.  By the order as above; by the right-hand
+// sides since its products of A22 and B are not as fast as the library's.  us, cuSOLVER and
+// it, 768 and 1500 of them: n 50 186 and 159, 188 and 220; 400 1592 and 1287, 1664 and
+// 1817; 800 3804 and 3413, 4046 and 4565; 1200 6447 and 6428, 7032 and 8776.
+bool lu64_takes(int64_t n, int64_t nrhs) { return n <= 1200 && nrhs <= 768; }
 
 static int lu64_status(mh_ctx* ctx, const int* info)
 {
@@ -442,16 +449,16 @@ static int lu64_status(mh_ctx* ctx, const int* info)
 // A X = B, A overwritten, X in place of B; MH_ERR_SINGULAR at a zero pivot.
 int lu64_solve(mh_ctx* ctx, int64_t n, double2* A, double2* B, int nrhs)
 {
-    const size_t whole = sizeof(double2) * ((size_t)(n + nrhs) * (size_t)n + (size_t)(2 * n + nrhs + 3));
     auto* gather = (int2*)ws_get(ctx, WS_PIV, sizeof(int2) * 2 * kW);
     auto* info = (int*)ws_get(ctx, WS_INFO, sizeof(int) * 2);
     if (!gather || !info) return MH_ERR_OOM;
     MH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_lu64_panel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)kPanelSmemMax));
     MH_CUDA_TRY(ctx, cudaMemsetAsync(info, 0, sizeof(int), ctx->stream));
-    if (n <= kWholeMax && whole <= kPanelSmemMax) {
+    if (nrhs <= whole_most(n)) {
         MH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_lu64_whole, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)kPanelSmemMax));
+        const size_t whole = sizeof(double2) * ((size_t)(n + nrhs) * (size_t)n + (size_t)(2 * n + nrhs + 3));
         const int rows = (int)(n + 31) / 32 * 32, groups = kPanelThreads / rows;
         k_lu64_whole<<<1, rows * groups, whole, ctx->stream>>>(A, B, (int)n, nrhs, rows, info);
         ctx->launches += 1;
