@@ -166,6 +166,7 @@ struct mh_ctx {
     // refinement sweeps launched before the first host check, per direction
     // (0: D x = b, 1: D^H x = b): the most any matrix needed in the last call
     int refine_ahead[2] = {2, 2};
+    int solve_clusters[9] = {};  // clusters of 1 .. 8 CTAs of the triangular solve that run at once (0: not asked yet)
     double* delh_table = nullptr;  // device, kTabAllWords doubles (built on first use)
     bool profile = false;
     // phase timing: events recorded on whichever stream issues the phase

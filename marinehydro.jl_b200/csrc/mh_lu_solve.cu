@@ -21,9 +21,12 @@
 // through a ring of shared-memory stages with cp.async (16 bytes a copy where n is
 // even, 8 otherwise; entries past the matrix are zero-filled) while eight consumer
 // warps multiply, and the tile stream runs ahead of the chain.
-// Cluster size: the CTAs that fill the chip with one per SM (8, 6, 4, 2 or 1 per
-// matrix), at most one per row block: a CTA's ring takes an SM's shared memory, so
-// a second wave of clusters would double the chain.
+// Cluster size: the most CTAs a matrix (up to 8, one per row block) that let all
+// clusters run at once; a CTA's ring takes an SM's shared memory, and a second wave
+// of clusters would double the chain.  A cluster lives in one GPC, so fewer fit than
+// the SMs would hold: the runtime says how many (us a solve at 800 panels with 4
+// right-hand sides, the SMs counted and this: 16 to 18 matrices 121 and 61, 23 and 24
+// 119 and 63, 34 to 37 130 and 77, 38 to 45 98 and 78, the others as they were).
 //
 // Every wait is bounded: a stage wait that runs out marks the matrix in `bad` (2),
 // a wait for a block marks it (3) and later blocks are not waited for; every block
@@ -439,6 +442,38 @@ SolveKernel solve_of(int nq)
     }
 }
 
+cudaLaunchConfig_t solve_config(cudaLaunchAttribute (&at)[1], int nbatch, int cs, size_t smem, cudaStream_t stream)
+{
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)cs;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)nbatch * (unsigned)cs);
+    cfg.blockDim = dim3(kScThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// Clusters of cs CTAs (with an SM's shared memory each) that run at once.
+cudaError_t clusters_at_once(mh_ctx* ctx, SolveKernel k, size_t smem, int cs, int* out)
+{
+    int& n = ctx->solve_clusters[cs];
+    if (n == 0) {
+        cudaLaunchAttribute at[1];
+        cudaLaunchConfig_t cfg = solve_config(at, 1, cs, smem, ctx->stream);
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, (const void*)k, &cfg);
+        if (e != cudaSuccess) {
+            n = 0;
+            return e;
+        }
+    }
+    *out = n;
+    return cudaSuccess;
+}
+
 }  // namespace
 
 bool lu_solve_cluster_fits(int64_t n) { return sc_smem((n + kScNB - 1) / kScNB, 1, 2) <= kScSmemMax; }
@@ -453,9 +488,6 @@ cudaError_t launch_lu_solve_cluster(mh_ctx* ctx, bool conj_trans, const float2* 
     int most = 8;
     while (sc_smem(nblk, most, 2) > kScSmemMax) --most;
     const int passes = (nrhs + most - 1) / most;
-    int cs = 1;
-    for (int c : {2, 4, 6, 8})
-        if (c <= nblk && (int64_t)nbatch * c <= 148) cs = c;
     const int vec = n % 2 == 0 && stride % 2 == 0 && ((uintptr_t)A & 15) == 0;
     for (int p = 0, q0 = 0; p < passes; ++p) {
         const int nq = (nrhs - q0 + passes - p - 1) / (passes - p);
@@ -465,17 +497,14 @@ cudaError_t launch_lu_solve_cluster(mh_ctx* ctx, bool conj_trans, const float2* 
         const size_t smem = sc_smem(nblk, nq, stages);
         cudaError_t e = raise_smem_cap((const void*)k, smem);
         if (e != cudaSuccess) return e;
+        int cs = (int)std::min<int64_t>(8, nblk);
+        for (int room = 0; cs > 1; --cs) {
+            if ((int64_t)nbatch * cs > 148) continue;
+            if ((e = clusters_at_once(ctx, k, smem, cs, &room)) != cudaSuccess) return e;
+            if (nbatch <= room) break;
+        }
         cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)cs;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned)nbatch * (unsigned)cs);
-        cfg.blockDim = dim3(kScThreads);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = stream;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
+        const cudaLaunchConfig_t cfg = solve_config(at, nbatch, cs, smem, stream);
         if ((e = cudaLaunchKernelEx(&cfg, k, A, n, stride, Dinv, dstride, X + (int64_t)q0 * n, xstride, stages, vec, bad,
                                     done, unset_flag)) != cudaSuccess)
             return e;

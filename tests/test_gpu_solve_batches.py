@@ -1,6 +1,7 @@
 """The clustered triangular solve on batches of matrices that differ from their
-neighbours: clusters of 8 CTAs per matrix down to one, both directions, one to five
-right-hand sides.
+neighbours: every cluster size (as many CTAs per matrix as let all clusters run at
+once, 8 for one matrix down to 1 for 160), batches around the sizes at which the
+clusters of a size no longer fit, both directions, one to nine right-hand sides.
 
 Bound as in test_gpu_solve_clusters.py: FP32 substitution with factors of a matrix
 whose condition is below 10 rounds to within 2e-6 of the largest entry; 1e-5 is
@@ -18,8 +19,9 @@ def _batch(rng, nb, n):
 
 
 @pytest.mark.parametrize("conj", [False, True])
-@pytest.mark.parametrize("nb,n,nrhs", [(1, 520, 2), (15, 513, 1), (22, 390, 2), (30, 330, 5), (48, 193, 2), (74, 130, 3),
-                                       (160, 130, 1)])
+@pytest.mark.parametrize("nb,n,nrhs", [(1, 520, 2), (15, 513, 1), (16, 520, 3), (18, 449, 4), (22, 390, 2), (24, 385, 8),
+                                       (27, 321, 1), (30, 330, 5), (36, 257, 4), (37, 258, 1), (45, 200, 9), (48, 193, 2),
+                                       (74, 130, 3), (75, 131, 2), (160, 130, 1)])
 def test_every_matrix_its_own(mh, gpu, conj, nb, n, nrhs):
     rng = np.random.default_rng(nb + n + nrhs)
     A = _batch(rng, nb, n)
