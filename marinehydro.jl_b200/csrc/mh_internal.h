@@ -50,7 +50,7 @@ struct mh_mesh {
 enum WsSlot : int {
     WS_S = 0, WS_D, WS_RHS, WS_PHI, WS_TMP, WS_PIV, WS_INFO, WS_LWORK,
     WS_DOF, WS_OUT, WS_LO, WS_DINV, WS_TMP32, WS_MISC, WS_SR, WS_TMP32B, WS_PANEL, WS_FB,
-    WS_ADJ, WS_WSD, WS_PART, WS_GBAR, WS_TAPE, WS_FLAGS, WS_FLAGS2, WS_NEAR, WS_NEARRES, WS_FALL, WS_REPACK, WS_NSLOTS
+    WS_ADJ, WS_WSD, WS_PART, WS_GBAR, WS_TAPE, WS_FLAGS, WS_NEAR, WS_NEARRES, WS_FALL, WS_REPACK, WS_NSLOTS
 };
 
 // Largest number of right-hand sides (radiating dofs + headings) per frequency.
@@ -245,21 +245,16 @@ cudaError_t launch_lu_solve_blocks32(mh_ctx* ctx, const float2* A, int64_t n, in
                                      int nbatch, const float2* Dinv, float2* X, float2* T,
                                      int64_t xstride, int nrhs);
 
-// Persistent (one CTA per matrix, one launch) solve with the factors of
-// launch_lu_tc / launch_lu_f32: X <- (LU)^-1 X, or (LU)^-H X when conj_trans.
-// bad (device, per matrix, may be null): a flag wait of the tensor-core
-// backend that runs out writes 3 there.  done (device, per matrix, may be
-// null; needs bad): matrices with done[b] or bad[b] nonzero are skipped.
-// stream: where to launch (null: the ctx stream); flags_slot: the workspace
-// slot of the hand-off flags (solves running concurrently need their own).
+// Whole solve (one CTA or cluster per matrix) with the factors of launch_lu_tc /
+// launch_lu_f32: X <- (LU)^-1 X, or (LU)^-H X when conj_trans.
+// bad (device, per matrix, may be null): a wait of the tensor-core backend that
+// runs out writes 2 or 3 there.  done (device, per matrix, may be null; needs
+// bad): matrices with done[b] or bad[b] nonzero are skipped.
 cudaError_t launch_lu_solve_persist(mh_ctx* ctx, int backend, bool conj_trans, const float2* A, int64_t n,
                                     int64_t stride, int nbatch, const float2* Dinv, float2* X, int64_t xstride,
-                                    int nrhs, int* bad = nullptr, const int* done = nullptr,
-                                    cudaStream_t stream = nullptr, int flags_slot = WS_FLAGS);
+                                    int nrhs, int* bad = nullptr, const int* done = nullptr);
 // The tensor-core backend's part of it (mh_lu_solve.cu): bad is required;
 // unset_flag (may be null): failure injection, a flag that nothing publishes.
-// lu_solve_cluster_fits: whether the solution fits a CTA's shared memory.
-bool lu_solve_cluster_fits(int64_t n);
 cudaError_t launch_lu_solve_cluster(mh_ctx* ctx, bool conj_trans, const float2* A, int64_t n, int64_t stride,
                                     int nbatch, const float2* Dinv, int64_t dstride, float2* X, int64_t xstride,
                                     int nrhs, int* bad, const int* done, const int* unset_flag, cudaStream_t stream);
