@@ -668,15 +668,12 @@ FP32_PEAK_TFLOPS = 74.5
 # Of the per pair-frequency operations, the Horner series (112) runs in FP32
 # at the mixed path's default series level (1), the rest (32) in FP64.
 WAVE_FP32_FLOPS_PER_PAIR_FREQ = 112.0
-# DRAM bytes of the LU phase per matrix of 2048, from an ncu capture of the
-# three LU kernels over one factorisation of 16 matrices of 2048 with the
-# default schedule (2 groups x 8 panels per outer step; the FP32 Schur
-# complement re-read once per 512-column outer step, the left-looking tile
-# updates, panels and diagonal blocks): 3.677 GB / 16 = 229.8 MB per matrix
-# (14.7 GB per 64; 16.7 GB with 256-column steps and right-looking strips).
-# Captured with the 64 KB U12 operand images; their halving since cuts
-# mostly L2 traffic (the images are re-read from L2 by every update CTA).
-LU_DRAM_BYTES_PER_MATRIX_2048 = 3.677e9 / 16
+# DRAM bytes of the LU phase per matrix of 2048, from an ncu capture of its
+# kernels over one factorisation of 20 matrices of 2048 with the schedule of 64
+# (2 groups x 8 panels per outer step): 3.710 GB / 20 = 185.5 MB per matrix (11.9
+# GB per 64).  Reads with cold caches per launch; writes leave L2 after a kernel
+# ends and hardly appear.
+LU_DRAM_BYTES_PER_MATRIX_2048 = 3.710e9 / 20
 
 
 def roofline(per_phase, n, args):

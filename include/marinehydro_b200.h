@@ -169,7 +169,7 @@ int mh_lu_autotune(mh_ctx* ctx, int64_t n, int64_t nbatch, int ncand, const int*
 int mh_ctx_set_wave_series_fp32(mh_ctx* ctx, int level);
 
 /* Failure injection for tests (no reference counterpart): while enabled, the
- * flag waits of the tensor-core backend's triangular solves on this ctx wait
+ * waits for other CTAs' blocks in the tensor-core backend's triangular solves wait
  * on a flag that nothing publishes, with a limit of 64 polls, so each wait
  * expires the way a lost hand-off would.  The solve marks its matrices:
  * mh_lu_solve_lowp returns MH_ERR_TIMEOUT, the batched mixed paths solve the

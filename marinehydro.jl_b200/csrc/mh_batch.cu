@@ -459,9 +459,9 @@ __device__ __forceinline__ unsigned long long abs_bits(double re, double im)
 // memory (no barrier until the end), and the warps' sums are added in warp
 // order.  Splitting the columns over the warps is what fills the chip when
 // the matrices are few or small: one thread per row running down all columns
-// (the form before this one) left a chain of n loads on n / 256 CTAs.
+// leaves a chain of n loads on n / 256 CTAs.
 // Measured on a B200, N = panels, w = matrices, q = right-hand sides, us per
-// product (HBM time at 6.5 TB/s in brackets), before -> now:
+// product (HBM time at 6.5 TB/s in brackets), a thread per row -> this:
 //   N 1224, w 16, q 8: 1625 -> 132 (59);   N 2048, w 1, q 3: 580 -> 30 (10);
 //   N 870, w 16, q 1: 258 -> 48 (30);      N 200, w 20, q 7: 177 -> 9 (2);
 //   N 1456, w 32, q 3: 455 -> 225 (167);   N 2997, w 24, q 2: 968 -> 602 (530);

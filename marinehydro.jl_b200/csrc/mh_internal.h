@@ -134,7 +134,7 @@ struct mh_ctx {
     int64_t launches = 0;
     int delh_method = MH_DELHOMMEAU_TABLE;
     int lu_backend = MH_LU_TCGEN05_F16;
-    // failure injection (tests): the triangular solves' flag waits wait on a
+    // failure injection (tests): the triangular solves' waits for blocks wait on a
     // flag that nothing publishes, so they expire
     bool inject_wait_timeout = false;
     // reduced-precision levels of the frequency-batched Delhommeau pass
