@@ -9,7 +9,9 @@
 //                  the exchanged rows, U12 = inv(L11) A12 by shuffles, A22 -= L21 U12;
 // then k_lu64_back, a CTA per column of B, substitutes back.  The pivot is the
 // entry of largest |re| + |im|, as in LAPACK's zgetrf; left of a panel nothing is
-// exchanged, since L is not used again.
+// exchanged, since L is not used again.  A zero pivot is refused, and so is a column
+// without a number left where infinite entries (of A, or by overflow) brought that
+// about; a NaN in A goes through to the solution.
 // What bounds it: n dependent pivot searches (about 1 us each with the update of
 // the panel's other columns in one CTA, 1.7 with 800 rows).  Measured, us, cuSOLVER's
 // zgetrf and zgetrs -> this, one right-hand side: n 24 118 -> 29, 50 157 -> 69, 100 263
@@ -140,7 +142,7 @@ k_lu64_panel(double2* __restrict__ A, int n, int k0, int w, int2* __restrict__ g
                 perm[j] = perm[at];
                 perm[at] = t;
                 moved[j] = at;
-                if (piv.x == 0.0 && piv.y == 0.0) atomicCAS(info, 0, k0 + j + 1);
+                if (!(big > 0.0)) atomicCAS(info, 0, big == 0.0 ? k0 + j + 1 : -(k0 + j + 1));
             }
             __syncthreads();
             const int pr = at;
@@ -264,7 +266,7 @@ k_lu64_whole(const double2* __restrict__ A, double2* __restrict__ B, int n, int 
         if (!(big >= 0.0)) at = j;  // no number in the column
         const double2 piv = p[j * n + at], ip = cinv(piv);
         for (int c = j + tid; c < W; c += blockDim.x) u[c] = p[c * n + at];
-        if (tid == 0 && piv.x == 0.0 && piv.y == 0.0) atomicCAS(info, 0, j + 1);
+        if (tid == 0 && !(big > 0.0)) atomicCAS(info, 0, big == 0.0 ? j + 1 : -(j + 1));
         __syncthreads();
         const int pr = at;
         big = -1.0;
@@ -341,7 +343,7 @@ k_lu64_update(double2* __restrict__ A, double2* __restrict__ B, int n, int nrhs,
 #pragma unroll
         for (int m = 0; m < kW - 1; ++m) {
             const double2 u = make_double2(__shfl_sync(0xffffffffu, t.x, base + m), __shfl_sync(0xffffffffu, t.y, base + m));
-            t = cfms(t, l11[i][m], u);  // zero for i <= m
+            if (i > m) t = cfms(t, l11[i][m], u);  // not by its zeros: an infinite entry is to stay one
         }
         top[i][c] = t;
         double2* col = column(c);
@@ -428,6 +430,18 @@ k_lu64_back(const double2* __restrict__ A, double2* __restrict__ B, int n)
     for (int r = tid; r < n; r += kBackThreads) col[r] = x[r];
 }
 
+// found: 1 a NaN, 2 an entry that is infinite and no NaN.
+__global__ void k_lu64_scan(const double2* __restrict__ A, int64_t count, int* __restrict__ found)
+{
+    int f = 0;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < count; t += (int64_t)gridDim.x * blockDim.x) {
+        const double2 a = A[t];
+        if (isnan(a.x) || isnan(a.y)) f |= 1;
+        else if (isinf(a.x) || isinf(a.y)) f |= 2;
+    }
+    if (f) atomicOr(found, f);
+}
+
 }  // namespace
 
 // What it takes: where it beats cuSOLVER.  By the order as above; by the right-hand
@@ -436,12 +450,25 @@ k_lu64_back(const double2* __restrict__ A, double2* __restrict__ B, int n)
 // 1817; 800 3804 and 3413, 4046 and 4565; 1200 6447 and 6428, 7032 and 8776.
 bool lu64_takes(int64_t n, int64_t nrhs) { return n <= 1200 && nrhs <= 768; }
 
-static int lu64_status(mh_ctx* ctx, const int* info)
+// info[0]: the first column (from 1) with a zero pivot, or minus the first without a
+// number, 0 for none.  A holds the factors, or (whole) what came in: in the factors an
+// infinite entry stays in its row of U, so a NaN that came in leaves none behind.
+static int lu64_status(mh_ctx* ctx, int64_t n, const double2* A, bool whole, int* info)
 {
     MH_CUDA_TRY(ctx, cudaGetLastError());
     int h = 0;
     MH_CUDA_TRY(ctx, cudaMemcpyAsync(&h, info, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     MH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    if (h < 0) {
+        int found = 0;
+        MH_CUDA_TRY(ctx, cudaMemsetAsync(info + 1, 0, sizeof(int), ctx->stream));
+        k_lu64_scan<<<(unsigned)std::min<int64_t>((n * n + 255) / 256, 592), 256, 0, ctx->stream>>>(A, n * n, info + 1);
+        ctx->launches += 1;
+        MH_CUDA_TRY(ctx, cudaMemcpyAsync(&found, info + 1, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        MH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+        const bool came_in = whole ? (found & 1) != 0 : (found & 2) == 0;
+        h = came_in && n > 1 ? 0 : -h;
+    }
     if (h > 0) return set_err(ctx, MH_ERR_SINGULAR, "zero pivot at column %d", h);
     return MH_OK;
 }
@@ -462,7 +489,7 @@ int lu64_solve(mh_ctx* ctx, int64_t n, double2* A, double2* B, int nrhs)
         const int rows = (int)(n + 31) / 32 * 32, groups = kPanelThreads / rows;
         k_lu64_whole<<<1, rows * groups, whole, ctx->stream>>>(A, B, (int)n, nrhs, rows, info);
         ctx->launches += 1;
-        return lu64_status(ctx, info);
+        return lu64_status(ctx, n, A, true, info);
     }
     for (int64_t k0 = 0; k0 < n;) {
         const int w = panel_width(n - k0);
@@ -476,7 +503,7 @@ int lu64_solve(mh_ctx* ctx, int64_t n, double2* A, double2* B, int nrhs)
     }
     k_lu64_back<<<nrhs, kBackThreads, sizeof(double2) * (size_t)n, ctx->stream>>>(A, B, (int)n);
     ctx->launches += 1;
-    return lu64_status(ctx, info);
+    return lu64_status(ctx, n, A, false, info);
 }
 
 }  // namespace mh
