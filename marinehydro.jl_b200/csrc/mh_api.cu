@@ -178,30 +178,8 @@ int sync_status(mh_ctx* ctx, const char* what)
 int lu_solve_fp64(mh_ctx* ctx, int64_t n, double2* A, double2* B, int64_t nrhs)
 {
     if (mh::lu64_takes(n, nrhs)) return mh::lu64_solve(ctx, n, A, B, (int)nrhs);
-    int lwork = 0;
-    cusolverStatus_t st = cusolverDnZgetrf_bufferSize(ctx->cusolver, (int)n, (int)n,
-                                                      (cuDoubleComplex*)A, (int)n, &lwork);
-    if (st != CUSOLVER_STATUS_SUCCESS)
-        return set_err(ctx, MH_ERR_CUDA, "cusolverDnZgetrf_bufferSize failed (%d)", (int)st);
-    auto* work = (cuDoubleComplex*)ws_get(ctx, WS_LWORK, sizeof(cuDoubleComplex) * (size_t)lwork);
-    auto* piv = (int*)ws_get(ctx, WS_PIV, sizeof(int) * (size_t)n);
-    auto* info = (int*)ws_get(ctx, WS_INFO, sizeof(int) * 2);
-    if (!work || !piv || !info) return MH_ERR_OOM;
-    st = cusolverDnZgetrf(ctx->cusolver, (int)n, (int)n, (cuDoubleComplex*)A, (int)n, work, piv, info);
-    if (st != CUSOLVER_STATUS_SUCCESS)
-        return set_err(ctx, MH_ERR_CUDA, "cusolverDnZgetrf failed (%d)", (int)st);
-    st = cusolverDnZgetrs(ctx->cusolver, CUBLAS_OP_N, (int)n, (int)nrhs, (const cuDoubleComplex*)A,
-                          (int)n, piv, (cuDoubleComplex*)B, (int)n, info + 1);
-    if (st != CUSOLVER_STATUS_SUCCESS)
-        return set_err(ctx, MH_ERR_CUDA, "cusolverDnZgetrs failed (%d)", (int)st);
-    int h_info[2] = {0, 0};
-    MH_CUDA_TRY(ctx, cudaMemcpyAsync(h_info, info, sizeof(h_info), cudaMemcpyDeviceToHost, ctx->stream));
-    int rc = sync_status(ctx, "LU solve");
-    if (rc) return rc;
-    if (h_info[0] > 0) return set_err(ctx, MH_ERR_SINGULAR, "zero pivot at column %d", h_info[0]);
-    if (h_info[0] < 0 || h_info[1] < 0)
-        return set_err(ctx, MH_ERR_ARG, "LAPACK argument %d invalid", -(h_info[0] ? h_info[0] : h_info[1]));
-    return MH_OK;
+    const int rc = mh::fp64_lu_solve(ctx, n, A, B, (int)nrhs);
+    return rc ? rc : sync_status(ctx, "LU solve");
 }
 
 // C = A B for n x n A and n x nrhs B (device, complex128).
