@@ -398,7 +398,8 @@ int mh_hydro_batch_vjp(mh_ctx* ctx, const mh_mesh* mesh,
  * inputs: the tangents of the mesh fields (t_vertices n_vertices x 3,
  * t_centers and t_normals nfaces x 3, t_areas nfaces; radii only select
  * branches and have none), of the frequencies (t_omegas) and of the dof
- * fields (t_dofs, layout of dofs); any may be NULL (zero).  Returns the
+ * fields (t_dofs, layout of dofs); any may be NULL (zero).  With the Delhommeau
+ * term every panel centre must be at or below the free surface.  Returns the
  * outputs (as mh_hydro_batch, each may be NULL) and their tangents
  * d_added_mass, d_damping, d_diffraction, d_froude_krylov (same layouts).
  * Replaces the reference's ForwardDiff path: Dual element types through

@@ -772,6 +772,7 @@ int mh_mesh_create(mh_ctx* ctx, int64_t nfaces, int64_t nvertices, const double*
     m->n = n;
     m->nv = nvertices;
     m->device = ctx->device;
+    for (int64_t i = 0; i < n; ++i) m->above = m->above || centers[2 * n + i] > 0.0;
     try {
         m->faces.assign(faces, faces + 4 * n);
         MeshPart part;
@@ -1017,6 +1018,10 @@ int mh_hydro_batch_jvp(mh_ctx* ctx, const mh_mesh* mesh, int64_t n_omega, const 
         return rc;
     if ((gf_mask & MH_GF_WU) && (gf_mask & MH_GF_DELHOMMEAU))
         return set_err(ctx, MH_ERR_ARG, "the tangent path takes one wave term (GFWu or Delhommeau)");
+    // pairs above the surface in the tangent kernels raised an illegal instruction on a B200
+    if ((gf_mask & MH_GF_DELHOMMEAU) && mesh->above)
+        return set_err(ctx, MH_ERR_ARG, "forward derivatives of the Delhommeau term need every panel centre at or "
+                                        "below the free surface");
     const int64_t n = mesh->n;
     if ((t_vertices && !finite_array(t_vertices, 3 * mesh->nv)) ||
         (t_centers && !finite_array(t_centers, 3 * n)) || (t_normals && !finite_array(t_normals, 3 * n)) ||

@@ -44,6 +44,7 @@ struct mh_mesh {
     std::vector<int64_t> faces;  // host copy, 4 x n column-major (vertex cotangent scatter)
     double* verts = nullptr;     // device, nv x 3 column-major (generated and combined meshes)
     std::vector<MeshPart> parts; // generated and combined meshes: their parts in order
+    bool above = false;          // a panel centre lies above the free surface
 };
 
 // Workspace slots of a context; each is a grow-only device buffer.

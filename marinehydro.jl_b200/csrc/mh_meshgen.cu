@@ -349,8 +349,13 @@ int make_generated(mh_ctx* ctx, const MeshPart& part, mh_mesh** out)
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(m->faces.data(), dF, sizeof(int64_t) * 4 * (size_t)n,
                                               cudaMemcpyDeviceToHost, st);
+    std::vector<double> cz;  // a hemisphere below the surface and the buoy have no centre above it
+    if (part.kind == MESH_HEMISPHERE && part.p[3] > 0.0) cz.resize((size_t)n);
+    if (e == cudaSuccess && !cz.empty())
+        e = cudaMemcpyAsync(cz.data(), m->geom + (G_CX + 2) * n, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, st);
     if (dF) cudaFreeAsync(dF, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    for (const double z : cz) m->above = m->above || z > 0.0;
     if (e != cudaSuccess) {
         if (m->geom) cudaFreeAsync(m->geom, st);
         if (m->verts) cudaFreeAsync(m->verts, st);
@@ -516,6 +521,7 @@ int mh_mesh_combine(mh_ctx* ctx, int count, const mh_mesh* const* meshes, mh_mes
         }
         off += m->n;
         voff += m->nv;
+        c->above = c->above || m->above;
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {

@@ -167,7 +167,8 @@ def hydro_batch_jvp(mesh: Mesh, omegas, dofs, betas=(), t_mesh: MeshTangent | No
     """Forward batch (as ``hydro_batch``) plus the tangents of its outputs
     along one direction of the inputs (``mh_hydro_batch_jvp``): the tangent
     of the mesh fields (a ``MeshTangent``; radii have no effect), of the
-    frequencies and of the dof fields (None = zero)."""
+    frequencies and of the dof fields (None = zero).  With the Delhommeau term
+    every panel centre must be at or below the free surface."""
     mask = gf_mask(green_functions)
     dm = device_mesh(mesh, ctx)
     om = np.ascontiguousarray(np.asarray(omegas, dtype=np.float64).reshape(-1))

@@ -2,7 +2,8 @@
 the library's pivoted LU, whose pivot search must not see them: a NaN comes through
 to the outputs, infinite entries are refused, and the context's later calls are what
 they were.  Wu's term is not defined above the free surface: a body that rises out of
-the water has NaN and infinite entries."""
+the water has NaN and infinite entries.  Forward derivatives of the Delhommeau term
+there are refused before anything is launched."""
 import numpy as np
 import pytest
 
@@ -61,3 +62,16 @@ def test_gradients_out_of_the_water(mh, gpu, precision):
                            precision=precision, ctx=gpu)
     assert np.isnan(r.added_mass).any()
     assert np.isnan(_jvp(mh, gpu, dry, mh.GFWu(), precision).d_added_mass).any()
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_forward_derivatives_of_delhommeau_above_the_surface_are_refused(mh, gpu, precision):
+    dry = mh.mesh_hemisphere(1.0, (0.0, 0.0, 0.3), (8, 10))
+    wet = mh.mesh_hemisphere(1.0, (0.0, 0.0, 0.0), (8, 10))
+    for mesh in (dry, mh.combine_meshes([wet, dry]), mh.generate_hemisphere(1.0, (0.0, 0.0, 0.3), (8, 10), ctx=gpu),
+                 mh.generate_combined([wet, dry], ctx=gpu)):
+        with pytest.raises(mh.ArgumentError, match="free surface"):
+            _jvp(mh, gpu, mesh, mh.ExactGuevelDelhommeau(), precision)
+    low = mh.generate_hemisphere(1.0, (0.0, 0.0, 0.01), (8, 10), ctx=gpu)  # its centres are below
+    for mesh in (wet, low):
+        assert np.isfinite(_jvp(mh, gpu, mesh, mh.ExactGuevelDelhommeau(), precision).d_added_mass).all()
