@@ -691,9 +691,9 @@ __global__ void k_refine_add(double2* __restrict__ x, const float2* __restrict__
     x[t] = make_double2(x[t].x + (double)d[t].x, x[t].y + (double)d[t].y);
 }
 
-// Keeps what is no finite number from cuSOLVER's zgetrf: where a column has a NaN its
-// pivot search can name a row outside the matrix, and the exchange then writes there
-// (a NaN anywhere came back as finite numbers).  flag: 1 a NaN, 2 an infinite entry of
+// Keeps what is no finite number from cuSOLVER's zgetrf: a NaN anywhere came back as
+// finite numbers.  Why is not known; a pivot search that names a row outside the matrix,
+// with which the exchange then swaps, would explain it.  flag: 1 a NaN, 2 an infinite entry of
 // matrix blockIdx.y; its last CTA then puts the identity in the matrix's place.  With
 // several CTAs a matrix, flag and ticket are zero before.  k_guard_poison, after the
 // factorisation, makes the solutions X of a matrix with a NaN (may be null), and all
